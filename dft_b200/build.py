@@ -30,6 +30,7 @@ SOURCES = {
     "capi.cu": [],
     "grid_ops.cu": [],
     "davidson.cu": [],
+    "dense_fp64.cu": [],
     "scf.cu": [],
     "radial.cu": ["-fmad=false"],
     "gram_tc.cu": [],

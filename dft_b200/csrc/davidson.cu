@@ -13,8 +13,8 @@
 //       :521-555, with the same 1e-10 guard), projected out of V twice and orthonormalised
 //       by the symmetric (SVQB) scheme, then appended; thick restart to [X] when full.
 //
-// Tall-skinny products (Gram V^T W, rotation V Y) are FP64 kernels with warp/block
-// reductions; the k x k eigenproblems are solved on the host (eigh.cpp).
+// Tall-skinny products (Gram V^T W, rotation V Y, the residual block) run on the FP64 tensor
+// pipe (dense_fp64.cu); the k x k eigenproblems are solved on the host (eigh.cpp).
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -61,98 +61,6 @@ __global__ void seed_kernel(Grid g, double* psi, long long ld, int nb, int seed0
             default: break;
         }
         out[p] = pl * exp(-r2 * factor);
-    }
-}
-
-constexpr int GT = 32;          // Gram output tile (GT x GT)
-constexpr int GP = 32;          // points per shared-memory stage
-constexpr int GRAM_THREADS = 256;
-
-// partial[c][i][j] = sum over chunk c of A_i[p] B_j[p] for one GT x GT output tile.
-// 256 threads = 16 x 16, each owns a 2 x 2 block of the tile.
-__global__ void __launch_bounds__(GRAM_THREADS) gram_kernel(const double* __restrict__ A, long long lda, int ka,
-                                                            const double* __restrict__ B, long long ldb, int kb,
-                                                            long long n, long long chunk, double* __restrict__ partial) {
-    __shared__ double sa[GT][GP + 1];
-    __shared__ double sb[GT][GP + 1];
-    const int ti = blockIdx.x * GT, tj = blockIdx.y * GT;
-    const long long p0 = (long long)blockIdx.z * chunk;
-    const long long p1 = min(n, p0 + chunk);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc00 = 0.0, acc01 = 0.0, acc10 = 0.0, acc11 = 0.0;
-    for (long long ps = p0; ps < p1; ps += GP) {
-        // stage GT vectors x GP points of A and B (coalesced along points)
-        for (int e = threadIdx.x; e < GT * GP; e += GRAM_THREADS) {
-            const int r = e / GP, c = e % GP;
-            const long long p = ps + c;
-            const int ia = ti + r, jb = tj + r;
-            sa[r][c] = (ia < ka && p < p1) ? A[(long long)ia * lda + p] : 0.0;
-            sb[r][c] = (jb < kb && p < p1) ? B[(long long)jb * ldb + p] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int c = 0; c < GP; ++c) {
-            const double a0 = sa[ty][c], a1 = sa[ty + 16][c];
-            const double b0 = sb[tx][c], b1 = sb[tx + 16][c];
-            acc00 += a0 * b0;
-            acc01 += a0 * b1;
-            acc10 += a1 * b0;
-            acc11 += a1 * b1;
-        }
-        __syncthreads();
-    }
-    double* out = partial + (long long)blockIdx.z * ka * kb;
-    const int i0 = ti + ty, i1 = ti + ty + 16, j0 = tj + tx, j1 = tj + tx + 16;
-    if (i0 < ka && j0 < kb) out[(long long)i0 * kb + j0] = acc00;
-    if (i0 < ka && j1 < kb) out[(long long)i0 * kb + j1] = acc01;
-    if (i1 < ka && j0 < kb) out[(long long)i1 * kb + j0] = acc10;
-    if (i1 < ka && j1 < kb) out[(long long)i1 * kb + j1] = acc11;
-}
-
-// out[e] = scale * sum_c partial[c][e]: one warp per element, lanes stride the chunks, fixed
-// shuffle order (deterministic)
-__global__ void gram_reduce_kernel(int nchunks, int nel, const double* __restrict__ partial, double scale,
-                                   double* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    const int warps = blockDim.x >> 5;
-    for (int e = blockIdx.x * warps + (threadIdx.x >> 5); e < nel; e += gridDim.x * warps) {
-        double s = 0.0;
-        for (int c = lane; c < nchunks; c += 32) s += partial[(long long)c * nel + e];
-        s = warp_sum(s);
-        if (lane == 0) out[e] = s * scale;
-    }
-}
-
-constexpr int RJ = 16;  // output columns per rotation block
-
-// out_j = beta*out_j + alpha * sum_i in_i * Y[i*m + j], j in a RJ-column slice per blockIdx.y
-__global__ void __launch_bounds__(256) rotate_kernel(const double* __restrict__ in, long long ldi, int k,
-                                                     const double* __restrict__ Y, int m, double* __restrict__ out,
-                                                     long long ldo, long long n, double alpha, double beta) {
-    extern __shared__ double sy[];  // k x RJ
-    const int j0 = blockIdx.y * RJ;
-    const int nj = min(RJ, m - j0);
-    for (int e = threadIdx.x; e < k * RJ; e += blockDim.x) {
-        const int i = e / RJ, jj = e % RJ;
-        sy[e] = jj < nj ? Y[(long long)i * m + j0 + jj] : 0.0;
-    }
-    __syncthreads();
-    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
-        double acc[RJ];
-#pragma unroll
-        for (int jj = 0; jj < RJ; ++jj) acc[jj] = 0.0;
-        for (int i = 0; i < k; ++i) {
-            const double v = __ldg(in + (long long)i * ldi + p);
-#pragma unroll
-            for (int jj = 0; jj < RJ; ++jj) acc[jj] += v * sy[i * RJ + jj];
-        }
-#pragma unroll
-        for (int jj = 0; jj < RJ; ++jj) {
-            if (jj < nj) {
-                double* o = out + (long long)(j0 + jj) * ldo + p;
-                *o = beta == 0.0 ? alpha * acc[jj] : beta * *o + alpha * acc[jj];
-            }
-        }
     }
 }
 
@@ -241,208 +149,7 @@ __global__ void rows_sum_kernel2(int nrows, int ncols, const double* partial, do
     }
 }
 
-// ------------------------------------------------------------------ host helpers -----
-
-struct Blocks {
-    dft_context* ctx;
-    Grid g;
-    long long ld;
-};
-
-// Narrow Gram products (ka <= 64, kb <= KB): one launch.  Warp w of every block owns rows
-// i = w, w + 8, ... of A (RPW of them) and all kb columns; its lanes stride the points and
-// keep RPW x KB sums in registers.  Block partials go to `partial`; the partials are then
-// added in two fixed-order levels inside the same launch: the last block to finish in each
-// group of GS_GROUP blocks (ticket[1 + group]) adds its group's partials, and the last group
-// to finish (ticket[0]) adds the group sums and writes dV * C.  Every thread of a reducing
-// block owns whole elements and issues its (at most GS_GROUP) loads at once, so the tail is a
-// few L2 round trips instead of one dependent chain per element.
-constexpr int GS_GROUP = 16;
-constexpr int GS_TICKETS = 256;  // ticket words: 1 + groups (blocks <= 4 x SMs)
-
-template <int RPW, int KB>
-__global__ void __launch_bounds__(256) gram_small_kernel(const double* __restrict__ A, long long lda, int ka,
-                                                         const double* __restrict__ B, long long ldb, int kb,
-                                                         long long n, double scale, double* __restrict__ partial,
-                                                         unsigned int* __restrict__ ticket, double* __restrict__ out) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double acc[RPW][KB];
-#pragma unroll
-    for (int r = 0; r < RPW; ++r)
-#pragma unroll
-        for (int j = 0; j < KB; ++j) acc[r][j] = 0.0;
-    // two points per step (both loads issued before the FMAs) for more loads in flight
-    const long long stride = (long long)gridDim.x * 32;
-    for (long long p = (long long)blockIdx.x * 32 + lane; p < n; p += 2 * stride) {
-        const long long p2 = p + stride;
-        const bool has2 = p2 < n;
-        double b[KB], b2[KB];
-#pragma unroll
-        for (int j = 0; j < KB; ++j) {
-            b[j] = j < kb ? __ldg(B + (long long)j * ldb + p) : 0.0;
-            b2[j] = (j < kb && has2) ? __ldg(B + (long long)j * ldb + p2) : 0.0;
-        }
-#pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-            const int i = warp + 8 * r;
-            const double a = i < ka ? __ldg(A + (long long)i * lda + p) : 0.0;
-            const double a2 = (i < ka && has2) ? __ldg(A + (long long)i * lda + p2) : 0.0;
-#pragma unroll
-            for (int j = 0; j < KB; ++j) acc[r][j] = fma(a2, b2[j], fma(a, b[j], acc[r][j]));
-        }
-    }
-    const int nel = ka * kb;
-    double* mine = partial + (long long)blockIdx.x * nel;
-#pragma unroll
-    for (int r = 0; r < RPW; ++r)
-#pragma unroll
-        for (int j = 0; j < KB; ++j) {
-            const double v = warp_sum(acc[r][j]);
-            const int i = warp + 8 * r;
-            if (lane == 0 && i < ka && j < kb) mine[i * kb + j] = v;
-        }
-    // level 1: the last block of this group adds the group's partials in block order
-    const int nblk = (int)gridDim.x;
-    const int ngroups = (nblk + GS_GROUP - 1) / GS_GROUP;
-    const int grp = (int)blockIdx.x / GS_GROUP;
-    const int g0 = grp * GS_GROUP;
-    const int gsz = min(GS_GROUP, nblk - g0);
-    double* gsum = partial + (long long)nblk * nel;  // [ngroups][nel]
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ticket + 1 + grp, 1u) == (unsigned)gsz - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int e = threadIdx.x; e < nel; e += blockDim.x) {
-        double v[GS_GROUP];
-#pragma unroll
-        for (int c = 0; c < GS_GROUP; ++c) v[c] = c < gsz ? __ldcg(partial + (long long)(g0 + c) * nel + e) : 0.0;
-        double sum = 0.0;
-#pragma unroll
-        for (int c = 0; c < GS_GROUP; ++c) sum += v[c];
-        gsum[(long long)grp * nel + e] = sum;
-    }
-    if (threadIdx.x == 0) ticket[1 + grp] = 0;  // ready for the next call
-    // level 2: the last group adds the group sums in group order
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == (unsigned)ngroups - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int e = threadIdx.x; e < nel; e += blockDim.x) {
-        double sum = 0.0;
-        for (int c0 = 0; c0 < ngroups; c0 += 8) {
-            double v[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) v[c] = c0 + c < ngroups ? __ldcg(gsum + (long long)(c0 + c) * nel + e) : 0.0;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) sum += v[c];
-        }
-        out[e] = sum * scale;
-    }
-    if (threadIdx.x == 0) *ticket = 0;
-}
-
-// C (ka x kb, host, row-major) = dV * A^T B
-void gram(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B, long long ldb,
-          int kb, std::vector<double>& C) {
-    C.assign((size_t)ka * kb, 0.0);
-    if (ka == 0 || kb == 0) return;
-    const int rpw = ka <= 8 ? 1 : ka <= 16 ? 2 : ka <= 32 ? 4 : 8;
-    const int kbt = kb <= 4 ? 4 : kb <= 8 ? 8 : 16;
-    if (ka <= 64 && kb <= 16 && rpw * kbt <= 64) {
-        // narrow product: one launch, the last block reduces
-        const size_t nel = (size_t)ka * kb;
-        const int nblk = (int)std::max<long long>(
-            1, std::min<long long>(std::min(4LL * ctx->num_sms, (long long)(GS_TICKETS - 1) * GS_GROUP),
-                                   (g.N + 255) / 256));
-        const int ngroups = (nblk + GS_GROUP - 1) / GS_GROUP;
-        double* partial = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * (nel * (nblk + ngroups) + nel) + 64);
-        double* res = partial + nel * (nblk + ngroups);
-        if (!ctx->gram_ticket) {
-            DFT_CUDA(cudaMalloc(&ctx->gram_ticket, sizeof(unsigned int) * GS_TICKETS));
-            DFT_CUDA(cudaMemsetAsync(ctx->gram_ticket, 0, sizeof(unsigned int) * GS_TICKETS, ctx->stream));
-        }
-        unsigned int* tk = (unsigned int*)ctx->gram_ticket;
-#define DFT_GS(R, K)                                                                                          \
-    gram_small_kernel<R, K><<<nblk, 256, 0, ctx->stream>>>(A, lda, ka, B, ldb, kb, g.N, g.dV, partial, tk, res)
-        switch (rpw * 100 + kbt) {
-            case 104: DFT_GS(1, 4); break;
-            case 108: DFT_GS(1, 8); break;
-            case 116: DFT_GS(1, 16); break;
-            case 204: DFT_GS(2, 4); break;
-            case 208: DFT_GS(2, 8); break;
-            case 216: DFT_GS(2, 16); break;
-            case 404: DFT_GS(4, 4); break;
-            case 408: DFT_GS(4, 8); break;
-            case 416: DFT_GS(4, 16); break;
-            case 804: DFT_GS(8, 4); break;
-            default: DFT_GS(8, 8); break;
-        }
-#undef DFT_GS
-        DFT_LAUNCH_CHECK();
-        count_launch(ctx);
-        double* h = pinned(ctx, nel);
-        DFT_CUDA(cudaMemcpyAsync(h, res, sizeof(double) * nel, cudaMemcpyDeviceToHost, ctx->stream));
-        sync(ctx);
-        std::memcpy(C.data(), h, sizeof(double) * nel);
-        return;
-    }
-    const int tx = (ka + GT - 1) / GT, ty = (kb + GT - 1) / GT;
-    long long target = 4LL * ctx->num_sms;
-    long long nch = std::max<long long>(1, target / (tx * ty));
-    long long chunk = (g.N + nch - 1) / nch;
-    chunk = ((chunk + GP - 1) / GP) * GP;
-    nch = (g.N + chunk - 1) / chunk;
-    nch = std::min<long long>(nch, 65535);
-    chunk = (g.N + nch - 1) / nch;
-    const size_t nel = (size_t)ka * kb;
-    double* partial = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * (nel * nch + nel));
-    double* res = partial + nel * nch;
-    gram_kernel<<<dim3(tx, ty, (unsigned)nch), GRAM_THREADS, 0, ctx->stream>>>(A, lda, ka, B, ldb, kb, g.N, chunk,
-                                                                               partial);
-    DFT_LAUNCH_CHECK();
-    const int rb = (int)std::min<size_t>((nel + 7) / 8, 4096);  // 8 warps per block, one element per warp
-    gram_reduce_kernel<<<rb, 256, 0, ctx->stream>>>((int)nch, (int)nel, partial, g.dV, res);
-    DFT_LAUNCH_CHECK();
-    count_launch(ctx, 2);
-    double* h = pinned(ctx, nel);
-    DFT_CUDA(cudaMemcpyAsync(h, res, sizeof(double) * nel, cudaMemcpyDeviceToHost, ctx->stream));
-    sync(ctx);
-    std::memcpy(C.data(), h, sizeof(double) * nel);
-}
-
 }  // namespace
-
-// out = beta*out + alpha * in * Y   (Y: k x m host row-major)
-void rotate(dft_context* ctx, const Grid& g, const double* in, long long ldi, int k, const std::vector<double>& Y, int m,
-            double* out, long long ldo, double alpha, double beta) {
-    if (m == 0) return;
-    if (k == 0) {
-        if (beta == 0.0)
-            for (int j = 0; j < m; ++j)
-                DFT_CUDA(cudaMemsetAsync(out + (long long)j * ldo, 0, sizeof(double) * (size_t)g.N, ctx->stream));
-        return;
-    }
-    double* dy = (double*)ws_get(ctx, WS_TMP, sizeof(double) * (size_t)k * m);
-    DFT_CUDA(cudaMemcpyAsync(dy, Y.data(), sizeof(double) * (size_t)k * m, cudaMemcpyHostToDevice, ctx->stream));
-    const int jt = (m + RJ - 1) / RJ;
-    const size_t smem = sizeof(double) * (size_t)k * RJ;
-    if (smem > 200 * 1024) fail(DFT_INVALID_ARGUMENT, "subspace too large for the rotation kernel (k=%d)", k);
-    static bool attr_set = false;
-    if (!attr_set) {
-        DFT_CUDA(cudaFuncSetAttribute(rotate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr_set = true;
-    }
-    long long bx = (g.N + 255) / 256;
-    bx = std::min<long long>(bx, std::max<long long>(1, (8LL * ctx->num_sms + jt - 1) / jt));
-    rotate_kernel<<<dim3((unsigned)bx, jt), 256, smem, ctx->stream>>>(in, ldi, k, dy, m, out, ldo, g.N, alpha, beta);
-    DFT_LAUNCH_CHECK();
-    count_launch(ctx);
-}
 
 namespace {
 
@@ -487,7 +194,19 @@ void gram_any(bool tc, dft_context* ctx, const Grid& g, const double* A, long lo
     // the tensor-core product pays only when both blocks are wide enough to fill its tiles;
     // narrow products (few bands) are latency-bound either way and stay in FP64
     if (tc && (long long)ka * kb >= 2048) gram_tc(ctx, g, A, lda, ka, B, ldb, kb, C);
-    else gram(ctx, g, A, lda, ka, B, ldb, kb, C);
+    else gram_fp64(ctx, g, A, lda, ka, B, ldb, kb, C);
+}
+
+// out (m rows of the block that `in` belongs to) = in * Y, in place where the rotation allows it,
+// else through W
+void rotate_onto(dft_context* ctx, const Grid& g, const double* in, int k, const std::vector<double>& Y, int m,
+                 double* out, long long ld, double* W) {
+    if (rotate_in_place(k, m)) {
+        rotate(ctx, g, in, ld, k, Y, m, out, ld, 1.0, 0.0);
+        return;
+    }
+    rotate(ctx, g, in, ld, k, Y, m, W, ld, 1.0, 0.0);
+    DFT_CUDA(cudaMemcpyAsync(out, W, sizeof(double) * (size_t)ld * m, cudaMemcpyDeviceToDevice, ctx->stream));
 }
 
 int orthonormalise(dft_context* ctx, const Grid& g, const double* V, int k, double* T, int nt, long long ld,
@@ -521,12 +240,13 @@ int orthonormalise(dft_context* ctx, const Grid& g, const double* V, int k, doub
                     for (int j = 0; j < nt; ++j) Yc[(size_t)(k + i) * nt + j] = Yk[(size_t)i * nt + j];
                 // in mixed-precision mode a wide rotation runs on the tensor cores like the Ritz
                 // rotations (the second pass restores orthonormality to the products' accuracy)
-                if (tc && k + nt >= 32 && (long long)(k + nt) * nt >= 2048)
+                if (tc && k + nt >= 32 && (long long)(k + nt) * nt >= 2048) {
                     rotate_tc(ctx, g, V, ld, k + nt, Yc, nt, W, ld);
-                else
-                    rotate(ctx, g, V, ld, k + nt, Yc, nt, W, ld, 1.0, 0.0);
-                DFT_CUDA(cudaMemcpyAsync(T, W, sizeof(double) * (size_t)ld * nt, cudaMemcpyDeviceToDevice,
-                                         ctx->stream));
+                    DFT_CUDA(cudaMemcpyAsync(T, W, sizeof(double) * (size_t)ld * nt, cudaMemcpyDeviceToDevice,
+                                             ctx->stream));
+                } else {
+                    rotate_onto(ctx, g, V, k + nt, Yc, nt, T, ld, W);
+                }
                 // In FP64 one pass suffices when the block was far from dependent: the loss of
                 // orthogonality of projected Cholesky QR is about eps * r * kappa(S), with
                 // r = max_i (T^T T)_ii / S_ii (the cancellation of the projection) and
@@ -559,8 +279,7 @@ int orthonormalise(dft_context* ctx, const Grid& g, const double* V, int k, doub
         // (O(nt^3/3) on the host); a nearly dependent block falls through to the SVQB below,
         // which drops the dependent directions
         if (cholesky_inverse_t(nt, S, chol_rel, Yk)) {
-            rotate(ctx, g, T, ld, nt, Yk, nt, W, ld, 1.0, 0.0);
-            DFT_CUDA(cudaMemcpyAsync(T, W, sizeof(double) * (size_t)ld * nt, cudaMemcpyDeviceToDevice, ctx->stream));
+            rotate_onto(ctx, g, T, nt, Yk, nt, T, ld, W);
             continue;
         }
         std::vector<double> Sc = S;
@@ -575,19 +294,13 @@ int orthonormalise(dft_context* ctx, const Grid& g, const double* V, int k, doub
         Yk.assign((size_t)nt * nk, 0.0);
         for (int i = 0; i < nt; ++i)
             for (int c = 0; c < nk; ++c) Yk[(size_t)i * nk + c] = Z[(size_t)i * nt + keep[c]] / std::sqrt(w[keep[c]]);
-        rotate(ctx, g, T, ld, nt, Yk, nk, W, ld, 1.0, 0.0);
-        DFT_CUDA(cudaMemcpyAsync(T, W, sizeof(double) * (size_t)ld * nk, cudaMemcpyDeviceToDevice, ctx->stream));
+        rotate_onto(ctx, g, T, nt, Yk, nk, T, ld, W);
         nt = nk;
     }
     return nt;
 }
 
 }  // namespace
-
-void gram_fp64(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B,
-               long long ldb, int kb, std::vector<double>& C) {
-    gram(ctx, g, A, lda, ka, B, ldb, kb, C);
-}
 
 int solve_orbitals(dft_context* ctx, const Grid& g, const double* V, int nocc, int nbands, double* psi,
                    long long ld, bool init, double* eig_host, double* resid_host, const EigOpts& o,
@@ -608,8 +321,9 @@ int solve_orbitals(dft_context* ctx, const Grid& g, const double* V, int nocc, i
     const size_t vecb = sizeof(double) * (size_t)ld;
     double* Vb = (double*)ws_get(ctx, WS_DAV0, vecb * kmax);
     double* AV = (double*)ws_get(ctx, WS_DAV1, vecb * kmax);
-    double* X = (double*)ws_get(ctx, WS_DAV2, vecb * nb);
-    double* AX = (double*)ws_get(ctx, WS_DAV3, vecb * nb);
+    // Ritz vectors and their H psi: stored only in mixed-precision solves
+    double* X = o.mixed_precision ? (double*)ws_get(ctx, WS_DAV2, vecb * nb) : nullptr;
+    double* AX = o.mixed_precision ? (double*)ws_get(ctx, WS_DAV3, vecb * nb) : nullptr;
     double* R = (double*)ws_get(ctx, WS_DAV4, vecb * nb);
     double* W = (double*)ws_get(ctx, WS_DAV5, vecb * std::max(nb, kr));
     const double kin = g.ix2 + g.iy2 + g.iz2;  // buildHamiltonianDiagonal :496-500 (1/dx^2 + 1/dy^2 + 1/dz^2)
@@ -678,15 +392,13 @@ int solve_orbitals(dft_context* ctx, const Grid& g, const double* V, int nocc, i
     };
     grow_G(0, k);
 
-    // out = in * Y: on the tensor cores in mixed-precision mode when the block is wide enough
-    auto rot = [&](const double* in, int kin, const std::vector<double>& Ym, int m, double* out) {
-        if (tc_mode && kin >= 32 && (long long)kin * m >= 2048) rotate_tc(ctx, g, in, ld, kin, Ym, m, out, ld);
-        else rotate(ctx, g, in, ld, kin, Ym, m, out, ld, 1.0, 0.0);
-    };
+    // rotations run on the tensor cores in mixed-precision mode when the block is wide enough
+    auto rot_tc = [&](int kin, int m) { return tc_mode && kin >= 32 && (long long)kin * m >= 2048; };
+    bool have_x = false;  // X holds the current Ritz vectors
     double* dtheta = (double*)ws_get(ctx, WS_DAV6, sizeof(double) * 2 * nb + sizeof(int) * nb + 64);
     double* dsigma = dtheta + nb;
     int* dsrc = (int*)(dsigma + nb);
-    std::vector<double> theta(nb), rn(nb), w, Z, Y;
+    std::vector<double> theta(nb), rn(nb), ss(nb), w, Z, Y;
     std::vector<int> active;
     int it = 0;
     bool done = false;
@@ -697,20 +409,29 @@ int solve_orbitals(dft_context* ctx, const Grid& g, const double* V, int nocc, i
         if (!eigh_lowest(k, Gc, nb, w, Z)) fail(DFT_NUMERICAL, "projected eigensolve failed");
         Y = Z;
         for (int j = 0; j < nb; ++j) theta[j] = w[j];
-        rot(Vb, k, Y, nb, X);
-        rot(AV, k, Y, nb, AX);
-        // ---- residuals --------------------------------------------------------------------
+        const double* hs;
         DFT_CUDA(cudaMemcpyAsync(dtheta, theta.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, ctx->stream));
-        double* partial = (double*)ws_get(ctx, WS_REDUCE, sizeof(double) * ((size_t)eb * nb + nb));
-        residual_kernel<<<dim3(eb, nb), 256, 0, ctx->stream>>>(AX, X, dtheta, R, ld, g.N, partial);
-        DFT_LAUNCH_CHECK();
-        rows_sum_kernel2<<<1, 256, 0, ctx->stream>>>(nb, eb, partial, partial + (size_t)eb * nb);
-        DFT_LAUNCH_CHECK();
-        count_launch(ctx, 2);
-        double* hs = pinned(ctx, nb);
-        DFT_CUDA(cudaMemcpyAsync(hs, partial + (size_t)eb * nb, sizeof(double) * nb, cudaMemcpyDeviceToHost,
-                                 ctx->stream));
-        sync(ctx);
+        if (rot_tc(k, nb)) {
+            rotate_tc(ctx, g, Vb, ld, k, Y, nb, X, ld);
+            rotate_tc(ctx, g, AV, ld, k, Y, nb, AX, ld);
+            have_x = true;
+            double* partial = (double*)ws_get(ctx, WS_REDUCE, sizeof(double) * ((size_t)eb * nb + nb));
+            residual_kernel<<<dim3(eb, nb), 256, 0, ctx->stream>>>(AX, X, dtheta, R, ld, g.N, partial);
+            DFT_LAUNCH_CHECK();
+            rows_sum_kernel2<<<1, 256, 0, ctx->stream>>>(nb, eb, partial, partial + (size_t)eb * nb);
+            DFT_LAUNCH_CHECK();
+            count_launch(ctx, 2);
+            double* h = pinned(ctx, nb);
+            DFT_CUDA(cudaMemcpyAsync(h, partial + (size_t)eb * nb, sizeof(double) * nb, cudaMemcpyDeviceToHost,
+                                     ctx->stream));
+            sync(ctx);
+            hs = h;
+        } else {
+            // R in one pass over V and AV; the Ritz vectors themselves are formed where they are used
+            ritz_residual(ctx, g, Vb, AV, ld, k, Y, theta.data(), nb, R, ss.data());
+            have_x = false;
+            hs = ss.data();
+        }
         bool occ_conv = true;
         active.clear();
         for (int b = 0; b < nb; ++b) {
@@ -740,6 +461,8 @@ int solve_orbitals(dft_context* ctx, const Grid& g, const double* V, int nocc, i
             if (occ_conv || mx < o.mixed_switch || stalled) {
                 // switch to FP64: restart from the Ritz block, re-orthonormalised and re-projected
                 tc_mode = false;
+                if (!have_x) rotate(ctx, g, Vb, ld, k, Y, nb, X, ld, 1.0, 0.0);
+                have_x = true;
                 DFT_CUDA(cudaMemcpyAsync(Vb, X, vecb * nb, cudaMemcpyDeviceToDevice, ctx->stream));
                 k = orthonormalise(ctx, g, Vb, 0, Vb, nb, ld, W);
                 if (k < nb) fail(DFT_NUMERICAL, "Ritz block lost rank at the FP64 switch");
@@ -765,10 +488,14 @@ int solve_orbitals(dft_context* ctx, const Grid& g, const double* V, int nocc, i
             } else {
                 Zk = Z;
             }
-            rot(Vb, k, Zk, keep, W);
-            DFT_CUDA(cudaMemcpyAsync(Vb, W, vecb * keep, cudaMemcpyDeviceToDevice, ctx->stream));
-            rot(AV, k, Zk, keep, W);
-            DFT_CUDA(cudaMemcpyAsync(AV, W, vecb * keep, cudaMemcpyDeviceToDevice, ctx->stream));
+            for (double* B : {Vb, AV}) {
+                if (rot_tc(k, keep)) {
+                    rotate_tc(ctx, g, B, ld, k, Zk, keep, W, ld);
+                    DFT_CUDA(cudaMemcpyAsync(B, W, vecb * keep, cudaMemcpyDeviceToDevice, ctx->stream));
+                } else {
+                    rotate_onto(ctx, g, B, k, Zk, keep, B, ld, W);
+                }
+            }
             k = keep;
             G.assign((size_t)k * k, 0.0);
             for (int i = 0; i < k; ++i) G[(size_t)i * k + i] = w[i];
@@ -828,8 +555,11 @@ int solve_orbitals(dft_context* ctx, const Grid& g, const double* V, int nocc, i
         k += nt;
     }
     // ---- outputs -----------------------------------------------------------------------
-    DFT_CUDA(cudaMemcpy2DAsync(psi, vecb, X, vecb, sizeof(double) * (size_t)g.N, nb, cudaMemcpyDeviceToDevice,
-                               ctx->stream));
+    if (have_x)
+        DFT_CUDA(cudaMemcpy2DAsync(psi, vecb, X, vecb, sizeof(double) * (size_t)g.N, nb, cudaMemcpyDeviceToDevice,
+                                   ctx->stream));
+    else
+        rotate(ctx, g, Vb, ld, k, Y, nb, psi, ld, 1.0, 0.0);
     for (int b = 0; b < nb; ++b) {
         eig_host[b] = theta[b];
         if (resid_host) resid_host[b] = rn[b];

@@ -1,0 +1,532 @@
+// FP64 tall-skinny products of the block eigensolver on the FP64 tensor pipe:
+//   gram_fp64    C = dV A^T B            (bands x bands, summed over the grid points)
+//   rotate       X = beta X + alpha V Y  (bands x points)
+//   ritz_residual  R = (AV) Y - (V Y) diag(theta) and |R_b|^2, without storing V Y or (AV) Y
+//
+// All three read band blocks band-major (points contiguous), which is the K-contiguous operand
+// layout of mma.m8n8k4.f64 for the Gram product and the N-contiguous one for the rotations, so
+// fragments are loaded straight from global memory: a lane's 16-byte load covers two points, and
+// since the order of the summed points (Gram) or of the output columns (rotation) is free, its
+// two halves feed two MMAs without any exchange.  Measured on B200 (148 SMs, 1965 MHz):
+// mma.m8n8k4.f64 sustains 37.1 TFLOP/s, plain FMA 33.0, and the MMA needs a quarter of the operand
+// reads of an 8 x 8 register tile; tcgen05 has no FP64 kind.
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+#include "ops.h"
+
+namespace dftb {
+
+namespace {
+
+// D (8 x 8) += A (8 x 4, row) B (4 x 8, col).  Lane l holds A[l/4][l%4], B[l%4][l/4] and
+// D[l/4][2 (l%4) + {0, 1}].
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d[0]), "+d"(d[1])
+        : "d"(a), "d"(b));
+}
+
+// Two neighbouring doubles: one 16-byte load where AL says that every row starts 16-byte aligned.
+template <bool AL>
+__device__ __forceinline__ double2 load2(const double* p) {
+    if (AL) return __ldg(reinterpret_cast<const double2*>(p));
+    return make_double2(__ldg(p), __ldg(p + 1));
+}
+
+// ---------------------------------------------------------------- Gram -----------------
+// A block of 8 warps (WM along the rows of A, WK = 8 / WM along the points) owns a tile of
+// WM x 16 rows and RN x 8 columns of C and one chunk of the points.  A warp walks its share of
+// the chunk 8 KU points at a time: per 8 points two A fragments and RN B fragments (one 16-byte
+// load each) feed 4 RN MMAs.  The WK partial tiles are added in shared memory in warp order; the
+// block's tile goes to partial[chunk].
+//
+// The chunks' partials are added in a fixed order.  Small products (nel <= GM_INLINE) do that in the same
+// launch, in two levels: the last block to finish in a group of GM_GROUP chunks (ticket[1 + group])
+// adds the group's partials, the last group (ticket[0]) adds the group sums and writes dV C.
+constexpr int GM_THREADS = 256;
+constexpr int GM_GROUP = 16;
+constexpr int GM_TICKETS = 256;  // ticket words: 1 + groups
+constexpr int GM_INLINE = 1024;
+
+template <int RN, int KU, bool AL>
+__global__ void __launch_bounds__(GM_THREADS, 2)
+    gram_mma_kernel(const double* __restrict__ A, long long lda, int ka, const double* __restrict__ B, long long ldb,
+                    int kb, long long n, long long chunk, int wm_count, double scale, double* __restrict__ partial,
+                    unsigned int* __restrict__ ticket, double* __restrict__ out) {
+    extern __shared__ double tile[];  // (16 wm_count) x (8 RN + 2)
+    constexpr int TS = 8 * RN + 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wm = warp % wm_count, wk = warp / wm_count, wk_count = 8 / wm_count;
+    const int g = lane >> 2, t = lane & 3;
+    const int m0 = blockIdx.x * 16 * wm_count, n0 = blockIdx.y * 8 * RN;
+    const long long p0 = (long long)blockIdx.z * chunk, p1 = min(n, p0 + chunk);
+    // fragment row 8 r is read while 8 r < va (A) or vb (B); rows past the end count as zero
+    const int va = ka - (m0 + wm * 16 + g), vb = kb - (n0 + g);
+    const double* pa = A + (long long)(m0 + wm * 16 + g) * lda;
+    const double* pb = B + (long long)(n0 + g) * ldb;
+    const long long a8 = 8 * lda, b8 = 8 * ldb;
+    const double2 zero2 = make_double2(0.0, 0.0);
+    double acc[2][RN][2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) acc[r][j][0] = acc[r][j][1] = 0.0;
+    const long long step = 8LL * KU * wk_count;
+    const long long full = p0 + (p1 - p0) / (8 * KU) * (8 * KU);  // end of the whole slices
+    long long p = p0 + 8LL * KU * wk;
+    for (; p < full; p += step) {
+        double2 a[KU][2], b[KU][RN];
+#pragma unroll
+        for (int u = 0; u < KU; ++u) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) a[u][r] = 8 * r < va ? load2<AL>(pa + r * a8 + p + 8 * u + 2 * t) : zero2;
+#pragma unroll
+            for (int j = 0; j < RN; ++j) b[u][j] = 8 * j < vb ? load2<AL>(pb + j * b8 + p + 8 * u + 2 * t) : zero2;
+        }
+#pragma unroll
+        for (int u = 0; u < KU; ++u) {
+#pragma unroll
+            for (int j = 0; j < RN; ++j)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) mma_f64(acc[r][j], a[u][r].x, b[u][j].x);
+#pragma unroll
+            for (int j = 0; j < RN; ++j)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) mma_f64(acc[r][j], a[u][r].y, b[u][j].y);
+        }
+    }
+    if (p == full)  // the warp whose turn it is takes the ragged end, point by point
+        for (; p < p1; p += 4) {
+            const bool in = p + t < p1;
+            double a[2], b[RN];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) a[r] = in && 8 * r < va ? __ldg(pa + r * a8 + p + t) : 0.0;
+#pragma unroll
+            for (int j = 0; j < RN; ++j) b[j] = in && 8 * j < vb ? __ldg(pb + j * b8 + p + t) : 0.0;
+#pragma unroll
+            for (int j = 0; j < RN; ++j)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) mma_f64(acc[r][j], a[r], b[j]);
+        }
+    for (int w = 0; w < wk_count; ++w) {
+        if (wk == w)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int j = 0; j < RN; ++j) {
+                    double* c = tile + (wm * 16 + r * 8 + g) * TS + j * 8 + 2 * t;
+                    c[0] = w ? c[0] + acc[r][j][0] : acc[r][j][0];
+                    c[1] = w ? c[1] + acc[r][j][1] : acc[r][j][1];
+                }
+        __syncthreads();
+    }
+    const int nel = ka * kb;
+    double* mine = partial + (long long)blockIdx.z * nel;
+    const int rows = min(16 * wm_count, ka - m0), cols = min(8 * RN, kb - n0);
+    for (int e = threadIdx.x; e < rows * cols; e += GM_THREADS) {
+        const int i = e / cols, j = e - i * cols;
+        mine[(long long)(m0 + i) * kb + n0 + j] = tile[i * TS + j];
+    }
+    if (!ticket) return;
+    // level 1: the last block of this group of chunks adds the group's partials in chunk order
+    const int nch = (int)gridDim.z, tiles = (int)(gridDim.x * gridDim.y);
+    const int ngroups = (nch + GM_GROUP - 1) / GM_GROUP;
+    const int grp = (int)blockIdx.z / GM_GROUP, c0 = grp * GM_GROUP, csz = min(GM_GROUP, nch - c0);
+    double* gsum = partial + (long long)nch * nel;  // [ngroups][nel]
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket + 1 + grp, 1u) == (unsigned)(csz * tiles) - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int e = threadIdx.x; e < nel; e += GM_THREADS) {
+        double v[GM_GROUP];
+#pragma unroll
+        for (int c = 0; c < GM_GROUP; ++c) v[c] = c < csz ? __ldcg(partial + (long long)(c0 + c) * nel + e) : 0.0;
+        double sum = 0.0;
+#pragma unroll
+        for (int c = 0; c < GM_GROUP; ++c) sum += v[c];
+        gsum[(long long)grp * nel + e] = sum;
+    }
+    if (threadIdx.x == 0) ticket[1 + grp] = 0;  // ready for the next call
+    // level 2: the last group adds the group sums in group order
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == (unsigned)ngroups - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int e = threadIdx.x; e < nel; e += GM_THREADS) {
+        double sum = 0.0;
+        for (int q0 = 0; q0 < ngroups; q0 += 16) {
+            double v[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = q0 + q < ngroups ? __ldcg(gsum + (long long)(q0 + q) * nel + e) : 0.0;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) sum += v[q];
+        }
+        out[e] = sum * scale;
+    }
+    if (threadIdx.x == 0) *ticket = 0;
+}
+
+// out[e] = scale * sum_c partial[c][e] for wide products: 32 neighbouring elements by 8 strands of
+// chunks per block (coalesced), the strands added in order.
+__global__ void __launch_bounds__(256) gram_sum_kernel(int nch, int nel, const double* __restrict__ partial,
+                                                       double scale, double* __restrict__ out) {
+    __shared__ double sh[8][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int e = blockIdx.x * 32 + x;
+    double s = 0.0;
+    if (e < nel)
+#pragma unroll 4
+        for (int c = y; c < nch; c += 8) s += partial[(long long)c * nel + e];
+    sh[y][x] = s;
+    __syncthreads();
+    if (y == 0 && e < nel) {
+        s = sh[0][x];
+#pragma unroll
+        for (int q = 1; q < 8; ++q) s += sh[q][x];
+        out[e] = s * scale;
+    }
+}
+
+struct GramShape {
+    int wm, mt, nt;
+    long long nch, chunk;
+    size_t smem;
+};
+
+template <int RN, int KU, bool AL>
+void gram_launch(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B,
+                 long long ldb, int kb, std::vector<double>& C) {
+    // rows: the warp count along M (of 8, 4, 2, 1) that pads the fewest rows, the larger of equals
+    // (more warps share each B fragment); 207 rows: 7 tiles of 32 (8 % padding) and not 2 of 128
+    int wm = 1;
+    long long best = -1;
+    for (int w = 1; w <= 8; w *= 2) {
+        const long long padded = (ka + 16LL * w - 1) / (16 * w) * (16 * w);
+        // at least 32 rows share a wide tile's B fragments: 16 would double the reads of B
+        if (w == 1 && RN > 4 && ka > 16) continue;
+        if (best < 0 || padded <= best) best = padded, wm = w;
+    }
+    const int mt = (ka + 16 * wm - 1) / (16 * wm), nt = (kb + 8 * RN - 1) / (8 * RN);
+    const size_t smem = sizeof(double) * 16 * wm * (8 * RN + 2);
+    // one wave of blocks: as many point chunks as fit the resident blocks, none shorter than two
+    // steps of every warp
+    const long long resident = 2LL * ctx->num_sms;
+    const long long unit = 8LL * KU * (8 / wm);
+    long long nch = std::max<long long>(1, resident / ((long long)mt * nt));
+    nch = std::min(nch, std::max<long long>(1, g.N / (2 * unit)));
+    const size_t nel = (size_t)ka * kb;
+    const bool inl = nel <= GM_INLINE;
+    if (inl) nch = std::min<long long>(nch, (long long)(GM_TICKETS - 1) * GM_GROUP);
+    nch = std::min<long long>(nch, 65535);
+    long long chunk = (g.N + nch - 1) / nch;
+    chunk = (chunk + unit - 1) / unit * unit;
+    nch = (g.N + chunk - 1) / chunk;
+    const long long ngroups = inl ? (nch + GM_GROUP - 1) / GM_GROUP : 0;
+    double* partial = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * (nel * (nch + ngroups) + nel) + 64);
+    double* res = partial + nel * (nch + ngroups);
+    if (inl && !ctx->gram_ticket) {
+        DFT_CUDA(cudaMalloc(&ctx->gram_ticket, sizeof(unsigned int) * GM_TICKETS));
+        DFT_CUDA(cudaMemsetAsync(ctx->gram_ticket, 0, sizeof(unsigned int) * GM_TICKETS, ctx->stream));
+    }
+    // smem: 128 rows x 74 doubles = 74 KB at most
+    if (smem > 48 * 1024)
+        DFT_CUDA(cudaFuncSetAttribute(gram_mma_kernel<RN, KU, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(sizeof(double) * 128 * (8 * RN + 2))));
+    gram_mma_kernel<RN, KU, AL><<<dim3(mt, nt, (unsigned)nch), GM_THREADS, smem, ctx->stream>>>(
+        A, lda, ka, B, ldb, kb, g.N, chunk, wm, g.dV, partial, inl ? (unsigned int*)ctx->gram_ticket : nullptr, res);
+    DFT_LAUNCH_CHECK();
+    if (!inl) {
+        gram_sum_kernel<<<(unsigned)((nel + 31) / 32), 256, 0, ctx->stream>>>((int)nch, (int)nel, partial, g.dV, res);
+        DFT_LAUNCH_CHECK();
+    }
+    count_launch(ctx, inl ? 1 : 2);
+    double* h = pinned(ctx, nel);
+    DFT_CUDA(cudaMemcpyAsync(h, res, sizeof(double) * nel, cudaMemcpyDeviceToHost, ctx->stream));
+    sync(ctx);
+    std::memcpy(C.data(), h, sizeof(double) * nel);
+}
+
+template <bool AL>
+void gram_pick(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B, long long ldb,
+               int kb, std::vector<double>& C) {
+    // columns: tiles of at most 72, all of the same width
+    const int tiles = (kb + 71) / 72;
+    const int rn = (((kb + tiles - 1) / tiles) + 7) / 8;
+    switch (rn) {
+        case 1: gram_launch<1, 4, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 2: gram_launch<2, 2, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 3: gram_launch<3, 2, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 4: gram_launch<4, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 5: gram_launch<5, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 6: gram_launch<6, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 7: gram_launch<7, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 8: gram_launch<8, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        default: gram_launch<9, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+    }
+}
+
+// every row of the block starts 16-byte aligned
+inline bool aligned16(const void* p, long long ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 2 == 0; }
+
+}  // namespace
+
+// C (ka x kb, host, row-major) = dV * A^T B
+void gram_fp64(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B, long long ldb,
+               int kb, std::vector<double>& C) {
+    C.assign((size_t)ka * kb, 0.0);
+    if (ka == 0 || kb == 0) return;
+    if (aligned16(A, lda) && aligned16(B, ldb)) gram_pick<true>(ctx, g, A, lda, ka, B, ldb, kb, C);
+    else gram_pick<false>(ctx, g, A, lda, ka, B, ldb, kb, C);
+}
+
+namespace {
+
+// ---------------------------------------------------------------- rotation -------------
+// out_j = beta out_j + alpha sum_i in_i Y[i][j] over i < k, for 8 RJ columns j from j0 = 8 RJ blockIdx.y.
+// A warp owns 16 PP points and all 8 RJ columns, so `in` is read once; per 4 rows of `in` it loads
+// PP 16-byte pairs of points per lane and RJ fragments of Y^T from shared memory for 2 PP RJ MMAs.
+// Y^T is laid out in fragment order (conflict-free).  The two points of a pair go to two MMAs, so
+// a lane ends with four neighbouring points of one column.
+// in2: the rows k1 <= i < k come from in2 (row i - k1).  ss: when not null, sum_p out_j[p]^2 of
+// this block goes to ss[j * gridDim.x + blockIdx.x].
+// out may be rows of `in` when one column tile covers all of m (rotate_in_place): a warp has read
+// every row at its points before it writes any of them, and no other warp reads those points.
+template <int RJ, int PP, bool AL>
+__global__ void __launch_bounds__(512, 1)
+    rotate_mma_kernel(const double* in, const double* in2, long long ldi, int k1, int k,
+                      const double* __restrict__ Y, int m, double* out, long long ldo, long long n,
+                      double alpha, double beta, double* __restrict__ ss) {
+    extern __shared__ double sy[];  // ceil(k / 4) x RJ x 32
+    __shared__ double red[16][8 * RJ];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int j0 = blockIdx.y * 8 * RJ;
+    const int steps = (k + 3) / 4;
+    for (int e = threadIdx.x; e < steps * RJ * 32; e += blockDim.x) {
+        const int l = e & 31, b = (e >> 5) % RJ, s = (e >> 5) / RJ;
+        const int i = 4 * s + (l & 3), j = j0 + 8 * b + (l >> 2);
+        sy[e] = i < k && j < m ? Y[(long long)i * m + j] : 0.0;
+    }
+    __syncthreads();
+    double sq[RJ];
+#pragma unroll
+    for (int b = 0; b < RJ; ++b) sq[b] = 0.0;
+    const double2 zero2 = make_double2(0.0, 0.0);
+    const long long tiles = (n + 16 * PP - 1) / (16 * PP);
+    for (long long tile = (long long)blockIdx.x * warps + warp; tile < tiles; tile += (long long)gridDim.x * warps) {
+        const long long p0 = tile * 16 * PP;
+        const bool whole = p0 + 16 * PP <= n;
+        double acc[RJ][PP][2][2];
+#pragma unroll
+        for (int b = 0; b < RJ; ++b)
+#pragma unroll
+            for (int q = 0; q < PP; ++q) acc[b][q][0][0] = acc[b][q][0][1] = acc[b][q][1][0] = acc[b][q][1][1] = 0.0;
+        auto fetch = [&](int s, double2 (&v)[PP]) {
+            const int i = 4 * s + t;
+            const double* row = (i < k1 ? in + (long long)i * ldi : in2 + (long long)(i - k1) * ldi) + p0 + 2 * g;
+#pragma unroll
+            for (int q = 0; q < PP; ++q) {
+                if (i >= k) {
+                    v[q] = zero2;
+                } else if (whole) {
+                    v[q] = AL ? *reinterpret_cast<const double2*>(row + 16 * q)
+                              : make_double2(row[16 * q], row[16 * q + 1]);
+                } else {
+                    const long long p = p0 + 16 * q + 2 * g;
+                    v[q].x = p < n ? row[16 * q] : 0.0;
+                    v[q].y = p + 1 < n ? row[16 * q + 1] : 0.0;
+                }
+            }
+        };
+        auto product = [&](int s, const double2 (&v)[PP]) {
+            const double* a = sy + (s * RJ) * 32 + lane;
+#pragma unroll
+            for (int b = 0; b < RJ; ++b) {
+                const double y = a[b * 32];
+#pragma unroll
+                for (int q = 0; q < PP; ++q) {
+                    mma_f64(acc[b][q][0], y, v[q].x);
+                    mma_f64(acc[b][q][1], y, v[q].y);
+                }
+            }
+        };
+        // four steps (16 rows of `in`) in flight
+        int s = 0;
+        for (; s + 4 <= steps; s += 4) {
+            double2 v[4][PP];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) fetch(s + u, v[u]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) product(s + u, v[u]);
+        }
+        for (; s < steps; ++s) {
+            double2 v[PP];
+            fetch(s, v);
+            product(s, v);
+        }
+#pragma unroll
+        for (int b = 0; b < RJ; ++b) {
+            const int j = j0 + 8 * b + g;
+            if (j >= m) continue;
+#pragma unroll
+            for (int q = 0; q < PP; ++q) {
+                const long long p = p0 + 16 * q + 4 * t;
+                double* o = out + (long long)j * ldo + p;
+                double r[4] = {acc[b][q][0][0], acc[b][q][1][0], acc[b][q][0][1], acc[b][q][1][1]};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    r[c] *= alpha;
+                    if (beta != 0.0 && p + c < n) r[c] += beta * o[c];
+                    if (p + c < n) sq[b] += r[c] * r[c];
+                }
+                if (AL && whole) {
+                    reinterpret_cast<double2*>(o)[0] = make_double2(r[0], r[1]);
+                    reinterpret_cast<double2*>(o)[1] = make_double2(r[2], r[3]);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (p + c < n) o[c] = r[c];
+                }
+            }
+        }
+    }
+    if (!ss) return;
+#pragma unroll
+    for (int b = 0; b < RJ; ++b) {
+        sq[b] += __shfl_xor_sync(0xffffffffu, sq[b], 1);
+        sq[b] += __shfl_xor_sync(0xffffffffu, sq[b], 2);
+        if (t == 0) red[warp][8 * b + g] = sq[b];
+    }
+    __syncthreads();
+    if (threadIdx.x < 8 * RJ && j0 + (int)threadIdx.x < m) {
+        double v = red[0][threadIdx.x];
+        for (int w = 1; w < warps; ++w) v += red[w][threadIdx.x];
+        ss[(long long)(j0 + threadIdx.x) * gridDim.x + blockIdx.x] = v;
+    }
+}
+
+// out[r] = sum of row r of partial (one block per row, fixed order)
+__global__ void __launch_bounds__(128) row_sum_kernel(int ncols, const double* __restrict__ partial,
+                                                      double* __restrict__ out) {
+    __shared__ double sh[4];
+    double s = 0.0;
+    for (int c = threadIdx.x; c < ncols; c += 128) s += partial[(long long)blockIdx.x * ncols + c];
+    s = block_sum(s, sh);
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
+}
+
+constexpr size_t ROT_SMEM = 200 * 1024;
+
+template <int RJ, int PP, bool AL>
+unsigned rotate_launch(dft_context* ctx, const double* in, const double* in2, long long ldi, int k1, int k,
+                       const double* Y, int m, double* out, long long ldo, long long n, double alpha, double beta,
+                       double* ss) {
+    const size_t smem = sizeof(double) * (size_t)((k + 3) / 4) * RJ * 32;
+    if (smem > 32 * 1024) {  // with the 9 KB of static shared memory beyond the default limit
+        DFT_CUDA(cudaFuncSetAttribute(rotate_mma_kernel<RJ, PP, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)ROT_SMEM));
+    }
+    const int jt = (m + 8 * RJ - 1) / (8 * RJ);
+    // 16 warps per SM (the register limit): as two blocks, or as one where Y^T takes most of the
+    // shared memory
+    const int threads = smem > 90 * 1024 ? 512 : 256;
+    const long long warps_needed = (n + 16 * PP - 1) / (16 * PP);
+    const long long resident = (long long)ctx->num_sms * 512 / threads;
+    const long long bx = std::max<long long>(
+        1, std::min<long long>((warps_needed * 32 + threads - 1) / threads, (resident + jt - 1) / jt));
+    rotate_mma_kernel<RJ, PP, AL><<<dim3((unsigned)bx, jt), threads, smem, ctx->stream>>>(in, in2, ldi, k1, k, Y, m,
+                                                                                         out, ldo, n, alpha, beta, ss);
+    DFT_LAUNCH_CHECK();
+    count_launch(ctx);
+    return (unsigned)bx;
+}
+
+// most blocks along x that rotate_launch uses (the row length of ss)
+inline size_t rotate_max_blocks(dft_context* ctx) { return (size_t)ctx->num_sms * 2; }
+
+// column tiles of at most 72 whose part of Y^T fits the shared memory, all of one width
+inline int rotate_tiles(int k, int m) {
+    const long long per_block = (long long)sizeof(double) * ((k + 3) / 4) * 32;
+    const int most = (int)std::max<long long>(1, std::min<long long>(9, (long long)ROT_SMEM / per_block));
+    return ((m + 7) / 8 + most - 1) / most;
+}
+
+template <bool AL>
+unsigned rotate_pick(dft_context* ctx, const double* in, const double* in2, long long ldi, int k1, int k,
+                     const double* Y, int m, double* out, long long ldo, long long n, double alpha, double beta,
+                     double* ss) {
+    const int tiles = rotate_tiles(k, m);
+    const int rj = ((m + tiles - 1) / tiles + 7) / 8;
+#define DFT_ROT(R, P) return rotate_launch<R, P, AL>(ctx, in, in2, ldi, k1, k, Y, m, out, ldo, n, alpha, beta, ss)
+    switch (rj) {
+        case 1: DFT_ROT(1, 2);
+        case 2: DFT_ROT(2, 2);
+        case 3: DFT_ROT(3, 1);
+        case 4: DFT_ROT(4, 1);
+        case 5: DFT_ROT(5, 1);
+        case 6: DFT_ROT(6, 1);
+        case 7: DFT_ROT(7, 1);
+        case 8: DFT_ROT(8, 1);
+        default: DFT_ROT(9, 1);
+    }
+#undef DFT_ROT
+}
+
+}  // namespace
+
+bool rotate_in_place(int k, int m) { return rotate_tiles(k, m) == 1; }
+
+// out = beta*out + alpha * in * Y   (Y: k x m host row-major)
+void rotate(dft_context* ctx, const Grid& g, const double* in, long long ldi, int k, const std::vector<double>& Y, int m,
+            double* out, long long ldo, double alpha, double beta) {
+    if (m == 0) return;
+    if (k == 0) {
+        if (beta == 0.0)
+            for (int j = 0; j < m; ++j)
+                DFT_CUDA(cudaMemsetAsync(out + (long long)j * ldo, 0, sizeof(double) * (size_t)g.N, ctx->stream));
+        return;
+    }
+    if (k > 1600) fail(DFT_INVALID_ARGUMENT, "subspace too large for the rotation kernel (k=%d)", k);
+    double* dy = (double*)ws_get(ctx, WS_TMP, sizeof(double) * (size_t)k * m);
+    DFT_CUDA(cudaMemcpyAsync(dy, Y.data(), sizeof(double) * (size_t)k * m, cudaMemcpyHostToDevice, ctx->stream));
+    if (aligned16(in, ldi) && aligned16(out, ldo))
+        rotate_pick<true>(ctx, in, in, ldi, k, k, dy, m, out, ldo, g.N, alpha, beta, nullptr);
+    else
+        rotate_pick<false>(ctx, in, in, ldi, k, k, dy, m, out, ldo, g.N, alpha, beta, nullptr);
+}
+
+// R_b = sum_i AV_i Y[i][b] - theta_b sum_i V_i Y[i][b] and ss[b] = sum_p R_b[p]^2 (host; synchronises),
+// as one rotation of the 2k rows [AV; V] by [Y; -Y diag(theta)]: V Y and (AV) Y are not stored.
+void ritz_residual(dft_context* ctx, const Grid& g, const double* V, const double* AV, long long ld, int k,
+                   const std::vector<double>& Y, const double* theta, int m, double* R, double* ss_host) {
+    if (k > 1600) fail(DFT_INVALID_ARGUMENT, "subspace too large for the rotation kernel (k=%d)", k);
+    const size_t nel = (size_t)k * m;
+    std::vector<double> Z(2 * nel);
+    std::copy(Y.begin(), Y.begin() + nel, Z.begin());
+    for (int i = 0; i < k; ++i)
+        for (int b = 0; b < m; ++b) Z[nel + (size_t)i * m + b] = -theta[b] * Y[(size_t)i * m + b];
+    double* dz = (double*)ws_get(ctx, WS_TMP, sizeof(double) * 2 * nel);
+    const size_t mb = rotate_max_blocks(ctx);
+    double* part = (double*)ws_get(ctx, WS_REDUCE, sizeof(double) * (mb * m + m));
+    double* sum = part + mb * m;
+    DFT_CUDA(cudaMemcpyAsync(dz, Z.data(), sizeof(double) * 2 * nel, cudaMemcpyHostToDevice, ctx->stream));
+    const bool al = aligned16(V, ld) && aligned16(AV, ld) && aligned16(R, ld);
+    const unsigned bx = al ? rotate_pick<true>(ctx, AV, V, ld, k, 2 * k, dz, m, R, ld, g.N, 1.0, 0.0, part)
+                           : rotate_pick<false>(ctx, AV, V, ld, k, 2 * k, dz, m, R, ld, g.N, 1.0, 0.0, part);
+    row_sum_kernel<<<m, 128, 0, ctx->stream>>>((int)bx, part, sum);
+    DFT_LAUNCH_CHECK();
+    count_launch(ctx);
+    double* h = pinned(ctx, m);
+    DFT_CUDA(cudaMemcpyAsync(h, sum, sizeof(double) * m, cudaMemcpyDeviceToHost, ctx->stream));
+    sync(ctx);
+    for (int b = 0; b < m; ++b) ss_host[b] = h[b];
+}
+
+}  // namespace dftb

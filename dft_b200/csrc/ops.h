@@ -120,15 +120,20 @@ double kinetic_energy(dft_context* ctx, const Grid& g, const double* psi, int nb
 void kinetic_per_band(dft_context* ctx, const Grid& g, const double* psi, int nbands, long long ld, double* out_host);
 void nuclear_potential(dft_context* ctx, const Grid& g, int nnuc, const int* Z, const double* xyz, double* vext);
 
-// C (ka x kb, host) = dV A^T B: FP64 (davidson.cu) or on the tensor cores with a TF32 hi+lo
+// C (ka x kb, host) = dV A^T B: FP64 (dense_fp64.cu) or on the tensor cores with a TF32 hi+lo
 // split (gram_tc.cu).
-// out = beta*out + alpha * in * Y (Y: k x m host row-major), FP64 (davidson.cu)
+// out = beta*out + alpha * in * Y (Y: k x m host row-major), FP64 (dense_fp64.cu).  out may be rows
+// of `in` where rotate_in_place(k, m) says so.
+bool rotate_in_place(int k, int m);
 void rotate(dft_context* ctx, const Grid& g, const double* in, long long ldi, int k, const std::vector<double>& Y, int m,
             double* out, long long ldo, double alpha, double beta);
 // X (m bands) = V (k bands) * Y (k x m, host row-major) on the tensor cores, TF32 hi+lo split
 // (gram_tc.cu).
 void rotate_tc(dft_context* ctx, const Grid& g, const double* V, long long ldv, int k, const std::vector<double>& Y,
                int m, double* X, long long ldx);
+// R_b = sum_i AV_i Y[i][b] - theta_b sum_i V_i Y[i][b], ss_host[b] = sum_p R_b[p]^2 (dense_fp64.cu)
+void ritz_residual(dft_context* ctx, const Grid& g, const double* V, const double* AV, long long ld, int k,
+                   const std::vector<double>& Y, const double* theta, int m, double* R, double* ss_host);
 void gram_fp64(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B,
                long long ldb, int kb, std::vector<double>& C);
 void gram_tc(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B, long long ldb,
