@@ -36,11 +36,11 @@ __device__ __forceinline__ double2 load2(const double* p) {
 }
 
 // ---------------------------------------------------------------- Gram -----------------
-// A block of 8 warps (WM along the rows of A, WK = 8 / WM along the points) owns a tile of
-// WM x 16 rows and RN x 8 columns of C and one chunk of the points.  A warp walks its share of
-// the chunk 8 KU points at a time: per 8 points two A fragments and RN B fragments (one 16-byte
-// load each) feed 4 RN MMAs.  The WK partial tiles are added in shared memory in warp order; the
-// block's tile goes to partial[chunk].
+// A block of 8 warps (WM along the rows of A, 8 / WM along the points) owns a tile of row_blocks x 8
+// rows and RN x 8 columns of C and one chunk of the points.  A warp walks its share of the chunk
+// 8 KU points at a time: per 8 points up to RM A fragments and RN B fragments (one 16-byte load each)
+// feed 2 RM RN MMAs.  The partial tiles along the points are added in shared memory in warp order;
+// the block's tile goes to partial[chunk].
 //
 // The chunks' partials are added in a fixed order.  Small products (nel <= GM_INLINE) do that in the same
 // launch, in two levels: the last block to finish in a group of GM_GROUP chunks (ticket[1 + group])
@@ -50,81 +50,94 @@ constexpr int GM_GROUP = 16;
 constexpr int GM_TICKETS = 256;  // ticket words: 1 + groups
 constexpr int GM_INLINE = 1024;
 
-template <int RN, int KU, bool AL>
-__global__ void __launch_bounds__(GM_THREADS, 2)
+template <int RM, int RN>
+constexpr int gram_ku() { return RM + RN <= 3 ? 4 : RM + RN <= 6 ? 2 : 1; }
+template <int RM, int RN>
+constexpr int gram_blocks() { return RM * RN > 18 ? 1 : 2; }  // resident blocks per SM (registers)
+
+template <int RM, int RN, bool AL>
+__global__ void __launch_bounds__(GM_THREADS, (gram_blocks<RM, RN>()))
     gram_mma_kernel(const double* __restrict__ A, long long lda, int ka, const double* __restrict__ B, long long ldb,
-                    int kb, long long n, long long chunk, int wm_count, double scale, double* __restrict__ partial,
-                    unsigned int* __restrict__ ticket, double* __restrict__ out) {
-    extern __shared__ double tile[];  // (16 wm_count) x (8 RN + 2)
-    constexpr int TS = 8 * RN + 2;
+                    int kb, long long n, long long chunk, int wm_count, int row_blocks, double scale,
+                    double* __restrict__ partial, unsigned int* __restrict__ ticket, double* __restrict__ out) {
+    extern __shared__ double tile[];  // (8 row_blocks) x (8 RN + 2)
+    constexpr int TS = 8 * RN + 2, KU = gram_ku<RM, RN>();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wm = warp % wm_count, wk = warp / wm_count, wk_count = 8 / wm_count;
     const int g = lane >> 2, t = lane & 3;
-    const int m0 = blockIdx.x * 16 * wm_count, n0 = blockIdx.y * 8 * RN;
+    const int m0 = blockIdx.x * 8 * row_blocks, n0 = blockIdx.y * 8 * RN;
+    const int rb = min(row_blocks, (ka - m0 + 7) / 8);  // row blocks of this tile
+    // this warp's row blocks: [r0, r0 + nr), the remainder to the first warps
+    const int nr = rb / wm_count + (wm < rb % wm_count);
+    const int r0 = wm * (rb / wm_count) + min(wm, rb % wm_count);
     const long long p0 = (long long)blockIdx.z * chunk, p1 = min(n, p0 + chunk);
     // fragment row 8 r is read while 8 r < va (A) or vb (B); rows past the end count as zero
-    const int va = ka - (m0 + wm * 16 + g), vb = kb - (n0 + g);
-    const double* pa = A + (long long)(m0 + wm * 16 + g) * lda;
+    const int va = min(8 * nr, ka - (m0 + 8 * r0 + g)), vb = kb - (n0 + g);
+    const double* pa = A + (long long)(m0 + 8 * r0 + g) * lda;
     const double* pb = B + (long long)(n0 + g) * ldb;
     const long long a8 = 8 * lda, b8 = 8 * ldb;
     const double2 zero2 = make_double2(0.0, 0.0);
-    double acc[2][RN][2];
+    double acc[RM][RN][2];
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < RM; ++r)
 #pragma unroll
         for (int j = 0; j < RN; ++j) acc[r][j][0] = acc[r][j][1] = 0.0;
     const long long step = 8LL * KU * wk_count;
     const long long full = p0 + (p1 - p0) / (8 * KU) * (8 * KU);  // end of the whole slices
     long long p = p0 + 8LL * KU * wk;
-    for (; p < full; p += step) {
-        double2 a[KU][2], b[KU][RN];
+    if (nr > 0)
+        for (; p < full; p += step) {
+            double2 a[KU][RM], b[KU][RN];
 #pragma unroll
-        for (int u = 0; u < KU; ++u) {
+            for (int u = 0; u < KU; ++u) {
 #pragma unroll
-            for (int r = 0; r < 2; ++r) a[u][r] = 8 * r < va ? load2<AL>(pa + r * a8 + p + 8 * u + 2 * t) : zero2;
+                for (int r = 0; r < RM; ++r)
+                    a[u][r] = 8 * r < va ? load2<AL>(pa + r * a8 + p + 8 * u + 2 * t) : zero2;
 #pragma unroll
-            for (int j = 0; j < RN; ++j) b[u][j] = 8 * j < vb ? load2<AL>(pb + j * b8 + p + 8 * u + 2 * t) : zero2;
+                for (int j = 0; j < RN; ++j)
+                    b[u][j] = 8 * j < vb ? load2<AL>(pb + j * b8 + p + 8 * u + 2 * t) : zero2;
+            }
+#pragma unroll
+            for (int u = 0; u < KU; ++u)
+#pragma unroll
+                for (int r = 0; r < RM; ++r) {
+                    if (r >= nr) break;
+#pragma unroll
+                    for (int j = 0; j < RN; ++j) mma_f64(acc[r][j], a[u][r].x, b[u][j].x);
+#pragma unroll
+                    for (int j = 0; j < RN; ++j) mma_f64(acc[r][j], a[u][r].y, b[u][j].y);
+                }
         }
-#pragma unroll
-        for (int u = 0; u < KU; ++u) {
-#pragma unroll
-            for (int j = 0; j < RN; ++j)
-#pragma unroll
-                for (int r = 0; r < 2; ++r) mma_f64(acc[r][j], a[u][r].x, b[u][j].x);
-#pragma unroll
-            for (int j = 0; j < RN; ++j)
-#pragma unroll
-                for (int r = 0; r < 2; ++r) mma_f64(acc[r][j], a[u][r].y, b[u][j].y);
-        }
-    }
-    if (p == full)  // the warp whose turn it is takes the ragged end, point by point
+    if (nr > 0 && p == full)  // the warp whose turn it is takes the ragged end, four points at a time
         for (; p < p1; p += 4) {
             const bool in = p + t < p1;
-            double a[2], b[RN];
+            double a[RM], b[RN];
 #pragma unroll
-            for (int r = 0; r < 2; ++r) a[r] = in && 8 * r < va ? __ldg(pa + r * a8 + p + t) : 0.0;
+            for (int r = 0; r < RM; ++r) a[r] = in && 8 * r < va ? __ldg(pa + r * a8 + p + t) : 0.0;
 #pragma unroll
             for (int j = 0; j < RN; ++j) b[j] = in && 8 * j < vb ? __ldg(pb + j * b8 + p + t) : 0.0;
 #pragma unroll
-            for (int j = 0; j < RN; ++j)
+            for (int r = 0; r < RM; ++r)
 #pragma unroll
-                for (int r = 0; r < 2; ++r) mma_f64(acc[r][j], a[r], b[j]);
+                for (int j = 0; j < RN; ++j) mma_f64(acc[r][j], a[r], b[j]);
         }
     for (int w = 0; w < wk_count; ++w) {
         if (wk == w)
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
+            for (int r = 0; r < RM; ++r) {
+                if (r >= nr) break;
 #pragma unroll
                 for (int j = 0; j < RN; ++j) {
-                    double* c = tile + (wm * 16 + r * 8 + g) * TS + j * 8 + 2 * t;
+                    double* c = tile + ((r0 + r) * 8 + g) * TS + j * 8 + 2 * t;
                     c[0] = w ? c[0] + acc[r][j][0] : acc[r][j][0];
                     c[1] = w ? c[1] + acc[r][j][1] : acc[r][j][1];
                 }
+            }
         __syncthreads();
     }
     const int nel = ka * kb;
     double* mine = partial + (long long)blockIdx.z * nel;
-    const int rows = min(16 * wm_count, ka - m0), cols = min(8 * RN, kb - n0);
+    const int rows = min(8 * row_blocks, ka - m0), cols = min(8 * RN, kb - n0);
     for (int e = threadIdx.x; e < rows * cols; e += GM_THREADS) {
         const int i = e / cols, j = e - i * cols;
         mine[(long long)(m0 + i) * kb + n0 + j] = tile[i * TS + j];
@@ -194,30 +207,21 @@ __global__ void __launch_bounds__(256) gram_sum_kernel(int nch, int nel, const d
     }
 }
 
-struct GramShape {
-    int wm, mt, nt;
-    long long nch, chunk;
-    size_t smem;
-};
-
-template <int RN, int KU, bool AL>
+template <int RM, int RN, bool AL>
 void gram_launch(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B,
                  long long ldb, int kb, std::vector<double>& C) {
-    // rows: the warp count along M (of 8, 4, 2, 1) that pads the fewest rows, the larger of equals
-    // (more warps share each B fragment); 207 rows: 7 tiles of 32 (8 % padding) and not 2 of 128
+    constexpr int KU = gram_ku<RM, RN>();
+    // row tiles of at most 8 warps x RM blocks of 8 rows, all of one height; the fewest warps along M
+    // that hold a tile (the others split the points)
+    const int blocks = (ka + 7) / 8, mt = (blocks + 8 * RM - 1) / (8 * RM);
+    const int row_blocks = (blocks + mt - 1) / mt;
     int wm = 1;
-    long long best = -1;
-    for (int w = 1; w <= 8; w *= 2) {
-        const long long padded = (ka + 16LL * w - 1) / (16 * w) * (16 * w);
-        // at least 32 rows share a wide tile's B fragments: 16 would double the reads of B
-        if (w == 1 && RN > 4 && ka > 16) continue;
-        if (best < 0 || padded <= best) best = padded, wm = w;
-    }
-    const int mt = (ka + 16 * wm - 1) / (16 * wm), nt = (kb + 8 * RN - 1) / (8 * RN);
-    const size_t smem = sizeof(double) * 16 * wm * (8 * RN + 2);
+    while (wm * RM < row_blocks) wm *= 2;
+    const int nt = (kb + 8 * RN - 1) / (8 * RN);
+    const size_t smem = sizeof(double) * 8 * row_blocks * (8 * RN + 2);
     // one wave of blocks: as many point chunks as fit the resident blocks, none shorter than two
     // steps of every warp
-    const long long resident = 2LL * ctx->num_sms;
+    const long long resident = (long long)gram_blocks<RM, RN>() * ctx->num_sms;
     const long long unit = 8LL * KU * (8 / wm);
     long long nch = std::max<long long>(1, resident / ((long long)mt * nt));
     nch = std::min(nch, std::max<long long>(1, g.N / (2 * unit)));
@@ -235,12 +239,12 @@ void gram_launch(dft_context* ctx, const Grid& g, const double* A, long long lda
         DFT_CUDA(cudaMalloc(&ctx->gram_ticket, sizeof(unsigned int) * GM_TICKETS));
         DFT_CUDA(cudaMemsetAsync(ctx->gram_ticket, 0, sizeof(unsigned int) * GM_TICKETS, ctx->stream));
     }
-    // smem: 128 rows x 74 doubles = 74 KB at most
     if (smem > 48 * 1024)
-        DFT_CUDA(cudaFuncSetAttribute(gram_mma_kernel<RN, KU, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(sizeof(double) * 128 * (8 * RN + 2))));
-    gram_mma_kernel<RN, KU, AL><<<dim3(mt, nt, (unsigned)nch), GM_THREADS, smem, ctx->stream>>>(
-        A, lda, ka, B, ldb, kb, g.N, chunk, wm, g.dV, partial, inl ? (unsigned int*)ctx->gram_ticket : nullptr, res);
+        DFT_CUDA(cudaFuncSetAttribute(gram_mma_kernel<RM, RN, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(sizeof(double) * 64 * RM * (8 * RN + 2))));
+    gram_mma_kernel<RM, RN, AL><<<dim3(mt, nt, (unsigned)nch), GM_THREADS, smem, ctx->stream>>>(
+        A, lda, ka, B, ldb, kb, g.N, chunk, wm, row_blocks, g.dV, partial,
+        inl ? (unsigned int*)ctx->gram_ticket : nullptr, res);
     DFT_LAUNCH_CHECK();
     if (!inl) {
         gram_sum_kernel<<<(unsigned)((nel + 31) / 32), 256, 0, ctx->stream>>>((int)nch, (int)nel, partial, g.dV, res);
@@ -253,22 +257,31 @@ void gram_launch(dft_context* ctx, const Grid& g, const double* A, long long lda
     std::memcpy(C.data(), h, sizeof(double) * nel);
 }
 
+template <int RN, bool AL>
+void gram_rows(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B, long long ldb,
+               int kb, std::vector<double>& C) {
+    // blocks of 8 rows per warp: as few as one warp column can hold up to 4, which shares each B
+    // fragment best
+    if (ka <= 8) gram_launch<1, RN, AL>(ctx, g, A, lda, ka, B, ldb, kb, C);
+    else if (ka <= 16) gram_launch<2, RN, AL>(ctx, g, A, lda, ka, B, ldb, kb, C);
+    else gram_launch<4, RN, AL>(ctx, g, A, lda, ka, B, ldb, kb, C);
+}
+
 template <bool AL>
 void gram_pick(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B, long long ldb,
                int kb, std::vector<double>& C) {
     // columns: tiles of at most 72, all of the same width
     const int tiles = (kb + 71) / 72;
-    const int rn = (((kb + tiles - 1) / tiles) + 7) / 8;
-    switch (rn) {
-        case 1: gram_launch<1, 4, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
-        case 2: gram_launch<2, 2, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
-        case 3: gram_launch<3, 2, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
-        case 4: gram_launch<4, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
-        case 5: gram_launch<5, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
-        case 6: gram_launch<6, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
-        case 7: gram_launch<7, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
-        case 8: gram_launch<8, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
-        default: gram_launch<9, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+    switch ((((kb + tiles - 1) / tiles) + 7) / 8) {
+        case 1: gram_rows<1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 2: gram_rows<2, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 3: gram_rows<3, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 4: gram_rows<4, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 5: gram_rows<5, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 6: gram_rows<6, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 7: gram_rows<7, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        case 8: gram_rows<8, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
+        default: gram_rows<9, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); break;
     }
 }
 
