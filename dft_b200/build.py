@@ -29,6 +29,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 SOURCES = {
     "capi.cu": [],
     "grid_ops.cu": [],
+    "jacobi_resident.cu": [],
     "davidson.cu": [],
     "dense_fp64.cu": [],
     "scf.cu": [],

@@ -177,7 +177,8 @@ enum WsSlot {
     WS_PG3 = 22,
     WS_PG4 = 23,
     WS_TMP3 = 24,    // superposition start tables (atomic_start.cu)
-    WS_NUM = 25,     // slots in use (dft_context::ws has room for 32)
+    WS_JACOBI_RING = 25,  // exchange ring of the resident Jacobi solve
+    WS_NUM = 26,     // slots in use (dft_context::ws has room for 32)
 };
 
 void* ws_get(dft_context* ctx, int slot, size_t bytes);

@@ -1375,21 +1375,6 @@ JacobiResult hartree(dft_context* ctx, const Grid& g, const double* rho, double*
         // no interior: the reference still runs its sweep loop, finds max|dV| = 0 < tol and stops
         return {max_sweeps == 0 ? 0L : 1L, 0.0};
     }
-    // launch shape: one persistent launch on small grids (launch-latency bound), one sweep per
-    // launch otherwise; 2/4/8 select the temporally blocked kernel
-    int tmax = ctx->jacobi_sweeps_per_launch;
-    if (tmax == 0) {
-        auto t = ctx->tuned.find({(long long)g.nx, (long long)g.ny, (long long)g.nz});
-        if (t != ctx->tuned.end()) tmax = t->second[1];
-    }
-    if (tmax == 0 || tmax == -2) {
-        JacobiResult r;
-        if (hartree_cluster(ctx, g, rho, vh, tol, max_sweeps, &r)) return r;
-        if (tmax == -2) fail(DFT_INVALID_ARGUMENT, "grid does not fit the cluster-resident Jacobi");
-    }
-    if (tmax == 0) tmax = g.N <= 64LL * 64 * 64 ? -1 : 1;
-    if (tmax == -1) return hartree_persistent(ctx, g, rho, vh, buf1, tol, max_sweeps);
-    if (tmax == 2 || tmax == 4 || tmax == 8) return hartree_tb(ctx, g, rho, vh, buf1, tol, max_sweeps, tmax);
     const double den = 2.0 * (g.ix2 + g.iy2 + g.iz2);
     dim3 block(JB_X, JB_Y);
     const int bx = (g.nx + JB_X - 1) / JB_X, by = (g.ny + JB_Y - 1) / JB_Y;
@@ -1398,22 +1383,54 @@ JacobiResult hartree(dft_context* ctx, const Grid& g, const double* rho, double*
     dim3 grid(bx, by, (g.nz + zc - 1) / zc);
     JacobiCtrl* hc = (JacobiCtrl*)pinned(ctx, (sizeof(JacobiCtrl) + 7) / 8);
     long launched = 0;
-    // Sweeps are launched in batches; a launch after the stop rule fired returns at once, so
-    // a batch may overrun the stopping sweep without changing the result.
-    long batch = 32;
-    while (true) {
-        const long nb = std::min<long>(batch, max_sweeps - launched);
-        for (long s = 0; s < nb; ++s) {
+    auto sweeps_launch = [&](long nb) {
+        for (long s = 0; s < nb; ++s)
             jacobi_sweep_kernel<<<grid, block, 0, ctx->stream>>>(g, rho, vh, buf1, ctrl, den, tol, max_sweeps, zc);
-        }
         DFT_LAUNCH_CHECK();
         count_launch(ctx, nb);
         launched += nb;
         DFT_CUDA(cudaMemcpyAsync(hc, ctrl, sizeof(JacobiCtrl), cudaMemcpyDeviceToHost, ctx->stream));
         sync(ctx);
-        if (hc->done || launched >= max_sweeps) break;
-        batch = std::min<long>(batch * 2, 512);
+    };
+    // launch shape: one launch with the grid resident in shared memory where it fits, one sweep per
+    // launch otherwise; 2/4/8 select the temporally blocked kernel
+    int tmax = ctx->jacobi_sweeps_per_launch;
+    if (tmax == 0) {
+        auto t = ctx->tuned.find({(long long)g.nx, (long long)g.ny, (long long)g.nz});
+        if (t != ctx->tuned.end()) tmax = t->second[1];
     }
+    JacobiResult r;
+    if (tmax == 0 || tmax == -1) {
+        // a warm start mostly meets the stop at its first sweep (multigrid starts always do): one
+        // sweep by itself is 3 us, a resident launch with its exchange ring cleared 20
+        if (guess) {
+            sweeps_launch(1);
+            if (hc->done) {
+                DFT_CUDA(cudaMemcpyAsync(vh, buf1, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));
+                return {1L, hc->last_diff};
+            }
+        }
+        double *from = launched ? buf1 : vh, *result = nullptr;
+        if (hartree_resident(ctx, g, rho, from, launched ? vh : buf1, tol, max_sweeps - launched, &r, &result)) {
+            if (result != vh)
+                DFT_CUDA(cudaMemcpyAsync(vh, buf1, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));
+            r.sweeps += launched;
+            return r;
+        }
+        if (launched && tmax == -1) tmax = 1;  // the sweep above stays
+    }
+    if (tmax == -2) {
+        if (hartree_cluster(ctx, g, rho, vh, tol, max_sweeps, &r)) return r;
+        fail(DFT_INVALID_ARGUMENT, "grid does not fit the cluster-resident Jacobi");
+    }
+    if (tmax == 0) tmax = 1;
+    if (tmax == -1) return hartree_persistent(ctx, g, rho, vh, buf1, tol, max_sweeps);
+    if (tmax == 2 || tmax == 4 || tmax == 8) return hartree_tb(ctx, g, rho, vh, buf1, tol, max_sweeps, tmax);
+    // Sweeps are launched in batches; a launch after the stop rule fired returns at once, so
+    // a batch may overrun the stopping sweep without changing the result.
+    for (long batch = guess ? 1 : 32; launched == 0 || !(hc->done || launched >= max_sweeps);
+         batch = std::min<long>(batch * 2, 512))
+        sweeps_launch(std::min<long>(batch, max_sweeps - launched));
     const long sweeps = (long)hc->sweep;
     if (sweeps & 1) {
         DFT_CUDA(cudaMemcpyAsync(vh, buf1, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));

@@ -32,6 +32,11 @@ struct JacobiResult {
 // zero_faces: zero boundary values even where the reference's rule would give Q/|r|.
 JacobiResult hartree(dft_context* ctx, const Grid& g, const double* rho, double* vh, double tol, long max_sweeps,
                      const double* guess = nullptr, bool zero_faces = false);
+// Jacobi sweeps from `start` in one launch with the grid resident in shared memory
+// (jacobi_resident.cu); both buffers hold the faces.  *result: the buffer that holds the final
+// iterate.  False (nothing launched) where the grid does not fit.
+bool hartree_resident(dft_context* ctx, const Grid& g, const double* rho, double* start, double* other, double tol,
+                      long max_sweeps, JacobiResult* res, double** result);
 // true when every face's last node lands exactly on the bound (the reference's boundary is then zero)
 bool faces_exact(const Grid& g);
 // The same solve on the library's fixed scratch array: no device allocation (grid_ops.cu).
