@@ -30,6 +30,7 @@ SOURCES = {
     "capi.cu": [],
     "grid_ops.cu": [],
     "jacobi_resident.cu": [],
+    "mg_fused.cu": [],
     "davidson.cu": [],
     "dense_fp64.cu": [],
     "scf.cu": [],

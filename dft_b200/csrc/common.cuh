@@ -93,8 +93,8 @@ struct Workspace {
 
 }  // namespace dftb
 
-// captured multigrid cycles (poisson_start.cu), keyed by grid and buffer addresses
-using MGGraphKey = std::array<long long, 6>;
+// captured multigrid cycles (poisson_start.cu): points and spacings of the grid, workspace address, direction
+using MGGraphKey = std::array<long long, 8>;
 struct MGGraph {
     cudaGraphExec_t exec;
     long long launches;  // kernels per replay
@@ -123,7 +123,7 @@ struct dft_context {
     int* dev_status = nullptr;         // device word set by kernels whose bounded waits gave up
     int hpsi_zchunk = 0;               // H psi march length per block (0 = auto)
     int ortho_adaptive = 1;            // FP64 orthonormalisation: skip the second pass when safe (1)
-    int mg_fused_restrict = 1;         // multigrid: one-pass 3-D restriction on fine grids <= 64^3 (1)
+    int mg_fused_restrict = 1;         // Poisson multigrid: fused passes (1) or separate ones (0)
     int mg_coarsest_sor = 1;           // multigrid: red-black SOR coarsest solve (1) or Jacobi sweeps (0)
     int tc_ring = 0;                   // tensor-core Gram: cp.async ring variant (1) or register staging (0)
     int tc_tma = 0;                    // tensor-core Gram: TMA-fed FP64 ring (1; before tc_ring)

@@ -5,10 +5,12 @@
 // the same tolerance; only the number of fine-grid sweeps changes.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <random>
 #include <vector>
 
 #include "common.cuh"
+#include "mg_fused.h"
 #include "neural.h"
 #include "ops.h"
 
@@ -50,46 +52,18 @@ __global__ void restrict_axis_kernel(const double* __restrict__ in, double* __re
     }
 }
 
-// Trilinear interpolation of the coarse solution (same bounds) onto the fine interior.
-__global__ void prolong_kernel(Grid f, Grid c, const double* __restrict__ vc, double* __restrict__ out) {
-    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < f.N; p += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(p % f.nx), j = (int)((p / f.nx) % f.ny), k = (int)(p / ((long long)f.nx * f.ny));
-        const bool face = i == 0 || i + 1 == f.nx || j == 0 || j + 1 == f.ny || k == 0 || k + 1 == f.nz;
-        if (face) {
-            out[p] = 0.0;
-            continue;
-        }
-        const double u[3] = {i * f.dx / c.dx, j * f.dy / c.dy, k * f.dz / c.dz};
-        const int m[3] = {c.nx, c.ny, c.nz};
-        int I[3];
-        double w[3];
-        for (int d = 0; d < 3; ++d) {
-            I[d] = min(max((int)floor(u[d]), 0), m[d] - 2);
-            w[d] = fmin(fmax(u[d] - I[d], 0.0), 1.0);
-        }
-        double s = 0.0;
-        for (int t = 0; t < 8; ++t) {
-            const int a = t & 1, b = (t >> 1) & 1, cc = t >> 2;
-            const double wt = (a ? w[0] : 1.0 - w[0]) * (b ? w[1] : 1.0 - w[1]) * (cc ? w[2] : 1.0 - w[2]);
-            s += wt * vc[((long long)(I[2] + cc) * c.ny + (I[1] + b)) * c.nx + (I[0] + a)];
-        }
-        out[p] = s;
-    }
-}
-
-// s = max |v| (1 if zero): the network's input/output scale, kept on the device.
-__global__ void absmax_kernel(long long n, const double* __restrict__ v, double* __restrict__ s) {
-    __shared__ double sh[32];
+// *s (zeroed before) = bits of max |v|, then 1 if that is zero: the network's input/output scale, kept
+// on the device.
+__global__ void __launch_bounds__(256) absmax_kernel(long long n, const double* __restrict__ v, double* __restrict__ s) {
     double m = 0.0;
-    for (long long p = threadIdx.x; p < n; p += blockDim.x) m = fmax(m, fabs(v[p]));
+    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
+        m = fmax(m, fabs(v[p]));
     m = warp_max(m);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double r = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r = fmax(r, sh[w]);
-        *s = r > 0.0 ? r : 1.0;
-    }
+    if ((threadIdx.x & 31) == 0)
+        atomicMax(reinterpret_cast<unsigned long long*>(s), (unsigned long long)__double_as_longlong(m));
+}
+__global__ void one_if_zero_kernel(double* s) {
+    if (!(*s > 0.0)) *s = 1.0;
 }
 
 __global__ void sum_kernel(long long n, const double* __restrict__ v, double* __restrict__ out) {
@@ -145,7 +119,7 @@ Grid coarse_grid(const Grid& g) {
 // level arrays are carved from one slab of doubles.
 struct Level {
     Grid g;
-    double *t1, *t2, *rc, *vc, *vs;
+    double *t1, *t2, *rc, *vc;
 };
 
 std::vector<Level> plan_levels(const Grid& fine) {
@@ -164,7 +138,7 @@ size_t slab_doubles(const Grid& fine, const std::vector<Level>& L) {
     size_t n = 8;  // the scale s
     Grid prev = fine;
     for (const Level& l : L) {
-        n += (size_t)prev.nz * prev.ny * l.g.nx + (size_t)prev.nz * l.g.ny * l.g.nx + 3 * (size_t)l.g.N + 8;
+        n += (size_t)prev.nz * prev.ny * l.g.nx + (size_t)prev.nz * l.g.ny * l.g.nx + 2 * (size_t)l.g.N + 8;
         prev = l.g;
     }
     return n;
@@ -185,65 +159,15 @@ double* carve(double* slab, const Grid& fine, std::vector<Level>& L) {
         l.t2 = take((size_t)prev.nz * l.g.ny * l.g.nx);
         l.rc = take((size_t)l.g.N);
         l.vc = take((size_t)l.g.N);
-        l.vs = take((size_t)l.g.N);
         prev = l.g;
     }
     return s;
 }
 
-// The same restriction in one pass (small fine grids, where the three passes are three
-// launch latencies): out(I,J,K) = prod_d (h_d/H_d) sum_k w_z sum_j w_y sum_i w_x in(i,j,k).
-// hat weights of one axis: w[t] for fine index lo + t (at most RW of them; coarse spacing
-// <= 2.5 fine spacings, which coarse_points guarantees)
-constexpr int RW = 6;
-__device__ __forceinline__ int hat_weights(int I, double h, double H, int nf, double* w) {
-    const double X = I * H;
-    const int lo = max(0, (int)ceil((X - H) / h)), hi = min(nf - 1, (int)floor((X + H) / h));
-#pragma unroll
-    for (int t = 0; t < RW; ++t) {
-        const int i = lo + t;
-        const double v = i <= hi ? 1.0 - fabs(i * h - X) / H : 0.0;
-        w[t] = v > 0.0 ? v : 0.0;
-    }
-    return lo;
-}
-
-__global__ void restrict3d_kernel(const double* __restrict__ in, double* __restrict__ out, Grid f, Grid c) {
-    const double scale = (f.dx / c.dx) * (f.dy / c.dy) * (f.dz / c.dz);
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < c.N; q += (long long)gridDim.x * blockDim.x) {
-        const int I = (int)(q % c.nx), J = (int)((q / c.nx) % c.ny), K = (int)(q / ((long long)c.nx * c.ny));
-        double wx[RW], wy[RW], wz[RW];
-        const int i0 = hat_weights(I, f.dx, c.dx, f.nx, wx);
-        const int j0 = hat_weights(J, f.dy, c.dy, f.ny, wy);
-        const int k0 = hat_weights(K, f.dz, c.dz, f.nz, wz);
-        double sz = 0.0;
-#pragma unroll
-        for (int tk = 0; tk < RW; ++tk) {
-            if (wz[tk] == 0.0) continue;
-            double sy = 0.0;
-#pragma unroll
-            for (int tj = 0; tj < RW; ++tj) {
-                if (wy[tj] == 0.0) continue;
-                const double* row = in + ((long long)(k0 + tk) * f.ny + (j0 + tj)) * f.nx + i0;
-                double sx = 0.0;
-#pragma unroll
-                for (int ti = 0; ti < RW; ++ti)
-                    if (wx[ti] != 0.0) sx += wx[ti] * row[ti];
-                sy += wy[tj] * sx;
-            }
-            sz += wz[tk] * sy;
-        }
-        out[q] = sz * scale;
-    }
-}
-
 void restrict3(dft_context* ctx, const Grid& f, const Grid& c, const double* in, double* t1, double* t2,
                double* out) {
-    if (ctx->mg_fused_restrict && f.N <= 64LL * 64 * 64 && c.dx <= 2.5 * f.dx && c.dy <= 2.5 * f.dy &&
-        c.dz <= 2.5 * f.dz) {
-        restrict3d_kernel<<<blocks_for(ctx, c.N), 256, 0, ctx->stream>>>(in, out, f, c);
-        DFT_LAUNCH_CHECK();
-        count_launch(ctx);
+    if (ctx->mg_fused_restrict) {
+        mg_restrict(ctx, f, c, in, out);
         return;
     }
     restrict_axis_kernel<<<blocks_for(ctx, (long long)f.nz * f.ny * c.nx), 256, 0, ctx->stream>>>(
@@ -275,20 +199,17 @@ long coarse_solve(dft_context* ctx, double* slab, const Grid& g, const double* r
     for (int i = (int)L.size() - 1; i >= 0; --i) {
         Level& l = L[i];
         // each level from the next coarser level's interpolated solution (zero on the coarsest)
-        if (i + 1 < (int)L.size())
-            DFT_CUDA(cudaMemcpyAsync(l.vc, l.vs, sizeof(double) * (size_t)l.g.N, cudaMemcpyDeviceToDevice, ctx->stream));
-        else
+        if (i + 1 == (int)L.size())
             DFT_CUDA(cudaMemsetAsync(l.vc, 0, sizeof(double) * (size_t)l.g.N, ctx->stream));
         cycles += multigrid(ctx, l.g, l.rc, l.vc, 1e-7, 20, nullptr);
         const Grid& to = i == 0 ? g : L[i - 1].g;
-        double* dst = i == 0 ? vup : L[i - 1].vs;
-        prolong_kernel<<<blocks_for(ctx, to.N), 256, 0, ctx->stream>>>(to, l.g, l.vc, dst);
-        DFT_LAUNCH_CHECK();
-        count_launch(ctx);
+        mg_interpolate(ctx, to, l.g, l.vc, i == 0 ? vup : L[i - 1].vc);
     }
-    absmax_kernel<<<1, 1024, 0, ctx->stream>>>(L[0].g.N, L[0].vc, s);
+    DFT_CUDA(cudaMemsetAsync(s, 0, sizeof(double), ctx->stream));
+    absmax_kernel<<<blocks_for(ctx, L[0].g.N), 256, 0, ctx->stream>>>(L[0].g.N, L[0].vc, s);
+    one_if_zero_kernel<<<1, 1, 0, ctx->stream>>>(s);
     DFT_LAUNCH_CHECK();
-    count_launch(ctx);
+    count_launch(ctx, 2);
     if (s_out) *s_out = s;
     if (gc_out) *gc_out = L[0].g;
     return cycles;
@@ -325,22 +246,12 @@ __global__ void mg_smooth_kernel(Grid g, const double* __restrict__ src, double 
     }
 }
 
-// r = s*src - (den v - sum) on the interior, 0 on faces; folds max |r| into *rmax (as the
-// bits of a non-negative double) when rmax is not null
+// r = s*src - (den v - sum) on the interior, 0 on faces
 __global__ void mg_residual_kernel(Grid g, const double* __restrict__ src, double sscale, const double* __restrict__ v,
-                                   double* __restrict__ r, unsigned long long* __restrict__ rmax) {
+                                   double* __restrict__ r) {
     const double den = 2.0 * (g.ix2 + g.iy2 + g.iz2);
-    double m = 0.0;
-    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < g.N; p += (long long)gridDim.x * blockDim.x) {
-        double rr = 0.0;
-        if (!on_face(g, p)) rr = sscale * src[p] - (den * v[p] - nb_sum(g, v, p));
-        r[p] = rr;
-        m = fmax(m, fabs(rr));
-    }
-    if (rmax) {
-        m = warp_max(m);
-        if ((threadIdx.x & 31) == 0) atomicMax(rmax, (unsigned long long)__double_as_longlong(m));
-    }
+    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < g.N; p += (long long)gridDim.x * blockDim.x)
+        r[p] = on_face(g, p) ? 0.0 : sscale * src[p] - (den * v[p] - nb_sum(g, v, p));
 }
 
 // v += trilinear interpolation of the coarse correction e (interior of the fine grid)
@@ -366,61 +277,6 @@ __global__ void prolong_add_kernel(Grid f, Grid c, const double* __restrict__ e,
     }
 }
 
-// Coarsest level: `sweeps` red-black SOR sweeps (relaxation omega) from zero in one block's
-// shared memory.  With the optimal omega the error falls by omega - 1 per sweep instead of the
-// Jacobi spectral radius, so a few sweeps do what 8 Jacobi sweeps per point of the longest axis did.
-constexpr int MG_COARSEST_MAX = 12288;
-__global__ void __launch_bounds__(1024) mg_coarsest_kernel(Grid g, const double* __restrict__ src,
-                                                           double* __restrict__ e, int sweeps, double omega) {
-    extern __shared__ double sm[];
-    const int n = (int)g.N;
-    double* a = sm;
-    for (int p = threadIdx.x; p < n; p += blockDim.x) a[p] = 0.0;
-    __syncthreads();
-    const double den = 2.0 * (g.ix2 + g.iy2 + g.iz2);
-    // omega == 1: plain Jacobi sweeps (the sweep reads the previous iterate: a second array)
-    if (omega == 1.0) {
-        double* b = sm + n;
-        for (int p = threadIdx.x; p < n; p += blockDim.x) b[p] = 0.0;
-        __syncthreads();
-        for (int s = 0; s < sweeps; ++s) {
-            const double* cur = (s & 1) ? b : a;
-            double* nxt = (s & 1) ? a : b;
-            for (int p = threadIdx.x; p < n; p += blockDim.x)
-                if (!on_face(g, p)) nxt[p] = (nb_sum(g, cur, p) + src[p]) / den;
-            __syncthreads();
-        }
-        if (sweeps & 1)
-            for (int p = threadIdx.x; p < n; p += blockDim.x) a[p] = b[p];
-        __syncthreads();
-    } else {
-        for (int s = 0; s < sweeps; ++s)
-            for (int colour = 0; colour < 2; ++colour) {
-                for (int p = threadIdx.x; p < n; p += blockDim.x) {
-                    const int i = p % g.nx, j = (p / g.nx) % g.ny, k = p / (g.nx * g.ny);
-                    if (((i + j + k) & 1) != colour || on_face(g, p)) continue;
-                    const double gs = (nb_sum(g, a, p) + src[p]) / den;
-                    a[p] += omega * (gs - a[p]);
-                }
-                __syncthreads();
-            }
-    }
-    for (int p = threadIdx.x; p < n; p += blockDim.x) e[p] = a[p];
-}
-
-// Optimal SOR relaxation for the 7-point operator on grid g (from the Jacobi spectral radius
-// of the Dirichlet problem) and the sweeps that cut the error by 1e-4.
-void coarsest_sor(const Grid& g, double* omega, int* sweeps) {
-    const double pi = 3.14159265358979323846;
-    const double rj = (g.ix2 * std::cos(pi / (g.nx - 1)) + g.iy2 * std::cos(pi / (g.ny - 1)) +
-                       g.iz2 * std::cos(pi / (g.nz - 1))) /
-                      (g.ix2 + g.iy2 + g.iz2);
-    *omega = 2.0 / (1.0 + std::sqrt(std::max(0.0, 1.0 - rj * rj)));
-    const double rate = std::max(*omega - 1.0, 1e-3);
-    const int need = (int)std::ceil(std::log(1e-4) / std::log(rate));
-    *sweeps = std::min(8 * std::max({g.nx, g.ny, g.nz}), std::max(4, need));
-}
-
 inline int mg_blocks(dft_context* ctx, long long n) {
     const long long b = (n + 255) / 256;
     return (int)std::max<long long>(1, std::min<long long>(b, (long long)ctx->num_sms * 8));
@@ -430,36 +286,18 @@ inline int mg_blocks(dft_context* ctx, long long n) {
 // ---------------------------------------------------------------- multigrid solve ------
 // V(2,2) cycles with weighted Jacobi (omega = 0.8) on the nested coarse grids, the same
 // charge-conserving restriction and trilinear interpolation, and a coarsest-level red-black
-// SOR solve in one block's shared memory.  Faces of every level are held at zero (the boundary of every grid
-// whose last nodes land on the bounds).
-struct MGLevel {
-    Grid g;
-    double *src, *v, *tmp, *res, *t1, *t2;  // t1/t2: restriction temporaries towards the next level
+// SOR solve in one block's shared memory (mg_fused.cu).  Faces of every level are held at zero (the boundary of
+// every grid whose last nodes land on the bounds).  The "multigrid_fused_restriction" = 0 key takes the
+// separate passes below instead.
+struct Restriction {
+    double *t1, *t2;  // temporaries of the separate restriction passes
 };
 
-std::vector<MGLevel> mg_plan(const Grid& fine) {
-    std::vector<MGLevel> L;
-    MGLevel f{};
-    f.g = fine;
-    L.push_back(f);
-    Grid cur = fine;
-    while (cur.N > MG_COARSEST_MAX || std::min({cur.nx, cur.ny, cur.nz}) > 9) {
-        const Grid c = coarse_grid(cur);
-        if (c.nx == cur.nx && c.ny == cur.ny && c.nz == cur.nz) break;
-        MGLevel l{};
-        l.g = c;
-        L.push_back(l);
-        cur = c;
-        if (L.size() >= 10) break;
-    }
-    return L;
-}
-
 size_t mg_doubles(const std::vector<MGLevel>& L) {
-    size_t n = 16;
+    size_t n = 16 + sizeof(MGHistory) / sizeof(double) + 6 * ((size_t)L[0].g.N + 2);
     for (size_t i = 0; i < L.size(); ++i) {
         const Grid& g = L[i].g;
-        n += 4 * ((size_t)g.N + 2);
+        if (i > 0) n += 4 * ((size_t)g.N + 2);
         if (i + 1 < L.size()) {
             const Grid& c = L[i + 1].g;
             n += (size_t)g.nz * g.ny * c.nx + (size_t)g.nz * c.ny * c.nx + 4;
@@ -468,57 +306,30 @@ size_t mg_doubles(const std::vector<MGLevel>& L) {
     return n;
 }
 
-void mg_carve(double* slab, std::vector<MGLevel>& L) {
-    double* p = slab + 16;
-    auto take = [&](size_t n) {
-        double* q = p;
-        p += (n + 1) / 2 * 2;
-        return q;
-    };
-    for (size_t i = 0; i < L.size(); ++i) {
-        const Grid& g = L[i].g;
-        L[i].src = i == 0 ? nullptr : take((size_t)g.N);
-        L[i].v = i == 0 ? nullptr : take((size_t)g.N);
-        L[i].tmp = take((size_t)g.N);
-        L[i].res = take((size_t)g.N);
-        if (i + 1 < L.size()) {
-            const Grid& c = L[i + 1].g;
-            L[i].t1 = take((size_t)g.nz * g.ny * c.nx);
-            L[i].t2 = take((size_t)g.nz * c.ny * c.nx);
-        }
-    }
-}
-
-void mg_smooth(dft_context* ctx, MGLevel& l, double sscale, int n) {
-    for (int s = 0; s < n; ++s) {
-        mg_smooth_kernel<<<mg_blocks(ctx, l.g.N), 256, 0, ctx->stream>>>(l.g, l.src, sscale, l.v, l.tmp, 0.8);
-        std::swap(l.v, l.tmp);
-    }
-    count_launch(ctx, n);
-}
-
-void vcycle(dft_context* ctx, std::vector<MGLevel>& L, size_t i, double sscale) {
+// One cycle by separate passes below and at level i: v -> v (tmp, res scratch)
+void separate_cycle(dft_context* ctx, std::vector<MGLevel>& L, std::vector<Restriction>& T, std::vector<double*>& res,
+                    size_t i, double sscale, double* v, double* tmp) {
     MGLevel& l = L[i];
-    if (i + 1 == L.size()) {
-        const size_t sm = sizeof(double) * 2 * (size_t)l.g.N;
-        double omega = 1.0;
-        int sweeps = 8 * std::max({l.g.nx, l.g.ny, l.g.nz});
-        if (ctx->mg_coarsest_sor) coarsest_sor(l.g, &omega, &sweeps);
-        mg_coarsest_kernel<<<1, 1024, sm, ctx->stream>>>(l.g, l.src, l.v, sweeps, omega);
-        DFT_LAUNCH_CHECK();
+    auto smooth = [&](const double* from, double* to) {
+        mg_smooth_kernel<<<mg_blocks(ctx, l.g.N), 256, 0, ctx->stream>>>(l.g, l.src, sscale, from, to, 0.8);
         count_launch(ctx);
-        return;
-    }
-    mg_smooth(ctx, l, sscale, 2);
-    mg_residual_kernel<<<mg_blocks(ctx, l.g.N), 256, 0, ctx->stream>>>(l.g, l.src, sscale, l.v, l.res, nullptr);
+    };
+    smooth(v, tmp);
+    smooth(tmp, v);
+    mg_residual_kernel<<<mg_blocks(ctx, l.g.N), 256, 0, ctx->stream>>>(l.g, l.src, sscale, v, res[i]);
     count_launch(ctx);
     MGLevel& c = L[i + 1];
-    restrict3(ctx, l.g, c.g, l.res, l.t1, l.t2, c.src);
-    DFT_CUDA(cudaMemsetAsync(c.v, 0, sizeof(double) * (size_t)c.g.N, ctx->stream));
-    vcycle(ctx, L, i + 1, 1.0);
-    prolong_add_kernel<<<mg_blocks(ctx, l.g.N), 256, 0, ctx->stream>>>(l.g, c.g, c.v, l.v);
+    restrict3(ctx, l.g, c.g, res[i], T[i].t1, T[i].t2, c.src);
+    if (i + 2 == L.size()) {
+        mg_coarsest_solve(ctx, c, c.src, ctx->mg_coarsest_sor != 0);
+    } else {
+        DFT_CUDA(cudaMemsetAsync(c.v, 0, sizeof(double) * (size_t)c.g.N, ctx->stream));
+        separate_cycle(ctx, L, T, res, i + 1, 1.0, c.v, c.tmp);
+    }
+    prolong_add_kernel<<<mg_blocks(ctx, l.g.N), 256, 0, ctx->stream>>>(l.g, c.g, c.v, v);
     count_launch(ctx);
-    mg_smooth(ctx, l, sscale, 2);
+    smooth(v, tmp);
+    smooth(tmp, v);
     DFT_LAUNCH_CHECK();
 }
 
@@ -532,92 +343,170 @@ long coarse_start(dft_context* ctx, double* slab, const Grid& g, const double* r
 
 int multigrid(dft_context* ctx, const Grid& g, const double* rho, double* v, double tol, int max_cycles,
               double* resid_out) {
-    std::vector<MGLevel> L = mg_plan(g);
+    std::vector<MGLevel> L = mg_levels(g);
     if (L.back().g.N > MG_COARSEST_MAX) fail(DFT_INVALID_ARGUMENT, "grid too small or too anisotropic for multigrid");
     double* slab = (double*)ws_get(ctx, WS_PG1, sizeof(double) * mg_doubles(L));
-    mg_carve(slab, L);
-    static bool attr = false;
-    if (!attr) {
-        DFT_CUDA(cudaFuncSetAttribute(mg_coarsest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(sizeof(double) * 2 * MG_COARSEST_MAX)));
-        attr = true;
+    double* next = slab + 16;
+    auto take = [&](size_t n) {
+        double* q = next;
+        next += (n + 1) / 2 * 2;  // keep 16-byte alignment
+        return q;
+    };
+    MGHistory* hist = (MGHistory*)take(sizeof(MGHistory) / sizeof(double));
+    // The solve runs on its own copies: the captured cycles below then depend on the grid alone.
+    // Cycles alternate between buf[0] and buf[1], so the last two iterates are at hand.
+    const size_t N = (size_t)g.N, bytes = sizeof(double) * N;
+    double* rhs = take(N);
+    double* buf[2] = {take(N), take(N)};
+    double *tmp = take(N), *tmp2 = take(N), *saved = take(N);
+    std::vector<Restriction> T(L.size());
+    std::vector<double*> res(L.size(), tmp2);
+    L[0].src = rhs;
+    for (size_t i = 0; i < L.size(); ++i) {
+        if (i > 0) {
+            L[i].src = take((size_t)L[i].g.N);
+            L[i].v = take((size_t)L[i].g.N);
+            L[i].tmp = take((size_t)L[i].g.N);
+            res[i] = take((size_t)L[i].g.N);
+        }
+        if (i + 1 < L.size()) {
+            T[i].t1 = take((size_t)L[i].g.nz * L[i].g.ny * L[i + 1].g.nx);
+            T[i].t2 = take((size_t)L[i].g.nz * L[i + 1].g.ny * L[i + 1].g.nx);
+        }
     }
-    // the fine level works in place on v (its faces must hold the boundary values); rho is
-    // its source, scaled by 4 pi
-    L[0].src = const_cast<double*>(rho);
-    L[0].v = v;
-    unsigned long long* rmax = (unsigned long long*)(slab + 8);
+    DFT_CUDA(cudaMemcpyAsync(rhs, rho, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    DFT_CUDA(cudaMemcpyAsync(buf[0], v, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    DFT_CUDA(cudaMemsetAsync(hist, 0, sizeof(MGHistory), ctx->stream));
     const double den = 2.0 * (g.ix2 + g.iy2 + g.iz2);
     const double fourpi = 4.0 * 3.14159265358979323846;
-    // one cycle: the V-cycle, then the residual's max norm into rmax
-    auto cycle = [&] {
-        vcycle(ctx, L, 0, fourpi);
-        if (L[0].v != v) {  // an odd number of smoothing swaps left the iterate in the temporary
-            DFT_CUDA(cudaMemcpyAsync(v, L[0].v, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));
-            L[0].tmp = L[0].v;
-            L[0].v = v;
-        }
-        DFT_CUDA(cudaMemsetAsync(rmax, 0, 8, ctx->stream));
-        mg_residual_kernel<<<mg_blocks(ctx, g.N), 256, 0, ctx->stream>>>(g, rho, fourpi, v, L[0].res, rmax);
-        DFT_LAUNCH_CHECK();
-        count_launch(ctx);
-    };
-    // The cycle's launch sequence is the same every time for this grid and these buffers: it
-    // is captured once as a CUDA graph and replayed (one launch instead of ~10 per level).
-    // A capture that fails for any reason leaves the direct launches in place.
-    cudaGraphExec_t exec = nullptr;
-    long long per_replay = 0;
-    if (ctx->multigrid_graphs) {
-        const MGGraphKey key{g.nx, g.ny, g.nz, (long long)(uintptr_t)slab, (long long)(uintptr_t)rho,
-                             (long long)(uintptr_t)v};
-        auto it = ctx->mg_graphs.find(key);
-        if (it != ctx->mg_graphs.end()) {
-            exec = it->second.exec;
-            per_replay = it->second.launches;
+    const bool sor = ctx->mg_coarsest_sor != 0;
+    // one cycle in -> out (in is kept), then the residual's max norm into the history
+    auto cycle = [&](const double* in, double* out) {
+        if (L.size() == 1) {
+            mg_start_cycle(ctx, hist);
+            L[0].v = out;
+            mg_coarsest_solve(ctx, L[0], rhs, sor);
+        } else if (ctx->mg_fused_restrict) {
+            double* a = mg_fused_level(g.N) ? tmp : out;
+            double* b = mg_fused_level(g.N) ? tmp2 : tmp;
+            mg_smooth_step(ctx, L[0], rhs, nullptr, in, a, 0, fourpi, nullptr, 1);
+            mg_smooth_step(ctx, L[0], rhs, nullptr, a, b, 0, fourpi, nullptr, 1);
+            mg_residual_restrict(ctx, L[0], L[1], rhs, nullptr, b, 0, fourpi, nullptr, 1, hist);
+            mg_cycle_from_zero(ctx, L, 1, L[1].src, nullptr, 0, 1.0, nullptr, 1, sor);
+            mg_correct_smooth(ctx, L[0], L[1], rhs, nullptr, b, tmp2, out, 0, fourpi, nullptr, 1);
         } else {
+            mg_start_cycle(ctx, hist);
+            DFT_CUDA(cudaMemcpyAsync(out, in, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+            separate_cycle(ctx, L, T, res, 0, fourpi, out, tmp);
+        }
+        mg_residual_max(ctx, g, rhs, fourpi, out, hist);
+    };
+    // The cycle's launch sequence is the same every time for this grid: each direction is captured once
+    // as a CUDA graph and replayed.  A capture that fails for any reason leaves the direct launches
+    // in place.
+    cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    long long per_replay[2] = {0, 0};
+    if (ctx->multigrid_graphs && L.size() > 1) {
+        auto bits = [](double x) {
+            long long b;
+            std::memcpy(&b, &x, sizeof b);
+            return b;
+        };
+        for (int w = 0; w < 2; ++w) {
+            const MGGraphKey key{g.nx, g.ny, g.nz, bits(g.dx), bits(g.dy), bits(g.dz), (long long)(uintptr_t)slab, w};
+            auto it = ctx->mg_graphs.find(key);
+            if (it != ctx->mg_graphs.end()) {
+                exec[w] = it->second.exec;
+                per_replay[w] = it->second.launches;
+                continue;
+            }
             const long long l0 = ctx->launches;
             cudaGraph_t graph = nullptr;
             bool captured = false;
             if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
                 try {
-                    cycle();
+                    cycle(buf[w], buf[1 - w]);
+                    captured = true;
                 } catch (const Error&) {
                 }
-                captured = cudaStreamEndCapture(ctx->stream, &graph) == cudaSuccess && graph != nullptr;
+                captured = cudaStreamEndCapture(ctx->stream, &graph) == cudaSuccess && graph != nullptr && captured;
             }
             cudaGetLastError();  // a failed capture leaves no sticky error; clear the last one
-            per_replay = ctx->launches - l0;
+            per_replay[w] = ctx->launches - l0;
             ctx->launches = l0;
-            if (captured && L[0].v == v && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
-                if (ctx->mg_graphs.size() >= 16) {  // keep a handful: the buffers of the current solves
-                    cudaGraphExecDestroy(ctx->mg_graphs.begin()->second.exec);
-                    ctx->mg_graphs.erase(ctx->mg_graphs.begin());
-                }
-                ctx->mg_graphs[key] = {exec, per_replay};
+            if (captured && cudaGraphInstantiate(&exec[w], graph, 0) == cudaSuccess) {
+                ctx->mg_graphs[key] = {exec[w], per_replay[w]};
             } else {
-                exec = nullptr;
+                exec[w] = nullptr;
                 cudaGetLastError();
             }
             if (graph) cudaGraphDestroy(graph);
         }
-    }
-    double* h = pinned(ctx, 1);
-    int c = 0;
-    double r = 0.0;
-    for (c = 1; c <= max_cycles; ++c) {
-        if (exec) {
-            DFT_CUDA(cudaGraphLaunch(exec, ctx->stream));
-            count_launch(ctx, per_replay);
-        } else {
-            cycle();
+        // keep a handful: the levels of the current solves (a graph just replayed may still be running)
+        if (ctx->mg_graphs.size() > 32) {
+            sync(ctx);
+            for (auto it = ctx->mg_graphs.begin(); it != ctx->mg_graphs.end() && ctx->mg_graphs.size() > 16;) {
+                if (it->second.exec == exec[0] || it->second.exec == exec[1]) {
+                    ++it;
+                    continue;
+                }
+                cudaGraphExecDestroy(it->second.exec);
+                it = ctx->mg_graphs.erase(it);
+            }
         }
-        DFT_CUDA(cudaMemcpyAsync(h, rmax, 8, cudaMemcpyDeviceToHost, ctx->stream));
-        sync(ctx);
-        r = h[0] / den;  // the size of the next Jacobi update
-        if (r < tol) break;
     }
+    int cur = 0;  // the buffer of the current iterate
+    auto run = [&](int m) {
+        for (int q = 0; q < m; ++q) {
+            if (exec[cur]) {
+                DFT_CUDA(cudaGraphLaunch(exec[cur], ctx->stream));
+                count_launch(ctx, per_replay[cur]);
+            } else {
+                cycle(buf[cur], buf[1 - cur]);
+            }
+            cur = 1 - cur;
+        }
+    };
+    MGHistory* h = (MGHistory*)pinned(ctx, sizeof(MGHistory) / sizeof(double));
+    int c = 0;
+    double r = 0.0, before = 0.0;
+    bool met = false;
+    // The count is that of a solve which looks at every cycle's residual.  The residual falls by a
+    // steady factor, so after two cycles the ones that cannot be the last yet by that factor are launched together
+    // (a host round trip is about 10 us, a cycle at 48^3 about 30); the history then shows the first one
+    // that met the tolerance.
+    while (c < max_cycles && !met) {
+        int m = 1;
+        if (c >= 2 && r < before && r > tol && tol > 0.0)
+            m = (int)std::max(1.0, std::min(16.0, std::floor(std::log(tol / r) / std::log(r / before))));
+        m = std::min(m, max_cycles - c);
+        if (m >= 3) DFT_CUDA(cudaMemcpyAsync(saved, buf[cur], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        const int from = cur;
+        run(m);
+        DFT_CUDA(cudaMemcpyAsync(h, hist, sizeof(MGHistory), cudaMemcpyDeviceToHost, ctx->stream));
+        sync(ctx);
+        for (int q = 1; q <= m && !met; ++q) {
+            before = r;
+            std::memcpy(&r, &h->r[(c + q) & 63], sizeof r);
+            r /= den;  // the size of the next Jacobi update
+            if (!(r < tol)) continue;
+            met = true;
+            if (q == m - 1) {
+                cur = 1 - cur;  // the last cycle was one too many: the iterate before it
+            } else if (q < m) {
+                DFT_CUDA(cudaMemcpyAsync(buf[from], saved, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+                cur = from;
+                run(q);
+            }
+            m = q;
+        }
+        c += m;
+        // a single level is solved from zero: every further cycle would repeat this one
+        if (L.size() == 1 && !met) c = max_cycles;
+    }
+    if (c > 0) DFT_CUDA(cudaMemcpyAsync(v, buf[cur], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     if (resid_out) *resid_out = r;
-    return std::min(c, max_cycles);
+    return c;
 }
 
 void poisson_start(dft_context* ctx, dft_pnet* net, const Grid& g, const double* rho, double* out, int cycles,
