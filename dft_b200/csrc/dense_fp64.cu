@@ -42,13 +42,57 @@ __device__ __forceinline__ double2 load2(const double* p) {
 // feed 2 RM RN MMAs.  The partial tiles along the points are added in shared memory in warp order;
 // the block's tile goes to partial[chunk].
 //
-// The chunks' partials are added in a fixed order.  Small products (nel <= GM_INLINE) do that in the same
-// launch, in two levels: the last block to finish in a group of GM_GROUP chunks (ticket[1 + group])
-// adds the group's partials, the last group (ticket[0]) adds the group sums and writes dV C.
+// Small products (nel <= GM_INLINE) add the chunks' partials in the same launch (gram_finish).
 constexpr int GM_THREADS = 256;
 constexpr int GM_GROUP = 16;
 constexpr int GM_TICKETS = 256;  // ticket words: 1 + groups
 constexpr int GM_INLINE = 1024;
+
+// The partials of nch chunks (partial[chunk], each of them `tiles` arrivals) are added in a fixed order by the
+// same launch, in two levels: the last arrival of a group of GM_GROUP chunks (ticket[1 + group]) adds the
+// group's partials, the last group (ticket[0]) adds the group sums and writes scale * C.  Called by
+// whole thread blocks with the chunk `at` they have just written.
+__device__ __forceinline__ void gram_finish(int nel, int tiles, int nch, int at, double* partial, double scale,
+                                            unsigned int* ticket, double* out) {
+    const int ngroups = (nch + GM_GROUP - 1) / GM_GROUP;
+    const int grp = at / GM_GROUP, c0 = grp * GM_GROUP, csz = min(GM_GROUP, nch - c0);
+    double* gsum = partial + (long long)nch * nel;  // [ngroups][nel]
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket + 1 + grp, 1u) == (unsigned)(csz * tiles) - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int e = threadIdx.x; e < nel; e += blockDim.x) {
+        double v[GM_GROUP];
+#pragma unroll
+        for (int c = 0; c < GM_GROUP; ++c) v[c] = c < csz ? __ldcg(partial + (long long)(c0 + c) * nel + e) : 0.0;
+        double sum = 0.0;
+#pragma unroll
+        for (int c = 0; c < GM_GROUP; ++c) sum += v[c];
+        gsum[(long long)grp * nel + e] = sum;
+    }
+    if (threadIdx.x == 0) ticket[1 + grp] = 0;  // ready for the next call
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == (unsigned)ngroups - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int e = threadIdx.x; e < nel; e += blockDim.x) {
+        double sum = 0.0;
+        for (int q0 = 0; q0 < ngroups; q0 += 16) {
+            double v[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = q0 + q < ngroups ? __ldcg(gsum + (long long)(q0 + q) * nel + e) : 0.0;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) sum += v[q];
+        }
+        out[e] = sum * scale;
+    }
+    if (threadIdx.x == 0) *ticket = 0;
+}
 
 template <int RM, int RN>
 constexpr int gram_ku() { return RM + RN <= 3 ? 4 : RM + RN <= 6 ? 2 : 1; }
@@ -142,48 +186,8 @@ __global__ void __launch_bounds__(GM_THREADS, (gram_blocks<RM, RN>()))
         const int i = e / cols, j = e - i * cols;
         mine[(long long)(m0 + i) * kb + n0 + j] = tile[i * TS + j];
     }
-    if (!ticket) return;
-    // level 1: the last block of this group of chunks adds the group's partials in chunk order
-    const int nch = (int)gridDim.z, tiles = (int)(gridDim.x * gridDim.y);
-    const int ngroups = (nch + GM_GROUP - 1) / GM_GROUP;
-    const int grp = (int)blockIdx.z / GM_GROUP, c0 = grp * GM_GROUP, csz = min(GM_GROUP, nch - c0);
-    double* gsum = partial + (long long)nch * nel;  // [ngroups][nel]
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ticket + 1 + grp, 1u) == (unsigned)(csz * tiles) - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int e = threadIdx.x; e < nel; e += GM_THREADS) {
-        double v[GM_GROUP];
-#pragma unroll
-        for (int c = 0; c < GM_GROUP; ++c) v[c] = c < csz ? __ldcg(partial + (long long)(c0 + c) * nel + e) : 0.0;
-        double sum = 0.0;
-#pragma unroll
-        for (int c = 0; c < GM_GROUP; ++c) sum += v[c];
-        gsum[(long long)grp * nel + e] = sum;
-    }
-    if (threadIdx.x == 0) ticket[1 + grp] = 0;  // ready for the next call
-    // level 2: the last group adds the group sums in group order
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == (unsigned)ngroups - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int e = threadIdx.x; e < nel; e += GM_THREADS) {
-        double sum = 0.0;
-        for (int q0 = 0; q0 < ngroups; q0 += 16) {
-            double v[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = q0 + q < ngroups ? __ldcg(gsum + (long long)(q0 + q) * nel + e) : 0.0;
-#pragma unroll
-            for (int q = 0; q < 16; ++q) sum += v[q];
-        }
-        out[e] = sum * scale;
-    }
-    if (threadIdx.x == 0) *ticket = 0;
+    if (ticket)
+        gram_finish(nel, (int)(gridDim.x * gridDim.y), (int)gridDim.z, (int)blockIdx.z, partial, scale, ticket, out);
 }
 
 // out[e] = scale * sum_c partial[c][e] for wide products: 32 neighbouring elements by 8 strands of
@@ -205,6 +209,284 @@ __global__ void __launch_bounds__(256) gram_sum_kernel(int nch, int nel, const d
         for (int q = 1; q < 8; ++q) s += sh[q][x];
         out[e] = s * scale;
     }
+}
+
+// ---------------------------------------------------------------- ordered Gram ---------
+// Blocks of up to 64 x 16 (the eigensolver of a small molecule) keep a fixed order of summation, so that
+// nothing downstream that turns on the last bit (the sign of an eigenvector of the projected
+// matrix) depends on how the work is split.  An MMA adds its four products one after the
+// other like four FMAs, so a chain of MMAs along the points is the scalar chain, bit for bit; each
+// element is a set of such chains, added in a fixed tree.
+//
+// gram_lanes_kernel (kb <= 4, 8 or 16 with ka <= 64, 64, 32): the points are dealt to nblk blocks of 32
+// chains; chain (b, l) takes the points 32 b + l + 32 m nblk.  The 32 chains of block b are added as a
+// butterfly (xor 16, 8, 4, 2, 1), then the blocks in order, GM_GROUP at a time.  A thread block works
+// through its blocks b in turn; four m of 32 points and all rows are staged ahead in shared memory by
+// cp.async (reading fragments straight from global memory costs 32 L1 lookups per load, one per
+// row and m: 50 us for 24 x 12 at 64^3).  A warp runs two chains for all RB x CB tiles.  The 272-byte pitch of
+// a staged 256-byte segment makes the 16-byte fragment reads free of bank conflicts.
+// 64^3, 24 x 12: 93 us with one FMA per lane and product, 36 us here.
+constexpr int GL_PITCH = 272;  // bytes per staged segment (row, m)
+
+__device__ __forceinline__ void stage(void* dst, const void* src, bool wide, int bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if (wide) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
+template <int RB, int CB>
+struct LanesShape {
+    static constexpr int ROWS = 8 * (RB + CB), STAGE = ROWS * 4 * GL_PITCH, SUM = 16 * RB * CB * 64 * 8;
+    static constexpr int S = (220 * 1024 - SUM) / STAGE >= 4 ? 4 : (220 * 1024 - SUM) / STAGE;  // stages in flight
+    static constexpr size_t SMEM = (size_t)S * STAGE + SUM;
+};
+
+template <int RB, int CB, bool AL>
+__global__ void __launch_bounds__(512, 1)
+    gram_lanes_kernel(const double* __restrict__ A, long long lda, int ka, const double* __restrict__ B, long long ldb,
+                      int kb, long long n, int nblk, double* __restrict__ partial) {
+    using Shape = LanesShape<RB, CB>;
+    extern __shared__ __align__(16) char stages[];  // S x (8 (RB + CB) rows) x 4 m; then the butterfly's sums
+    constexpr int TILES = RB * CB, ROWS = Shape::ROWS, STAGE = Shape::STAGE, S = Shape::S;
+    double* sum = reinterpret_cast<double*>(stages + S * STAGE);  // 8 warps x 2 chains x TILES x 64
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const long long stride = (long long)nblk * 32;
+    const int steps = (int)((n + 4 * stride - 1) / (4 * stride));  // per block b (the last ones may be empty)
+    const int nb = ((int)blockIdx.x < nblk) ? (nblk - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int total = nb * steps;
+    // stage q of this thread block: step q % steps of its block number q / steps
+    auto fill = [&](int q) {
+        if (q < total) {
+            const int b = (int)blockIdx.x + q / steps * (int)gridDim.x, s = q % steps;
+            char* to = stages + q % S * STAGE;
+            constexpr int PER = AL ? 16 : 32;  // copies per segment
+            for (int e = threadIdx.x; e < ROWS * 4 * PER; e += 512) {
+                const int c = e % PER, m = e / PER & 3, row = e / (4 * PER);
+                const bool of_a = row < 8 * RB;
+                const int r = of_a ? row : row - 8 * RB;
+                const bool real = r < (of_a ? ka : kb);
+                const double* base = of_a ? A + (long long)(real ? r : 0) * lda : B + (long long)(real ? r : 0) * ldb;
+                const long long p = (long long)b * 32 + (4 * s + m) * stride + c * (AL ? 2 : 1);
+                const int in = !real || p >= n ? 0 : AL ? (p + 1 < n ? 16 : 8) : 8;
+                stage(to + (row * 4 + m) * GL_PITCH + c * (AL ? 16 : 8), in ? base + p : base, AL, in);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double acc[2][TILES][2];
+    for (int q = 0; q < S - 1; ++q) fill(q);
+    for (int q = 0; q < total; ++q) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+        __syncthreads();  // stage q has landed, and everyone is done with stage q - 1
+        fill(q + S - 1);
+        if (q % steps == 0)
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int x = 0; x < TILES; ++x) acc[c][x][0] = acc[c][x][1] = 0.0;
+        const char* from = stages + q % S * STAGE + warp * 16;
+        double2 a[RB], b[CB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+            a[r] = *reinterpret_cast<const double2*>(from + ((8 * r + g) * 4 + t) * GL_PITCH);
+#pragma unroll
+        for (int j = 0; j < CB; ++j)
+            b[j] = *reinterpret_cast<const double2*>(from + ((8 * (RB + j) + g) * 4 + t) * GL_PITCH);
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+#pragma unroll
+            for (int j = 0; j < CB; ++j) {
+                mma_f64(acc[0][r * CB + j], a[r].x, b[j].x);
+                mma_f64(acc[1][r * CB + j], a[r].y, b[j].y);
+            }
+        if (q % steps != steps - 1) continue;
+        // butterfly over the block's 32 chains: chain 2 w + c is in warp w
+#pragma unroll
+        for (int half = 8; half >= 1; half >>= 1) {
+            if (warp >= half && warp < 2 * half) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int x = 0; x < TILES; ++x)
+                        reinterpret_cast<double2*>(sum)[(((warp - half) * 2 + c) * TILES + x) * 32 + lane] =
+                            make_double2(acc[c][x][0], acc[c][x][1]);
+            }
+            __syncthreads();
+            if (warp < half) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int x = 0; x < TILES; ++x) {
+                        const double2 o = reinterpret_cast<double2*>(sum)[((warp * 2 + c) * TILES + x) * 32 + lane];
+                        acc[c][x][0] += o.x;
+                        acc[c][x][1] += o.y;
+                    }
+            }
+            __syncthreads();
+        }
+        const int nel = ka * kb, blk = (int)blockIdx.x + q / steps * (int)gridDim.x;
+        if (warp == 0) {
+            double* mine = partial + (long long)blk * nel;
+#pragma unroll
+            for (int r = 0; r < RB; ++r)
+#pragma unroll
+                for (int j = 0; j < CB; ++j)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int i = 8 * r + g, k = 8 * j + 2 * t + h;
+                        if (i < ka && k < kb) mine[i * kb + k] = acc[0][r * CB + j][h] + acc[1][r * CB + j][h];
+                    }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// out[e] = scale * the blocks' partials, added GM_GROUP blocks at a time in block order, then the groups in order
+constexpr int GL_GROUPS = 64;  // at most 64 x 16 blocks
+__global__ void __launch_bounds__(8 * GL_GROUPS) gram_lanes_sum_kernel(int nblk, int nel,
+                                                                       const double* __restrict__ partial, double scale,
+                                                                       double* __restrict__ out) {
+    __shared__ double sh[GL_GROUPS][8];
+    const int e = blockIdx.x * 8 + threadIdx.x, grp = threadIdx.y, groups = blockDim.y;
+    if (e < nel) {
+        double v[GM_GROUP];
+#pragma unroll
+        for (int c = 0; c < GM_GROUP; ++c)
+            v[c] = grp * GM_GROUP + c < nblk ? __ldg(partial + (long long)(grp * GM_GROUP + c) * nel + e) : 0.0;
+        double sum = 0.0;
+#pragma unroll
+        for (int c = 0; c < GM_GROUP; ++c) sum += v[c];
+        sh[grp][threadIdx.x] = sum;
+    }
+    __syncthreads();
+    if (grp || e >= nel) return;
+    double sum = 0.0;
+    for (int q = 0; q < groups; ++q) sum += sh[q][threadIdx.x];
+    out[e] = sum * scale;
+}
+
+// gram_chunk_kernel (the other blocks up to 64 x 16): one chain per chunk of the points and element.  Warp w
+// owns row tile w; a chunk's points in order, 4 per MMA, eight steps of loads in flight.
+template <int CB>
+__global__ void __launch_bounds__(256, 2)
+    gram_chunk_kernel(const double* __restrict__ A, long long lda, int ka, const double* __restrict__ B, long long ldb,
+                      int kb, long long n, long long chunk, double* __restrict__ partial) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const long long p0 = (long long)blockIdx.x * chunk, p1 = min(n, p0 + chunk);
+    const int i = 8 * warp + g, vb = kb - g;
+    const double* pa = A + (long long)(i < ka ? i : 0) * lda;
+    const double* pb = B + (long long)g * ldb;
+    double acc[CB][2];
+#pragma unroll
+    for (int j = 0; j < CB; ++j) acc[j][0] = acc[j][1] = 0.0;
+    constexpr int U = 8;
+    for (long long p = p0; p < p1; p += 4 * U) {
+        double a[U], b[U][CB];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const long long q = p + 4 * u + t;
+            a[u] = q < p1 && i < ka ? __ldg(pa + q) : 0.0;
+#pragma unroll
+            for (int j = 0; j < CB; ++j) b[u][j] = q < p1 && 8 * j < vb ? __ldg(pb + 8 * j * ldb + q) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int j = 0; j < CB; ++j) mma_f64(acc[j], a[u], b[u][j]);
+    }
+    double* mine = partial + (long long)blockIdx.x * ka * kb;
+#pragma unroll
+    for (int j = 0; j < CB; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = 8 * j + 2 * t + h;
+            if (i < ka && k < kb) mine[i * kb + k] = acc[j][h];
+        }
+}
+
+// out[e] = scale * sum_c partial[c][e]: one warp per element, lanes stride the chunks, butterfly
+__global__ void __launch_bounds__(256) gram_chunk_sum_kernel(int nch, int nel, const double* __restrict__ partial,
+                                                             double scale, double* __restrict__ out) {
+    const int lane = threadIdx.x & 31, e = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (e >= nel) return;
+    double s = 0.0;
+#pragma unroll 4
+    for (int c = lane; c < nch; c += 32) s += partial[(long long)c * nel + e];
+    s = warp_sum(s);
+    if (lane == 0) out[e] = s * scale;
+}
+
+unsigned int* gram_tickets(dft_context* ctx) {
+    if (!ctx->gram_ticket) {
+        DFT_CUDA(cudaMalloc(&ctx->gram_ticket, sizeof(unsigned int) * GM_TICKETS));
+        DFT_CUDA(cudaMemsetAsync(ctx->gram_ticket, 0, sizeof(unsigned int) * GM_TICKETS, ctx->stream));
+    }
+    return (unsigned int*)ctx->gram_ticket;
+}
+
+void gram_to_host(dft_context* ctx, const double* res, size_t nel, std::vector<double>& C) {
+    double* h = pinned(ctx, nel);
+    DFT_CUDA(cudaMemcpyAsync(h, res, sizeof(double) * nel, cudaMemcpyDeviceToHost, ctx->stream));
+    sync(ctx);
+    std::memcpy(C.data(), h, sizeof(double) * nel);
+}
+
+template <int RB, int CB, bool AL>
+void gram_lanes(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B, long long ldb,
+                int kb, std::vector<double>& C) {
+    const size_t nel = (size_t)ka * kb;
+    const int nblk = (int)std::max<long long>(
+        1, std::min<long long>(std::min(4LL * ctx->num_sms, (long long)GL_GROUPS * GM_GROUP), (g.N + 255) / 256));
+    const int ngroups = (nblk + GM_GROUP - 1) / GM_GROUP;
+    double* partial = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * (nel * nblk + nel));
+    double* res = partial + nel * nblk;
+    constexpr size_t smem = LanesShape<RB, CB>::SMEM;
+    DFT_CUDA(cudaFuncSetAttribute(gram_lanes_kernel<RB, CB, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    gram_lanes_kernel<RB, CB, AL><<<std::min(nblk, ctx->num_sms), 512, smem, ctx->stream>>>(
+        A, lda, ka, B, ldb, kb, g.N, nblk, partial);
+    DFT_LAUNCH_CHECK();
+    gram_lanes_sum_kernel<<<(unsigned)((nel + 7) / 8), dim3(8, ngroups), 0, ctx->stream>>>(nblk, (int)nel, partial, g.dV,
+                                                                                            res);
+    DFT_LAUNCH_CHECK();
+    count_launch(ctx, 2);
+    gram_to_host(ctx, res, nel, C);
+}
+
+// ka <= 64 and kb <= 16
+template <bool AL>
+void gram_ordered(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B,
+                  long long ldb, int kb, std::vector<double>& C) {
+    // the row counts and column widths at which the order changes
+    const int rows = ka <= 8 ? 1 : ka <= 16 ? 2 : ka <= 32 ? 4 : 8, cols = kb <= 4 ? 4 : kb <= 8 ? 8 : 16;
+    if (rows * cols <= 64) {
+        switch (rows * 10 + (cols + 7) / 8) {
+            case 11: gram_lanes<1, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); return;
+            case 12: gram_lanes<1, 2, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); return;
+            case 21: gram_lanes<2, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); return;
+            case 22: gram_lanes<2, 2, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); return;
+            case 41: gram_lanes<4, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); return;
+            case 42: gram_lanes<4, 2, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); return;
+            default: gram_lanes<8, 1, AL>(ctx, g, A, lda, ka, B, ldb, kb, C); return;
+        }
+    }
+    const size_t nel = (size_t)ka * kb;
+    const int tiles = (ka + 31) / 32;
+    long long nch = std::max<long long>(1, 4LL * ctx->num_sms / tiles);
+    long long chunk = ((g.N + nch - 1) / nch + 31) / 32 * 32;
+    nch = std::min<long long>((g.N + chunk - 1) / chunk, 65535);
+    chunk = (g.N + nch - 1) / nch;
+    double* partial = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * (nel * nch + nel));
+    double* res = partial + nel * nch;
+    const int threads = 32 * ((ka + 7) / 8);
+    if (kb <= 8)
+        gram_chunk_kernel<1><<<(unsigned)nch, threads, 0, ctx->stream>>>(A, lda, ka, B, ldb, kb, g.N, chunk, partial);
+    else
+        gram_chunk_kernel<2><<<(unsigned)nch, threads, 0, ctx->stream>>>(A, lda, ka, B, ldb, kb, g.N, chunk, partial);
+    DFT_LAUNCH_CHECK();
+    gram_chunk_sum_kernel<<<(unsigned)((nel + 7) / 8), 256, 0, ctx->stream>>>((int)nch, (int)nel, partial, g.dV, res);
+    DFT_LAUNCH_CHECK();
+    count_launch(ctx, 2);
+    gram_to_host(ctx, res, nel, C);
 }
 
 template <int RM, int RN, bool AL>
@@ -235,26 +517,19 @@ void gram_launch(dft_context* ctx, const Grid& g, const double* A, long long lda
     const long long ngroups = inl ? (nch + GM_GROUP - 1) / GM_GROUP : 0;
     double* partial = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * (nel * (nch + ngroups) + nel) + 64);
     double* res = partial + nel * (nch + ngroups);
-    if (inl && !ctx->gram_ticket) {
-        DFT_CUDA(cudaMalloc(&ctx->gram_ticket, sizeof(unsigned int) * GM_TICKETS));
-        DFT_CUDA(cudaMemsetAsync(ctx->gram_ticket, 0, sizeof(unsigned int) * GM_TICKETS, ctx->stream));
-    }
     if (smem > 48 * 1024)
         DFT_CUDA(cudaFuncSetAttribute(gram_mma_kernel<RM, RN, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)(sizeof(double) * 64 * RM * (8 * RN + 2))));
     gram_mma_kernel<RM, RN, AL><<<dim3(mt, nt, (unsigned)nch), GM_THREADS, smem, ctx->stream>>>(
         A, lda, ka, B, ldb, kb, g.N, chunk, wm, row_blocks, g.dV, partial,
-        inl ? (unsigned int*)ctx->gram_ticket : nullptr, res);
+        inl ? gram_tickets(ctx) : nullptr, res);
     DFT_LAUNCH_CHECK();
     if (!inl) {
         gram_sum_kernel<<<(unsigned)((nel + 31) / 32), 256, 0, ctx->stream>>>((int)nch, (int)nel, partial, g.dV, res);
         DFT_LAUNCH_CHECK();
     }
     count_launch(ctx, inl ? 1 : 2);
-    double* h = pinned(ctx, nel);
-    DFT_CUDA(cudaMemcpyAsync(h, res, sizeof(double) * nel, cudaMemcpyDeviceToHost, ctx->stream));
-    sync(ctx);
-    std::memcpy(C.data(), h, sizeof(double) * nel);
+    gram_to_host(ctx, res, nel, C);
 }
 
 template <int RN, bool AL>
@@ -270,6 +545,10 @@ void gram_rows(dft_context* ctx, const Grid& g, const double* A, long long lda, 
 template <bool AL>
 void gram_pick(dft_context* ctx, const Grid& g, const double* A, long long lda, int ka, const double* B, long long ldb,
                int kb, std::vector<double>& C) {
+    if (ka <= 64 && kb <= 16) {
+        gram_ordered<AL>(ctx, g, A, lda, ka, B, ldb, kb, C);
+        return;
+    }
     // columns: tiles of at most 72, all of the same width
     const int tiles = (kb + 71) / 72;
     switch ((((kb + tiles - 1) / tiles) + 7) / 8) {
@@ -425,6 +704,122 @@ __global__ void __launch_bounds__(512, 1)
     }
 }
 
+// R_b = sum_i AV_i Y[i][b] - theta_b sum_i V_i Y[i][b], the two sums kept apart and rounded once each as
+// if (AV) Y and V Y had been formed; layout and ss as in rotate_mma_kernel.
+template <int RJ, int PP, bool AL>
+__global__ void __launch_bounds__(512, 1)
+    residual_mma_kernel(const double* __restrict__ AV, const double* __restrict__ V, long long ld, int k,
+                        const double* __restrict__ Y, const double* __restrict__ theta, int m, double* __restrict__ R,
+                        long long n, double* __restrict__ ss) {
+    extern __shared__ double sy[];  // ceil(k / 4) x RJ x 32
+    __shared__ double red[16][8 * RJ];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int steps = (k + 3) / 4;
+    for (int e = threadIdx.x; e < steps * RJ * 32; e += blockDim.x) {
+        const int l = e & 31, b = (e >> 5) % RJ, s = (e >> 5) / RJ;
+        const int i = 4 * s + (l & 3), j = 8 * b + (l >> 2);
+        sy[e] = i < k && j < m ? Y[(long long)i * m + j] : 0.0;
+    }
+    __syncthreads();
+    double sq[RJ], th[RJ];
+#pragma unroll
+    for (int b = 0; b < RJ; ++b) {
+        sq[b] = 0.0;
+        th[b] = 8 * b + g < m ? theta[8 * b + g] : 0.0;
+    }
+    const long long tiles = (n + 16 * PP - 1) / (16 * PP);
+    for (long long tile = (long long)blockIdx.x * warps + warp; tile < tiles; tile += (long long)gridDim.x * warps) {
+        const long long p0 = tile * 16 * PP;
+        const bool whole = p0 + 16 * PP <= n;
+        double acc[2][RJ][PP][2][2];  // AV, V
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+#pragma unroll
+            for (int b = 0; b < RJ; ++b)
+#pragma unroll
+                for (int q = 0; q < PP; ++q)
+                    acc[f][b][q][0][0] = acc[f][b][q][0][1] = acc[f][b][q][1][0] = acc[f][b][q][1][1] = 0.0;
+        auto fetch = [&](const double* F, int s, double2 (&v)[PP]) {
+            const int i = 4 * s + t;
+            const double* row = F + (long long)i * ld + p0 + 2 * g;
+#pragma unroll
+            for (int q = 0; q < PP; ++q) {
+                if (i >= k) {
+                    v[q] = make_double2(0.0, 0.0);
+                } else if (whole) {
+                    v[q] = load2<AL>(row + 16 * q);
+                } else {
+                    const long long p = p0 + 16 * q + 2 * g;
+                    v[q].x = p < n ? __ldg(row + 16 * q) : 0.0;
+                    v[q].y = p + 1 < n ? __ldg(row + 16 * q + 1) : 0.0;
+                }
+            }
+        };
+        constexpr int U = 2;
+        for (int s = 0; s < steps; s += U) {
+            double2 v[U][2][PP];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                fetch(AV, s + u, v[u][0]);
+                fetch(V, s + u, v[u][1]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (s + u >= steps) break;
+                const double* a = sy + ((s + u) * RJ) * 32 + lane;
+#pragma unroll
+                for (int b = 0; b < RJ; ++b) {
+                    const double y = a[b * 32];
+#pragma unroll
+                    for (int f = 0; f < 2; ++f)
+#pragma unroll
+                        for (int q = 0; q < PP; ++q) {
+                            mma_f64(acc[f][b][q][0], y, v[u][f][q].x);
+                            mma_f64(acc[f][b][q][1], y, v[u][f][q].y);
+                        }
+                }
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < RJ; ++b) {
+            const int j = 8 * b + g;
+            if (j >= m) continue;
+#pragma unroll
+            for (int q = 0; q < PP; ++q) {
+                const long long p = p0 + 16 * q + 4 * t;
+                double* o = R + (long long)j * ld + p;
+                double r[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    r[c] = fma(-th[b], acc[1][b][q][c & 1][c >> 1], acc[0][b][q][c & 1][c >> 1]);
+                    if (p + c < n) sq[b] += r[c] * r[c];
+                }
+                if (AL && whole) {
+                    reinterpret_cast<double2*>(o)[0] = make_double2(r[0], r[1]);
+                    reinterpret_cast<double2*>(o)[1] = make_double2(r[2], r[3]);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (p + c < n) o[c] = r[c];
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < RJ; ++b) {
+        sq[b] += __shfl_xor_sync(0xffffffffu, sq[b], 1);
+        sq[b] += __shfl_xor_sync(0xffffffffu, sq[b], 2);
+        if (t == 0) red[warp][8 * b + g] = sq[b];
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < min(8 * RJ, m)) {
+        double v = red[0][threadIdx.x];
+        for (int w = 1; w < warps; ++w) v += red[w][threadIdx.x];
+        ss[(long long)threadIdx.x * gridDim.x + blockIdx.x] = v;
+    }
+}
+
 // out[r] = sum of row r of partial (one block per row, fixed order)
 __global__ void __launch_bounds__(128) row_sum_kernel(int ncols, const double* __restrict__ partial,
                                                       double* __restrict__ out) {
@@ -515,24 +910,65 @@ void rotate(dft_context* ctx, const Grid& g, const double* in, long long ldi, in
         rotate_pick<false>(ctx, in, in, ldi, k, k, dy, m, out, ldo, g.N, alpha, beta, nullptr);
 }
 
-// R_b = sum_i AV_i Y[i][b] - theta_b sum_i V_i Y[i][b] and ss[b] = sum_p R_b[p]^2 (host; synchronises),
-// as one rotation of the 2k rows [AV; V] by [Y; -Y diag(theta)]: V Y and (AV) Y are not stored.
+namespace {
+
+template <int RJ, int PP, bool AL>
+unsigned residual_launch(dft_context* ctx, const double* AV, const double* V, long long ld, int k, const double* Y,
+                         const double* theta, int m, double* R, long long n, double* ss) {
+    const size_t smem = sizeof(double) * (size_t)((k + 3) / 4) * RJ * 32;
+    if (smem > 32 * 1024)
+        DFT_CUDA(cudaFuncSetAttribute(residual_mma_kernel<RJ, PP, AL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)ROT_SMEM));
+    const int threads = smem > 90 * 1024 ? 512 : 256;
+    const long long warps_needed = (n + 16 * PP - 1) / (16 * PP), resident = (long long)ctx->num_sms * 512 / threads;
+    const long long bx = std::max<long long>(1, std::min<long long>((warps_needed * 32 + threads - 1) / threads, resident));
+    residual_mma_kernel<RJ, PP, AL><<<(unsigned)bx, threads, smem, ctx->stream>>>(AV, V, ld, k, Y, theta, m, R, n, ss);
+    DFT_LAUNCH_CHECK();
+    count_launch(ctx);
+    return (unsigned)bx;
+}
+
+template <bool AL>
+unsigned residual_pick(dft_context* ctx, const double* AV, const double* V, long long ld, int k, const double* Y,
+                       const double* theta, int m, double* R, long long n, double* ss) {
+    switch ((m + 7) / 8) {
+        case 1: return residual_launch<1, 2, AL>(ctx, AV, V, ld, k, Y, theta, m, R, n, ss);
+        case 2: return residual_launch<2, 1, AL>(ctx, AV, V, ld, k, Y, theta, m, R, n, ss);
+        case 3: return residual_launch<3, 1, AL>(ctx, AV, V, ld, k, Y, theta, m, R, n, ss);
+        default: return residual_launch<4, 1, AL>(ctx, AV, V, ld, k, Y, theta, m, R, n, ss);
+    }
+}
+
+}  // namespace
+
+// R_b = sum_i AV_i Y[i][b] - theta_b sum_i V_i Y[i][b] and ss[b] = sum_p R_b[p]^2 (host; synchronises):
+// V Y and (AV) Y are not stored.  Up to 32 columns keep the two sums apart; wider blocks, whose
+// accumulators would not fit, run as one rotation of the 2k rows [AV; V] by [Y; -Y diag(theta)].
 void ritz_residual(dft_context* ctx, const Grid& g, const double* V, const double* AV, long long ld, int k,
                    const std::vector<double>& Y, const double* theta, int m, double* R, double* ss_host) {
     if (k > 1600) fail(DFT_INVALID_ARGUMENT, "subspace too large for the rotation kernel (k=%d)", k);
     const size_t nel = (size_t)k * m;
-    std::vector<double> Z(2 * nel);
+    const bool apart = m <= 32 && rotate_tiles(k, m) == 1;
+    std::vector<double> Z(apart ? nel + m : 2 * nel);
     std::copy(Y.begin(), Y.begin() + nel, Z.begin());
-    for (int i = 0; i < k; ++i)
-        for (int b = 0; b < m; ++b) Z[nel + (size_t)i * m + b] = -theta[b] * Y[(size_t)i * m + b];
-    double* dz = (double*)ws_get(ctx, WS_TMP, sizeof(double) * 2 * nel);
+    if (apart)
+        std::copy(theta, theta + m, Z.begin() + nel);
+    else
+        for (int i = 0; i < k; ++i)
+            for (int b = 0; b < m; ++b) Z[nel + (size_t)i * m + b] = -theta[b] * Y[(size_t)i * m + b];
+    double* dz = (double*)ws_get(ctx, WS_TMP, sizeof(double) * Z.size());
     const size_t mb = rotate_max_blocks(ctx);
     double* part = (double*)ws_get(ctx, WS_REDUCE, sizeof(double) * (mb * m + m));
     double* sum = part + mb * m;
-    DFT_CUDA(cudaMemcpyAsync(dz, Z.data(), sizeof(double) * 2 * nel, cudaMemcpyHostToDevice, ctx->stream));
+    DFT_CUDA(cudaMemcpyAsync(dz, Z.data(), sizeof(double) * Z.size(), cudaMemcpyHostToDevice, ctx->stream));
     const bool al = aligned16(V, ld) && aligned16(AV, ld) && aligned16(R, ld);
-    const unsigned bx = al ? rotate_pick<true>(ctx, AV, V, ld, k, 2 * k, dz, m, R, ld, g.N, 1.0, 0.0, part)
-                           : rotate_pick<false>(ctx, AV, V, ld, k, 2 * k, dz, m, R, ld, g.N, 1.0, 0.0, part);
+    unsigned bx;
+    if (apart)
+        bx = al ? residual_pick<true>(ctx, AV, V, ld, k, dz, dz + nel, m, R, g.N, part)
+                : residual_pick<false>(ctx, AV, V, ld, k, dz, dz + nel, m, R, g.N, part);
+    else
+        bx = al ? rotate_pick<true>(ctx, AV, V, ld, k, 2 * k, dz, m, R, ld, g.N, 1.0, 0.0, part)
+                : rotate_pick<false>(ctx, AV, V, ld, k, 2 * k, dz, m, R, ld, g.N, 1.0, 0.0, part);
     row_sum_kernel<<<m, 128, 0, ctx->stream>>>((int)bx, part, sum);
     DFT_LAUNCH_CHECK();
     count_launch(ctx);

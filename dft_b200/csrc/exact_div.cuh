@@ -6,8 +6,8 @@
 // one FMA and RN(q + r zh) is the correctly rounded quotient (Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  Four dependent FP64
 // operations instead of the 126 cycles measured for a general division.  Both theorems assume that
-// nothing under- or overflows: numerators outside [2^-899, 2^900) and zeros take the general division,
-// as does every numerator when the divisor itself is outside [2^-100, 2^100].
+// nothing under- or overflows: numerators outside [2^-899, 2^900) take the general division, as does
+// every numerator when the divisor is not in [2^-100, 2^100].
 #pragma once
 
 #include <cmath>
@@ -19,25 +19,28 @@ struct ExactDiv {
     int general;  // 1: the divisor is out of range, always divide
 };
 
+#ifdef __CUDACC__
+__host__ __device__
+#endif
 inline ExactDiv exact_div(double b) {
     ExactDiv d{b, 0.0, 0.0, 1};
-    const double a = std::fabs(b);
-    if (a >= 0x1p-100 && a <= 0x1p100) {
+    if (b >= 0x1p-100 && b <= 0x1p100) {
         d.zh = 1.0 / b;
-        d.zl = std::fma(-b, d.zh, 1.0) / b;  // 1 - b zh is exact
+        d.zl = fma(-b, d.zh, 1.0) / b;  // 1 - b zh is exact
         d.general = 0;
     }
     return d;
 }
 
 #ifdef __CUDACC__
-// the quotient for numerators in range; bad: outside it (the value is then not used)
+// the quotient for zero and for numerators in range; bad: others (the value is then not used)
 __device__ __forceinline__ double divide_fast(double a, const ExactDiv& d, bool& bad) {
-    const unsigned e = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu;
-    bad = e - 124u >= 1800u;
+    const unsigned hi = (unsigned)__double2hiint(a), e = (hi >> 20) & 0x7ffu;
+    const bool zero = ((hi & 0x7fffffffu) | (unsigned)__double2loint(a)) == 0;
+    bad = e - 124u >= 1800u && !zero;
     const double q = __fma_rn(a, d.zh, __dmul_rn(a, d.zl));
     const double r = __fma_rn(-d.b, q, a);
-    return __fma_rn(r, d.zh, q);
+    return zero ? a : __fma_rn(r, d.zh, q);  // b is positive
 }
 __device__ __forceinline__ double divide(double a, const ExactDiv& d) {
     bool bad;

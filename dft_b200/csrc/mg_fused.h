@@ -1,4 +1,4 @@
-// Fused multigrid passes shared by the Poisson cycles (poisson_start.cu) and the eigensolver's
+// Multigrid passes shared by the Poisson cycles (poisson_start.cu) and the eigensolver's
 // preconditioner (precond_mg.cu): weighted-Jacobi V(2,2) on nested grids with the same bounds.
 //
 // Per level the equation is d v_p - sum_nb w v_nb = s src_p with d = 2 (ix2 + iy2 + iz2) + shift_a and
@@ -15,10 +15,20 @@ namespace dftb {
 constexpr double MG_OMEGA = 0.8;
 constexpr int MG_COARSEST_MAX = 12288;  // most points of the coarsest level
 
+// Per axis point of the next coarser level, x then y then z: five restriction weights from fine point
+// lo on; per axis point of this level: interpolation weight and cell.
+struct MGTable {
+    const double* w;
+    const int* lo;
+    const double* iw;
+    const int* ic;
+};
+
 struct MGLevel {
     Grid g;
-    long long ld;                      // field stride of this level's arrays
-    double *src, *v, *tmp;             // coarse levels: right-hand side, iterate, scratch
+    long long ld;           // field stride of this level's arrays
+    double *src, *v, *tmp;  // coarse levels: right-hand side, iterate, scratch
+    MGTable table;          // towards the next coarser level
 };
 
 // The nested grids from g down to the coarsest (array pointers unset, ld = N).
@@ -31,24 +41,18 @@ struct MGHistory {
     unsigned long long count;
 };
 
-// c.src = R(s src - (d v - sum w v)): residual and restriction (transposed trilinear weights) in one pass.
-// hist: when given, starts the next cycle's word there.
-void mg_residual_restrict(dft_context* ctx, const MGLevel& f, const MGLevel& c, const double* src, const int* map,
-                          const double* v, int open, double s, const double* shift, int nb,
-                          MGHistory* hist);
-// out = R(in): the restriction alone
-void mg_restrict(dft_context* ctx, const Grid& f, const Grid& c, const double* in, double* out);
-// out = one weighted-Jacobi step from v
-void mg_smooth_step(dft_context* ctx, const MGLevel& f, const double* src, const int* map, const double* v, double* out,
-                    int open, double s, const double* shift, int nb);
-// One V(2,2) cycle below and at level i from a zero start on every level: L[i].src -> L[i].v (map: field
-// a of level i reads row map[a] of src).  Level i's v and tmp may be swapped; the result is in v.
-void mg_cycle_from_zero(dft_context* ctx, std::vector<MGLevel>& L, size_t i, const double* src, const int* map, int open,
-                        double s, const double* shift, int nb, bool sor);
-// v = (v2 + P e) smoothed twice: out, by way of tmp where the level is large (returns with the result
-// in out)
-void mg_correct_smooth(dft_context* ctx, const MGLevel& f, const MGLevel& c, const double* src, const int* map,
-                       const double* v, double* tmp, double* out, int open, double s, const double* shift, int nb);
+// One V(2,2) cycle at level i: L[i].v = cycle(from) for the right-hand side s src, from zero when
+// from == nullptr (from is kept; it must not be L[i].v or L[i].tmp).  map: field a reads row map[a]
+// of src.  sor: the coarsest level (fixed faces, one field) by red-black SOR instead of Jacobi sweeps.
+// hist: when given, its next cycle's word is the maximum over the unknowns of |s src - (d v - sum w v)|
+// after the cycle (one field).
+void mg_cycle(dft_context* ctx, std::vector<MGLevel>& L, size_t i, const double* src, const int* map, const double* from,
+              int open, double s, const double* shift, int nb, bool sor, MGHistory* hist);
+// out = R(in): the restriction alone (transposed trilinear weights; needs f.table)
+void mg_restrict(dft_context* ctx, const MGLevel& f, const Grid& c, const double* in, double* out);
+// The levels' transfer tables into slab (mg_table_doubles), one launch.
+size_t mg_table_doubles(const std::vector<MGLevel>& L);
+void mg_tables(dft_context* ctx, std::vector<MGLevel>& L, double* slab);
 // out = P e on the interior, 0 on the faces
 void mg_interpolate(dft_context* ctx, const Grid& f, const Grid& c, const double* e, double* out);
 // starts the next cycle's word of hist by itself
@@ -57,10 +61,5 @@ void mg_start_cycle(dft_context* ctx, MGHistory* hist);
 void mg_residual_max(dft_context* ctx, const Grid& g, const double* src, double s, const double* v, MGHistory* hist);
 // L.back().v = the coarsest level's solution for its src by red-black SOR, or by Jacobi sweeps
 void mg_coarsest_solve(dft_context* ctx, const MGLevel& l, const double* src, bool sor);
-// the same by Jacobi sweeps for nb open fields (map, s, shift as above)
-void mg_coarsest_fields(dft_context* ctx, const MGLevel& l, const double* src, const int* map, double s,
-                        const double* shift, int nb);
-// whether a level of n points in all its fields takes the long tile passes
-bool mg_fused_level(long long n);
 
 }  // namespace dftb

@@ -139,13 +139,15 @@ size_t slab_doubles(const Grid& fine, const std::vector<Level>& L) {
     Grid prev = fine;
     for (const Level& l : L) {
         n += (size_t)prev.nz * prev.ny * l.g.nx + (size_t)prev.nz * l.g.ny * l.g.nx + 2 * (size_t)l.g.N + 8;
+        // the transfer table between prev and l
+        n += 6 * (size_t)(l.g.nx + l.g.ny + l.g.nz) + 2 * (size_t)(prev.nx + prev.ny + prev.nz) + 4;
         prev = l.g;
     }
     return n;
 }
 
-// Carves the level arrays; returns the scale slot.
-double* carve(double* slab, const Grid& fine, std::vector<Level>& L) {
+// Carves the level arrays and the place of the transfer tables; returns the scale slot.
+double* carve(double* slab, const Grid& fine, std::vector<Level>& L, double** tables) {
     double* s = slab;
     double* p = slab + 8;
     Grid prev = fine;
@@ -161,15 +163,12 @@ double* carve(double* slab, const Grid& fine, std::vector<Level>& L) {
         l.vc = take((size_t)l.g.N);
         prev = l.g;
     }
+    *tables = p;
     return s;
 }
 
 void restrict3(dft_context* ctx, const Grid& f, const Grid& c, const double* in, double* t1, double* t2,
                double* out) {
-    if (ctx->mg_fused_restrict) {
-        mg_restrict(ctx, f, c, in, out);
-        return;
-    }
     restrict_axis_kernel<<<blocks_for(ctx, (long long)f.nz * f.ny * c.nx), 256, 0, ctx->stream>>>(
         in, t1, f.nx, f.ny, f.nz, 0, c.nx, f.dx, c.dx);
     restrict_axis_kernel<<<blocks_for(ctx, (long long)f.nz * c.ny * c.nx), 256, 0, ctx->stream>>>(
@@ -185,12 +184,26 @@ void restrict3(dft_context* ctx, const Grid& f, const Grid& c, const double* in,
 long coarse_solve(dft_context* ctx, double* slab, const Grid& g, const double* rho, double* vup, double** s_out,
                   Grid* gc_out) {
     std::vector<Level> L = plan_levels(g);
-    double* s = carve(slab, g, L);
+    double* tables;
+    double* s = carve(slab, g, L, &tables);
     const bool zero = faces_exact(g);  // the coarse boundary follows the fine grid's
     const double* src = rho;
     Grid sg = g;
-    for (Level& l : L) {
-        restrict3(ctx, sg, l.g, src, l.t1, l.t2, l.rc);
+    std::vector<MGLevel> nest;  // g and the levels, with their transfer tables
+    MGLevel m{};
+    m.g = g;
+    m.ld = g.N;
+    nest.push_back(m);
+    for (const Level& l : L) {
+        m.g = l.g;
+        m.ld = l.g.N;
+        nest.push_back(m);
+    }
+    if (ctx->mg_fused_restrict) mg_tables(ctx, nest, tables);
+    for (size_t i = 0; i < L.size(); ++i) {
+        Level& l = L[i];
+        if (ctx->mg_fused_restrict) mg_restrict(ctx, nest[i], l.g, src, l.rc);
+        else restrict3(ctx, sg, l.g, src, l.t1, l.t2, l.rc);
         src = l.rc;
         sg = l.g;
     }
@@ -294,7 +307,7 @@ struct Restriction {
 };
 
 size_t mg_doubles(const std::vector<MGLevel>& L) {
-    size_t n = 16 + sizeof(MGHistory) / sizeof(double) + 6 * ((size_t)L[0].g.N + 2);
+    size_t n = 16 + sizeof(MGHistory) / sizeof(double) + mg_table_doubles(L) + 2 + 6 * ((size_t)L[0].g.N + 2);
     for (size_t i = 0; i < L.size(); ++i) {
         const Grid& g = L[i].g;
         if (i > 0) n += 4 * ((size_t)g.N + 2);
@@ -353,6 +366,7 @@ int multigrid(dft_context* ctx, const Grid& g, const double* rho, double* v, dou
         return q;
     };
     MGHistory* hist = (MGHistory*)take(sizeof(MGHistory) / sizeof(double));
+    mg_tables(ctx, L, take(mg_table_doubles(L)));
     // The solve runs on its own copies: the captured cycles below then depend on the grid alone.
     // Cycles alternate between buf[0] and buf[1], so the last two iterates are at hand.
     const size_t N = (size_t)g.N, bytes = sizeof(double) * N;
@@ -362,6 +376,7 @@ int multigrid(dft_context* ctx, const Grid& g, const double* rho, double* v, dou
     std::vector<Restriction> T(L.size());
     std::vector<double*> res(L.size(), tmp2);
     L[0].src = rhs;
+    L[0].tmp = tmp;
     for (size_t i = 0; i < L.size(); ++i) {
         if (i > 0) {
             L[i].src = take((size_t)L[i].g.N);
@@ -382,24 +397,15 @@ int multigrid(dft_context* ctx, const Grid& g, const double* rho, double* v, dou
     const bool sor = ctx->mg_coarsest_sor != 0;
     // one cycle in -> out (in is kept), then the residual's max norm into the history
     auto cycle = [&](const double* in, double* out) {
-        if (L.size() == 1) {
-            mg_start_cycle(ctx, hist);
+        if (ctx->mg_fused_restrict || L.size() == 1) {
             L[0].v = out;
-            mg_coarsest_solve(ctx, L[0], rhs, sor);
-        } else if (ctx->mg_fused_restrict) {
-            double* a = mg_fused_level(g.N) ? tmp : out;
-            double* b = mg_fused_level(g.N) ? tmp2 : tmp;
-            mg_smooth_step(ctx, L[0], rhs, nullptr, in, a, 0, fourpi, nullptr, 1);
-            mg_smooth_step(ctx, L[0], rhs, nullptr, a, b, 0, fourpi, nullptr, 1);
-            mg_residual_restrict(ctx, L[0], L[1], rhs, nullptr, b, 0, fourpi, nullptr, 1, hist);
-            mg_cycle_from_zero(ctx, L, 1, L[1].src, nullptr, 0, 1.0, nullptr, 1, sor);
-            mg_correct_smooth(ctx, L[0], L[1], rhs, nullptr, b, tmp2, out, 0, fourpi, nullptr, 1);
+            mg_cycle(ctx, L, 0, rhs, nullptr, in, 0, fourpi, nullptr, 1, sor, hist);
         } else {
             mg_start_cycle(ctx, hist);
             DFT_CUDA(cudaMemcpyAsync(out, in, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
             separate_cycle(ctx, L, T, res, 0, fourpi, out, tmp);
+            mg_residual_max(ctx, g, rhs, fourpi, out, hist);
         }
-        mg_residual_max(ctx, g, rhs, fourpi, out, hist);
     };
     // The cycle's launch sequence is the same every time for this grid: each direction is captured once
     // as a CUDA graph and replayed.  A capture that fails for any reason leaves the direct launches

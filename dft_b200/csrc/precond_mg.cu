@@ -103,7 +103,9 @@ void vcycle_batch(dft_context* ctx, const Grid& g, const double* R, const int* s
     // slab: per band one fine scratch field, and right-hand side, iterate and scratch per coarse level
     size_t per_band = (size_t)ld + 2;
     for (size_t i = 1; i < L.size(); ++i) per_band += 3 * (size_t)L[i].g.N + 6;
-    double* p = (double*)ws_get(ctx, WS_PG2, sizeof(double) * (per_band * nb + 64));
+    double* p = (double*)ws_get(ctx, WS_PG2, sizeof(double) * (per_band * nb + 64 + mg_table_doubles(L)));
+    mg_tables(ctx, L, p);
+    p += (mg_table_doubles(L) + 1) / 2 * 2;
     auto take = [&](size_t n) {
         double* q = p;
         p += (n * nb + 1) / 2 * 2;
@@ -116,12 +118,7 @@ void vcycle_batch(dft_context* ctx, const Grid& g, const double* R, const int* s
         L[i].v = take((size_t)L[i].g.N);
         L[i].tmp = take((size_t)L[i].g.N);
     }
-    if (L.size() == 1) {
-        // the grid is its own coarsest level
-        mg_coarsest_fields(ctx, L[0], R, src_dev, s, shift, nb);
-        return;
-    }
-    mg_cycle_from_zero(ctx, L, 0, R, src_dev, 1, s, shift, nb, false);
+    mg_cycle(ctx, L, 0, R, src_dev, nullptr, 1, s, shift, nb, false, nullptr);
 }
 
 }  // namespace

@@ -8,8 +8,10 @@ import dft_b200
 pytestmark = pytest.mark.gpu
 
 # odd and even axes (coarse spacings of exactly and just below two fine ones), boxes shorter than a
-# tile, one flat enough for a single level, one above the size that takes the long tile passes
-DIMS = [(9, 8, 7), (12, 15, 20), (17, 33, 18), (41, 26, 30), (64, 50, 49), (120, 24, 12), (97, 96, 90)]
+# tile, one whose flat axis gets finer on the coarse grid, levels on both sides of the size up to
+# which a level takes the tile passes
+DIMS = [(9, 8, 7), (12, 15, 20), (17, 33, 18), (41, 26, 30), (64, 50, 49), (120, 24, 12), (200, 40, 4),
+        (97, 96, 90)]
 
 
 def _grid(dims, h=0.3):
