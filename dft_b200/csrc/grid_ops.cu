@@ -16,6 +16,7 @@
 
 #include "ops.h"
 #include "xc_device.cuh"
+#include "xc_fast.cuh"
 #include "xc_grad.cuh"
 
 namespace dftb {
@@ -1635,30 +1636,44 @@ JacobiResult hartree_noalloc(dft_context* ctx, const Grid& g, const double* rho,
 // =============================================================== XC ==================
 namespace {
 
-// Pass 1: functional at every point above the floor.  Writes d f/d n_sigma and the gradient
-// coefficients c_sigma (zero below the floor, reference :626-706) and per-block partial sums
-// of n eps dV (reference :749-842).  One evaluation serves both spins and the energy.
+constexpr int XP = 128;
+
+// Pass 1: functional at every point above the floor (xc_fast.cuh).  GGA: writes d f/d n_sigma and the
+// gradient coefficients c_sigma (zero below the floor, reference :626-706); LDA: the potentials themselves, either
+// of which may be absent.  Per-block partial sums of n eps dV (reference :749-842).  One
+// evaluation serves both spins and the energy.  Bound by its instructions (FP64 pipe 43 % busy, of which
+// logarithms, cube roots and divisions are most); 128 threads and 96 registers leave 20 warps on an SM, 158 -> 146 us
+// against 16.  Both passes, PBE at 128^3: 568 -> 223 us; PZ81 at 75 x 63 x 91: 62 -> 34 us.
 template <int KIND, bool POT, bool ENERGY>
-__global__ void __launch_bounds__(256) xc_point_kernel(Grid g, const double* __restrict__ na,
-                                                       const double* __restrict__ nb, double* __restrict__ da,
-                                                       double* __restrict__ db, double* __restrict__ ca,
-                                                       double* __restrict__ cb, double* __restrict__ partial) {
+__global__ void __launch_bounds__(XP, 5)
+    xc_point_kernel(Grid g, XCScale h, const double* __restrict__ na, const double* __restrict__ nb,
+                    double* __restrict__ da, double* __restrict__ db, double* __restrict__ ca, double* __restrict__ cb,
+                    double* __restrict__ partial) {
     __shared__ double sh[8];
     double e = 0.0;
+    const bool small = g.N < (1LL << 31);
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < g.N; p += (long long)gridDim.x * blockDim.x) {
         const double a = na[p], b = nb[p];
         const double n = a + b;
         double rda = 0.0, rdb = 0.0, rca = 0.0, rcb = 0.0;
         if (n > xcf::RHO_FLOOR) {
-            const int i = (int)(p % g.nx);
-            const int j = (int)((p / g.nx) % g.ny);
-            const int k = (int)(p / ((long long)g.nx * g.ny));
             double ga = 0.0, gb = 0.0;
             if (KIND == 1) {
-                ga = gradmag(g, na, p, i, j, k);
-                gb = gradmag(g, nb, p, i, j, k);
+                int i, j, k;
+                if (small) {  // 32-bit divisions
+                    const unsigned q = (unsigned)p, row = q / (unsigned)g.nx;
+                    i = (int)(q - row * (unsigned)g.nx);
+                    k = (int)(row / (unsigned)g.ny);
+                    j = (int)(row - (unsigned)k * (unsigned)g.ny);
+                } else {
+                    i = (int)(p % g.nx);
+                    j = (int)((p / g.nx) % g.ny);
+                    k = (int)(p / ((long long)g.nx * g.ny));
+                }
+                ga = grad_of(g, h, na, p, i, j, k);
+                gb = grad_of(g, h, nb, p, i, j, k);
             }
-            const xcf::Result r = xcf::evaluate<KIND>(a, b, ga, gb);
+            const xcf::Result r = xcf::evaluate_fast<KIND>(a, b, ga, gb);
             rda = r.va;
             rdb = r.vb;
             rca = r.ca;
@@ -1666,11 +1681,14 @@ __global__ void __launch_bounds__(256) xc_point_kernel(Grid g, const double* __r
             if (ENERGY) e += n * r.eps * g.dV;
         }
         if (POT) {
-            da[p] = rda;
-            db[p] = rdb;
             if (KIND == 1) {
+                da[p] = rda;
+                db[p] = rdb;
                 ca[p] = rca;
                 cb[p] = rcb;
+            } else {
+                if (da) da[p] = rda;
+                if (db) db[p] = rdb;
             }
         }
     }
@@ -1680,69 +1698,87 @@ __global__ void __launch_bounds__(256) xc_point_kernel(Grid g, const double* __r
     }
 }
 
-// div(c grad f) at (i,j,k), reference calculateCartesianDivergence :216-572
-__device__ __forceinline__ double ddiv(const Grid& g, const double* __restrict__ c, const double* __restrict__ f,
-                                       long long p, int i, int j, int k) {
-    const double cc = c[p];
-    double dx, dy, dz;
-    {
-        const double fc = cc * dderiv(g, f, p, i, j, k, 0);
-        if (i == 0) dx = (c[p + 1] * dderiv(g, f, p + 1, i + 1, j, k, 0) - fc) / g.dx;
-        else if (i == g.nx - 1) dx = (fc - c[p - 1] * dderiv(g, f, p - 1, i - 1, j, k, 0)) / g.dx;
-        else
-            dx = (c[p + 1] * dderiv(g, f, p + 1, i + 1, j, k, 0) - c[p - 1] * dderiv(g, f, p - 1, i - 1, j, k, 0)) /
-                 (2.0 * g.dx);
-    }
-    {
-        const long long s = g.nx;
-        const double fc = cc * dderiv(g, f, p, i, j, k, 1);
-        if (j == 0) dy = (c[p + s] * dderiv(g, f, p + s, i, j + 1, k, 1) - fc) / g.dy;
-        else if (j == g.ny - 1) dy = (fc - c[p - s] * dderiv(g, f, p - s, i, j - 1, k, 1)) / g.dy;
-        else
-            dy = (c[p + s] * dderiv(g, f, p + s, i, j + 1, k, 1) - c[p - s] * dderiv(g, f, p - s, i, j - 1, k, 1)) /
-                 (2.0 * g.dy);
-    }
-    {
-        const long long s = (long long)g.nx * g.ny;
-        const double fc = cc * dderiv(g, f, p, i, j, k, 2);
-        if (k == 0) dz = (c[p + s] * dderiv(g, f, p + s, i, j, k + 1, 2) - fc) / g.dz;
-        else if (k == g.nz - 1) dz = (fc - c[p - s] * dderiv(g, f, p - s, i, j, k - 1, 2)) / g.dz;
-        else
-            dz = (c[p + s] * dderiv(g, f, p + s, i, j, k + 1, 2) - c[p - s] * dderiv(g, f, p - s, i, j, k - 1, 2)) /
-                 (2.0 * g.dz);
-    }
-    return dx + dy + dz;
+// d(c df)/dx at index i of a line of n points, one-sided at the ends (reference calculateCartesianDivergence and
+// calculateCartesianDerivative, ExchangeCorrelationMolecule.cpp:11-572): the fluxes at r = i + 1
+// and l = i - 1 (i itself at an end) need f there on the far side (P, M) and at i, and at an end the
+// inner neighbour takes the far side's place with the sign turned.  Same four loads and operations everywhere.
+struct XCAxis {
+    int P, M, r, l;     // offsets from i
+    double wr, wl, w;
+};
+__device__ __forceinline__ XCAxis xc_axis(int i, int n, double h1, double h2) {
+    XCAxis a;
+    const int l = max(i - 1, 0), r = min(i + 1, n - 1);
+    a.r = r - i;
+    a.l = l - i;
+    a.P = i == n - 1 ? -1 : min(r + 1, n - 1) - i;
+    a.M = i == 0 ? 1 : max(l - 1, 0) - i;
+    a.wr = r == n - 1 ? h1 : h2;
+    a.wl = l == 0 ? h1 : h2;
+    if (i == n - 1) a.wr = -a.wr;
+    if (i == 0) a.wl = -a.wl;
+    a.w = r - l == 2 ? h2 : h1;
+    return a;
+}
+__device__ __forceinline__ double xc_axis_div(const XCAxis& a, double cr, double cl, double P, double f, double M) {
+    return (cr * ((P - f) * a.wr) - cl * ((f - M) * a.wl)) * a.w;
 }
 
-// Pass 2 (GGA only): v_sigma = d_sigma - div(c_sigma grad n_sigma) above the floor, else 0.
-__global__ void __launch_bounds__(256) xc_div_kernel(Grid g, const double* __restrict__ na,
-                                                     const double* __restrict__ nb, const double* __restrict__ da,
-                                                     const double* __restrict__ db, const double* __restrict__ ca,
-                                                     const double* __restrict__ cb, double* __restrict__ va,
-                                                     double* __restrict__ vb) {
-    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < g.N; p += (long long)gridDim.x * blockDim.x) {
-        const double n = na[p] + nb[p];
-        double ra = 0.0, rb = 0.0;
-        if (n > xcf::RHO_FLOOR) {
-            const int i = (int)(p % g.nx);
-            const int j = (int)((p / g.nx) % g.ny);
-            const int k = (int)(p / ((long long)g.nx * g.ny));
-            if (va) ra = da[p] - ddiv(g, ca, na, p, i, j, k);
-            if (vb) rb = db[p] - ddiv(g, cb, nb, p, i, j, k);
+// Pass 2 (GGA only): v_sigma = d_sigma - div(c_sigma grad n_sigma) above the floor, else 0.  A thread
+// marches along z with five planes of n_sigma and three of c_sigma in registers, all loads of a plane in
+// flight together whether or not the point is above the floor.  57 us at 128^3 from a cold
+// L2; with loads under the test of the floor and branches at the faces it took 98, and one thread per point
+// with 19 divisions per spin 81 us at 96^3.
+constexpr int XD_X = 32, XD_Y = 8;
+__global__ void __launch_bounds__(XD_X* XD_Y, 2)
+    xc_div_kernel(Grid g, XCScale h, const double* __restrict__ na, const double* __restrict__ nb,
+                  const double* __restrict__ da, const double* __restrict__ db, const double* __restrict__ ca,
+                  const double* __restrict__ cb, double* __restrict__ va, double* __restrict__ vb, int zc) {
+    const int i = blockIdx.x * XD_X + threadIdx.x, j = blockIdx.y * XD_Y + threadIdx.y;
+    if (i >= g.nx || j >= g.ny) return;
+    const int kb = blockIdx.z * zc, ke = min(g.nz, kb + zc);
+    const long long s2 = (long long)g.nx * g.ny, col = (long long)j * g.nx + i;
+    const double *n_[2] = {na + col, nb + col}, *c_[2] = {ca + col, cb + col}, *d_[2] = {da + col, db + col};
+    const XCAxis X = xc_axis(i, g.nx, h.x1, h.x2), Y = xc_axis(j, g.ny, h.y1, h.y2);
+    const int yP = Y.P * g.nx, yM = Y.M * g.nx, yr = Y.r * g.nx, yl = Y.l * g.nx;
+    double f[2][5], c[2][3];  // planes k - 2 .. k + 2 and k - 1 .. k + 1, the grid's ends repeated
+    auto plane = [&](int k) { return min(max(k, 0), g.nz - 1) * s2; };
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) f[s][t + 1] = __ldg(n_[s] + plane(kb - 2 + t));
+        c[s][1] = __ldg(c_[s] + plane(kb - 1));
+        c[s][2] = __ldg(c_[s] + plane(kb));
+    }
+#pragma unroll 2
+    for (int k = kb; k < ke; ++k) {
+        const long long p = k * s2, p1 = plane(k + 1), p2 = plane(k + 2);
+        double L[2][9];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) f[s][t] = f[s][t + 1];
+            f[s][4] = __ldg(n_[s] + p2);
+            c[s][0] = c[s][1];
+            c[s][1] = c[s][2];
+            c[s][2] = __ldg(c_[s] + p1);
+            const double *fn = n_[s] + p, *cn = c_[s] + p;
+            L[s][0] = __ldg(fn + X.P), L[s][1] = __ldg(fn + X.M), L[s][2] = __ldg(cn + X.r), L[s][3] = __ldg(cn + X.l);
+            L[s][4] = __ldg(fn + yP), L[s][5] = __ldg(fn + yM), L[s][6] = __ldg(cn + yr), L[s][7] = __ldg(cn + yl);
+            L[s][8] = __ldg(d_[s] + p);
         }
-        if (va) va[p] = ra;
-        if (vb) vb[p] = rb;
-    }
-}
-
-// LDA potential: the divergence term vanishes identically (c = 0), v = d above the floor.
-__global__ void xc_lda_copy_kernel(long long n, const double* __restrict__ na, const double* __restrict__ nb,
-                                   const double* __restrict__ da, const double* __restrict__ db, double* va,
-                                   double* vb) {
-    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
-        const bool on = na[p] + nb[p] > xcf::RHO_FLOOR;
-        if (va) va[p] = on ? da[p] : 0.0;
-        if (vb) vb[p] = on ? db[p] : 0.0;
+        const XCAxis Z = xc_axis(k, g.nz, h.z1, h.z2);
+        const bool on = f[0][2] + f[1][2] > xcf::RHO_FLOOR;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const double f0 = f[s][2];
+            const double zP = k == g.nz - 1 ? f[s][1] : f[s][4], zM = k == 0 ? f[s][3] : f[s][0];
+            const double dx = xc_axis_div(X, L[s][2], L[s][3], L[s][0], f0, L[s][1]);
+            const double dy = xc_axis_div(Y, L[s][6], L[s][7], L[s][4], f0, L[s][5]);
+            const double dz = xc_axis_div(Z, c[s][2], c[s][0], zP, f0, zM);
+            double* v = s == 0 ? va : vb;
+            if (v) v[p + col] = on ? L[s][8] - (dx + dy + dz) : 0.0;
+        }
     }
 }
 
@@ -1764,23 +1800,26 @@ double xc_impl(dft_context* ctx, const Grid& g, const double* na, const double* 
                bool want_energy) {
     const bool pot = va || vb;
     const size_t N = (size_t)g.N;
-    double* tmp = pot ? (double*)ws_get(ctx, WS_XC, sizeof(double) * 4 * N) : nullptr;
-    double *da = tmp, *db = tmp ? tmp + N : nullptr, *ca = tmp ? tmp + 2 * N : nullptr, *cb = tmp ? tmp + 3 * N : nullptr;
-    const int nbk = std::max(1, std::min((int)((g.N + 255) / 256), ctx->num_sms * 8));
+    double* tmp = pot && KIND == 1 ? (double*)ws_get(ctx, WS_XC, sizeof(double) * 4 * N) : nullptr;
+    double *da = tmp ? tmp : va, *db = tmp ? tmp + N : vb, *ca = tmp ? tmp + 2 * N : nullptr,
+           *cb = tmp ? tmp + 3 * N : nullptr;
+    const XCScale inv = xc_scale(g);
+    const int nbk = (int)std::max<long long>(1, std::min<long long>((g.N + XP - 1) / XP, ctx->num_sms * 10));
     double* partial = (double*)ws_get(ctx, WS_REDUCE, sizeof(double) * ((size_t)nbk + 8));
     if (pot && want_energy)
-        xc_point_kernel<KIND, true, true><<<nbk, 256, 0, ctx->stream>>>(g, na, nb, da, db, ca, cb, partial);
+        xc_point_kernel<KIND, true, true><<<nbk, XP, 0, ctx->stream>>>(g, inv, na, nb, da, db, ca, cb, partial);
     else if (pot)
-        xc_point_kernel<KIND, true, false><<<nbk, 256, 0, ctx->stream>>>(g, na, nb, da, db, ca, cb, partial);
+        xc_point_kernel<KIND, true, false><<<nbk, XP, 0, ctx->stream>>>(g, inv, na, nb, da, db, ca, cb, partial);
     else
-        xc_point_kernel<KIND, false, true><<<nbk, 256, 0, ctx->stream>>>(g, na, nb, da, db, ca, cb, partial);
+        xc_point_kernel<KIND, false, true><<<nbk, XP, 0, ctx->stream>>>(g, inv, na, nb, da, db, ca, cb, partial);
     DFT_LAUNCH_CHECK();
     count_launch(ctx);
-    if (pot) {
-        if (KIND == 1)
-            xc_div_kernel<<<nbk, 256, 0, ctx->stream>>>(g, na, nb, da, db, ca, cb, va, vb);
-        else
-            xc_lda_copy_kernel<<<nbk, 256, 0, ctx->stream>>>(g.N, na, nb, da, db, va, vb);
+    if (pot && KIND == 1) {
+        const int bx = (g.nx + XD_X - 1) / XD_X, by = (g.ny + XD_Y - 1) / XD_Y;
+        int zc = 32;
+        while (zc > 4 && (long long)bx * by * ((g.nz + zc - 1) / zc) < 6LL * ctx->num_sms) zc >>= 1;
+        xc_div_kernel<<<dim3(bx, by, (g.nz + zc - 1) / zc), dim3(XD_X, XD_Y), 0, ctx->stream>>>(
+            g, inv, na, nb, da, db, ca, cb, va, vb, zc);
         DFT_LAUNCH_CHECK();
         count_launch(ctx);
     }

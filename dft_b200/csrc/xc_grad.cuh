@@ -6,28 +6,24 @@
 
 namespace dftb {
 
-// calculateCartesianDerivative, reference ExchangeCorrelationMolecule.cpp:11-170
-__device__ __forceinline__ double dderiv(const Grid& g, const double* __restrict__ f, long long p, int i, int j, int k,
-                                         int dir) {
-    if (dir == 0) {
-        if (i == 0) return (f[p + 1] - f[p]) / g.dx;
-        if (i == g.nx - 1) return (f[p] - f[p - 1]) / g.dx;
-        return (f[p + 1] - f[p - 1]) / (2.0 * g.dx);
-    }
-    if (dir == 1) {
-        const long long s = g.nx;
-        if (j == 0) return (f[p + s] - f[p]) / g.dy;
-        if (j == g.ny - 1) return (f[p] - f[p - s]) / g.dy;
-        return (f[p + s] - f[p - s]) / (2.0 * g.dy);
-    }
-    const long long s = (long long)g.nx * g.ny;
-    if (k == 0) return (f[p + s] - f[p]) / g.dz;
-    if (k == g.nz - 1) return (f[p] - f[p - s]) / g.dz;
-    return (f[p + s] - f[p - s]) / (2.0 * g.dz);
+// Reciprocal spacings of the one-sided and the central differences.
+struct XCScale {
+    double x1, y1, z1, x2, y2, z2;
+};
+inline XCScale xc_scale(const Grid& g) {
+    return {1.0 / g.dx, 1.0 / g.dy, 1.0 / g.dz, 0.5 / g.dx, 0.5 / g.dy, 0.5 / g.dz};
 }
 
-__device__ __forceinline__ double gradmag(const Grid& g, const double* __restrict__ f, long long p, int i, int j, int k) {
-    const double gx = dderiv(g, f, p, i, j, k, 0), gy = dderiv(g, f, p, i, j, k, 1), gz = dderiv(g, f, p, i, j, k, 2);
+// |grad f|, central differences, one-sided on the faces (calculateCartesianDerivative, reference
+// ExchangeCorrelationMolecule.cpp:11-170)
+__device__ __forceinline__ double grad_of(const Grid& g, const XCScale& h, const double* __restrict__ f, long long p,
+                                          int i, int j, int k) {
+    const int s1 = g.nx;
+    const long long s2 = (long long)g.nx * g.ny;
+    const bool xl = i > 0, xr = i + 1 < g.nx, yl = j > 0, yr = j + 1 < g.ny, zl = k > 0, zr = k + 1 < g.nz;
+    const double gx = (f[xr ? p + 1 : p] - f[xl ? p - 1 : p]) * (xl && xr ? h.x2 : h.x1);
+    const double gy = (f[yr ? p + s1 : p] - f[yl ? p - s1 : p]) * (yl && yr ? h.y2 : h.y1);
+    const double gz = (f[zr ? p + s2 : p] - f[zl ? p - s2 : p]) * (zl && zr ? h.z2 : h.z1);
     return sqrt(gx * gx + gy * gy + gz * gz);
 }
 

@@ -32,6 +32,7 @@
 
 #include "ops.h"
 #include "xc_device.cuh"
+#include "xc_fast.cuh"
 #include "xc_grad.cuh"
 
 namespace dftb {
@@ -156,7 +157,7 @@ __global__ void slab_shell_copy_kernel(int nx, int ny, int nzl, const double* __
 // Sum of n eps dV over the points [p_lo, p_hi) of a slab (one partial per block), gradients
 // from the whole slab as in xc_point_kernel.
 template <int KIND>
-__global__ void __launch_bounds__(256) slab_xc_energy_kernel(Grid s, long long p_lo, long long p_hi,
+__global__ void __launch_bounds__(256) slab_xc_energy_kernel(Grid s, XCScale h, long long p_lo, long long p_hi,
                                                              const double* __restrict__ na,
                                                              const double* __restrict__ nb,
                                                              double* __restrict__ partial) {
@@ -172,10 +173,10 @@ __global__ void __launch_bounds__(256) slab_xc_energy_kernel(Grid s, long long p
             const int k = (int)(p / ((long long)s.nx * s.ny));
             double ga = 0.0, gb = 0.0;
             if (KIND == 1) {
-                ga = gradmag(s, na, p, i, j, k);
-                gb = gradmag(s, nb, p, i, j, k);
+                ga = grad_of(s, h, na, p, i, j, k);
+                gb = grad_of(s, h, nb, p, i, j, k);
             }
-            e += n * xcf::evaluate<KIND>(a, b, ga, gb).eps * s.dV;
+            e += n * xcf::evaluate_fast<KIND>(a, b, ga, gb).eps * s.dV;
         }
     }
     e = block_sum(e, sh);
@@ -275,9 +276,9 @@ double zslab_xc(dft_context* ctx, const Grid& g, int z_lo, int z_hi, int own_lo,
     const int nbk = (int)std::max<long long>(1, std::min<long long>((p_hi - p_lo + 255) / 256, (long long)ctx->num_sms * 8));
     double* partial = (double*)ws_get(ctx, WS_REDUCE, sizeof(double) * (size_t)nbk);
     if (kind == DFT_XC_PBE96)
-        slab_xc_energy_kernel<1><<<nbk, 256, 0, ctx->stream>>>(s, p_lo, p_hi, na, nb, partial);
+        slab_xc_energy_kernel<1><<<nbk, 256, 0, ctx->stream>>>(s, xc_scale(s), p_lo, p_hi, na, nb, partial);
     else
-        slab_xc_energy_kernel<0><<<nbk, 256, 0, ctx->stream>>>(s, p_lo, p_hi, na, nb, partial);
+        slab_xc_energy_kernel<0><<<nbk, 256, 0, ctx->stream>>>(s, xc_scale(s), p_lo, p_hi, na, nb, partial);
     DFT_LAUNCH_CHECK();
     count_launch(ctx);
     double* h = pinned(ctx, (size_t)nbk);
