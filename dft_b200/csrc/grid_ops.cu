@@ -177,13 +177,15 @@ constexpr int HB_X = 32, HB_Y = 8;
 // One thread per (i,j) column of one band, marching k over a z-chunk (32 registers, 8 blocks
 // per SM).  reference KohnShamHamiltonianMolecule.cpp:59-177: lap = k0*c (+ neighbours in the
 // order x-, x+, y-, y+, z-, z+), H psi = -0.5*lap + V*c; absent neighbours are skipped.
+// Blocks go through the bands before the next z-chunk, so the bands in flight together read the same V
+// (192^3, 16 bands: with each band's chunks in turn V comes from memory once per band, 440 us against 420).
 __global__ void __launch_bounds__(HB_X* HB_Y) hpsi1_kernel(Grid g, const double* __restrict__ V,
                                                           const double* __restrict__ psi, double* __restrict__ out,
-                                                          long long ld, int zchunk, int nzc, double k0) {
+                                                          long long ld, int zchunk, int nbands, double k0) {
     const int i = blockIdx.x * HB_X + threadIdx.x;
     const int j = blockIdx.y * HB_Y + threadIdx.y;
-    const int band = blockIdx.z / nzc;
-    const int kc = blockIdx.z - band * nzc;
+    const int kc = blockIdx.z / nbands;
+    const int band = blockIdx.z - kc * nbands;
     if (i >= g.nx || j >= g.ny) return;
     const double* __restrict__ p = psi + (long long)band * ld;
     double* __restrict__ o = out + (long long)band * ld;
@@ -207,6 +209,57 @@ __global__ void __launch_bounds__(HB_X* HB_Y) hpsi1_kernel(Grid g, const double*
         o[idx] = __dadd_rn(__dmul_rn(-0.5, lap), __dmul_rn(__ldg(V + idx), cur));
         below = cur;
         cur = above;
+    }
+}
+
+// The same for even row lengths and 16-byte aligned arrays: a thread takes two columns with 16-byte loads, half
+// the load instructions per byte and half as much again in flight (more planes per thread instead cost
+// occupancy: 480 to 520 us).  Bound by memory: psi once, H psi once, V about once.  192^3, 16
+// bands: 484 -> 409 us.
+constexpr int HP_BLOCKS = 6;  // per SM: 40 registers
+__global__ void __launch_bounds__(256, HP_BLOCKS)
+    hpsi_pair_kernel(Grid g, const double* __restrict__ V, const double* __restrict__ psi, double* __restrict__ out,
+                     long long ld, int zchunk, int nbands, double k0) {
+    const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int kc = blockIdx.z / nbands, band = blockIdx.z - kc * nbands;
+    if (i >= g.nx || j >= g.ny) return;
+    const int sxy = g.nx * g.ny;
+    const int kb = kc * zchunk, ke = min(g.nz, kb + zchunk);
+    const long long at = (long long)kb * sxy + (long long)j * g.nx + i;
+    const double* __restrict__ p = psi + (long long)band * ld + at;
+    const double* __restrict__ v = V + at;
+    double* __restrict__ o = out + (long long)band * ld + at;
+    const bool xl = i > 0, xr = i + 2 < g.nx, yl = j > 0, yr = j + 1 < g.ny;
+    const int oxl = xl ? -1 : 0, oxr = xr ? 2 : 0, oyl = yl ? -g.nx : 0, oyr = yr ? g.nx : 0;
+    auto two = [](const double* q) { return __ldg((const double2*)q); };
+    double2 below = kb > 0 ? two(p - sxy) : make_double2(0.0, 0.0);
+    double2 cur = two(p);
+    for (int k = kb; k < ke; ++k) {
+        const bool zl = k > 0, zr = k + 1 < g.nz;
+        const double2 ab = zr ? two(p + sxy) : make_double2(0.0, 0.0);
+        const double2 w = two(v), ym = two(p + oyl), yp = two(p + oyr);
+        const double xm = __ldg(p + oxl), xp = __ldg(p + oxr);
+        auto point = [&](bool l, bool r, double c, double lft, double rgt, double a, double b, double d, double u,
+                         double pot) {
+            double lap = __dmul_rn(k0, c);
+            if (l) lap = __dadd_rn(lap, __dmul_rn(lft, g.ix2));
+            if (r) lap = __dadd_rn(lap, __dmul_rn(rgt, g.ix2));
+            if (yl) lap = __dadd_rn(lap, __dmul_rn(a, g.iy2));
+            if (yr) lap = __dadd_rn(lap, __dmul_rn(b, g.iy2));
+            if (zl) lap = __dadd_rn(lap, __dmul_rn(d, g.iz2));
+            if (zr) lap = __dadd_rn(lap, __dmul_rn(u, g.iz2));
+            return __dadd_rn(__dmul_rn(-0.5, lap), __dmul_rn(pot, c));
+        };
+        double2 r;
+        r.x = point(xl, true, cur.x, xm, cur.y, ym.x, yp.x, below.x, ab.x, w.x);
+        r.y = point(true, xr, cur.y, cur.x, xp, ym.y, yp.y, below.y, ab.y, w.y);
+        *(double2*)o = r;
+        below = cur;
+        cur = ab;
+        p += sxy;
+        v += sxy;
+        o += sxy;
     }
 }
 
@@ -599,6 +652,20 @@ CUtensorMap hpsi_tensor_map(const Grid& g, const double* psi, long long ld, int 
     return tm;
 }
 
+// Planes per block of a march over nz planes, `columns` blocks per plane and `slots` blocks resident: the chunk
+// with the fewest planes in a row, whole waves counted and three planes of start per block (128^3, 5
+// bands: chunks of 32 left a second wave of 4 %, 79 us; 26 planes: 61).
+inline int march_chunk(int nz, long long columns, long long slots) {
+    int best = nz;
+    long long cost = -1;
+    for (int chunks = 1; chunks <= std::max(1, nz / 4); ++chunks) {
+        const int zc = (nz + chunks - 1) / chunks;
+        const long long waves = (columns * ((nz + zc - 1) / zc) + slots - 1) / slots, c = waves * (zc + 3);
+        if (cost < 0 || c < cost) cost = c, best = zc;
+    }
+    return best;
+}
+
 inline int pick_zchunk(const Grid& g, long long columns_blocks, int nbands, int num_sms) {
     // enough CTAs to fill the machine a few times over, but chunks long enough to amortise
     // the two-plane warm-up of the z march
@@ -683,7 +750,26 @@ void apply_hamiltonian(dft_context* ctx, const Grid& g, const double* V, const d
     // machine a few times over
     int zset = ctx->hpsi_zchunk;
     if (zset == 0 && tuned != ctx->tuned.end()) zset = tuned->second[3];
-    const int zc = zset > 0 ? std::min(zset, g.nz) : pick_zchunk(g, (long long)bx * by, groups, ctx->num_sms);
+    const bool single = nbt == 1 && ctx->hpsi_variant != 1 && variant != 3;
+    if (single && g.nx % 2 == 0 && ld % 2 == 0 && ((uintptr_t)V | (uintptr_t)psi | (uintptr_t)hpsi) % 16 == 0) {
+        // two columns per thread; 16 threads across where that leaves fewer of them idle
+        const int pairs = g.nx / 2, tx = (pairs + 15) / 16 * 16 < (pairs + 31) / 32 * 32 ? 16 : 32, ty = 256 / tx;
+        const int px = (pairs + tx - 1) / tx, py = (g.ny + ty - 1) / ty;
+        const int pz = zset > 0 ? std::min(zset, g.nz)
+                                : march_chunk(g.nz, (long long)px * py * nbands, (long long)HP_BLOCKS * ctx->num_sms);
+        const int chunks = (g.nz + pz - 1) / pz, most = std::max(1, 65535 / chunks);
+        for (int b0 = 0; b0 < nbands; b0 += most) {
+            const int nb = std::min(most, nbands - b0);
+            hpsi_pair_kernel<<<dim3(px, py, nb * chunks), dim3(tx, ty), 0, ctx->stream>>>(
+                g, V, psi + (long long)b0 * ld, hpsi + (long long)b0 * ld, ld, pz, nb, k0);
+            DFT_LAUNCH_CHECK();
+            count_launch(ctx);
+        }
+        return;
+    }
+    const int zc = zset > 0 ? std::min(zset, g.nz)
+                   : single ? march_chunk(g.nz, (long long)bx * by * nbands, 8LL * ctx->num_sms)
+                            : pick_zchunk(g, (long long)bx * by, groups, ctx->num_sms);
     const int nzc = (g.nz + zc - 1) / zc;
     // gridDim.z limit is 65535: split the band block if needed
     const int max_groups = std::max(1, 65535 / nzc);
@@ -704,7 +790,7 @@ void apply_hamiltonian(dft_context* ctx, const Grid& g, const double* V, const d
         } else if (variant == 3) {
             hpsi1p_kernel<<<grid, block, 0, ctx->stream>>>(g, V, pi, po, ld, zc, nzc, k0);
         } else {
-            hpsi1_kernel<<<grid, block, 0, ctx->stream>>>(g, V, pi, po, ld, zc, nzc, k0);
+            hpsi1_kernel<<<grid, block, 0, ctx->stream>>>(g, V, pi, po, ld, zc, nb, k0);
         }
         DFT_LAUNCH_CHECK();
         count_launch(ctx);
@@ -1640,11 +1726,11 @@ constexpr int XP = 128;
 
 // Pass 1: functional at every point above the floor (xc_fast.cuh).  GGA: writes d f/d n_sigma and the
 // gradient coefficients c_sigma (zero below the floor, reference :626-706); LDA: the potentials themselves, either
-// of which may be absent.  Per-block partial sums of n eps dV (reference :749-842).  One
+// of which may be absent.  partial: when given, per-block sums of n eps dV (reference :749-842).  One
 // evaluation serves both spins and the energy.  Bound by its instructions (FP64 pipe 43 % busy, of which
 // logarithms, cube roots and divisions are most); 128 threads and 96 registers leave 20 warps on an SM, 158 -> 146 us
 // against 16.  Both passes, PBE at 128^3: 568 -> 223 us; PZ81 at 75 x 63 x 91: 62 -> 34 us.
-template <int KIND, bool POT, bool ENERGY>
+template <int KIND, bool POT>
 __global__ void __launch_bounds__(XP, 5)
     xc_point_kernel(Grid g, XCScale h, const double* __restrict__ na, const double* __restrict__ nb,
                     double* __restrict__ da, double* __restrict__ db, double* __restrict__ ca, double* __restrict__ cb,
@@ -1678,7 +1764,7 @@ __global__ void __launch_bounds__(XP, 5)
             rdb = r.vb;
             rca = r.ca;
             rcb = r.cb;
-            if (ENERGY) e += n * r.eps * g.dV;
+            e += n * r.eps * g.dV;
         }
         if (POT) {
             if (KIND == 1) {
@@ -1692,7 +1778,7 @@ __global__ void __launch_bounds__(XP, 5)
             }
         }
     }
-    if (ENERGY) {
+    if (partial) {
         e = block_sum(e, sh);
         if (threadIdx.x == 0) partial[blockIdx.x] = e;
     }
@@ -1806,12 +1892,12 @@ double xc_impl(dft_context* ctx, const Grid& g, const double* na, const double* 
     const XCScale inv = xc_scale(g);
     const int nbk = (int)std::max<long long>(1, std::min<long long>((g.N + XP - 1) / XP, ctx->num_sms * 10));
     double* partial = (double*)ws_get(ctx, WS_REDUCE, sizeof(double) * ((size_t)nbk + 8));
-    if (pot && want_energy)
-        xc_point_kernel<KIND, true, true><<<nbk, XP, 0, ctx->stream>>>(g, inv, na, nb, da, db, ca, cb, partial);
-    else if (pot)
-        xc_point_kernel<KIND, true, false><<<nbk, XP, 0, ctx->stream>>>(g, inv, na, nb, da, db, ca, cb, partial);
+    // one kernel with and without the energy, so the potentials' bits do not depend on it
+    if (pot)
+        xc_point_kernel<KIND, true><<<nbk, XP, 0, ctx->stream>>>(g, inv, na, nb, da, db, ca, cb,
+                                                                 want_energy ? partial : nullptr);
     else
-        xc_point_kernel<KIND, false, true><<<nbk, XP, 0, ctx->stream>>>(g, inv, na, nb, da, db, ca, cb, partial);
+        xc_point_kernel<KIND, false><<<nbk, XP, 0, ctx->stream>>>(g, inv, na, nb, da, db, ca, cb, partial);
     DFT_LAUNCH_CHECK();
     count_launch(ctx);
     if (pot && KIND == 1) {
