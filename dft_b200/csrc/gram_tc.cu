@@ -5,18 +5,19 @@
 // lo = TF32(x - hi)), and the product is formed as hi*hi + hi*lo + lo*hi with FP32
 // accumulation in tensor memory (TMEM): relative error ~1e-6, the "FP32-level" precision the
 // block eigensolver uses while residuals are large.  Per block:
-//   * 256 threads stage a 32-point K slice of A (128 rows) and B (<= 256 rows) from HBM,
-//     split them and store hi/lo planes in shared memory in the canonical K-major layout
-//     (8-row x 16-byte core matrices, no swizzle), double-buffered; the next slice's FP64
-//     values are loaded into registers while the tensor cores consume the current one;
+//   * 16 warps take 32-point K slices of at most 128 rows of one operand and 256 of the other
+//     from HBM, split them and store hi/lo planes in shared memory in the canonical K-major layout
+//     (128-byte swizzled rows), double-buffered; the FP64 values of the next slice are on their
+//     way into registers meanwhile;
 //   * one thread issues 12 tcgen05.mma.kind::tf32 (4 K=8 steps x 3 products) into a
 //     128 x N FP32 accumulator in TMEM and commits them to an mbarrier;
 //   * after its K range the block reads the accumulator back with tcgen05.ld (each warp its
 //     32 TMEM lanes) and writes FP64 partial sums; a deterministic FP64 reduction over blocks
-//     (gram_reduce_kernel in davidson.cu) finishes the product.
+//     (gram_tc_reduce_kernel) finishes the product.
 // Every mbarrier wait is bounded; a block that gives up sets an error flag, waits (bounded)
 // for its own MMAs, frees its TMEM and returns.
 #include <cstdint>
+#include <type_traits>
 #include <vector>
 
 #include "ops.h"
@@ -33,17 +34,28 @@ constexpr long long TC_SPIN_LIMIT = 1LL << 22;  // try_wait polls before a block
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// round to nearest, ties away from zero, as cvt.rna.tf32.f32 does in many more instructions
 __device__ __forceinline__ uint32_t to_tf32(float x) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return r;
+    const uint32_t r = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    return x == x ? r : 0x7fffffffu;
 }
 
-// canonical K-major, no-swizzle placement of element (row, k) of an R-row x 32-point slice:
-// core matrix (8 rows x 4 fp32) index = (k/4) * (R/8) + row/8, 128 bytes each
-__device__ __forceinline__ int kmajor_offset_words(int row, int k, int R) {
-    return (((k >> 2) * (R >> 3) + (row >> 3)) << 5) + ((row & 7) << 2) + (k & 3);
+// x ~ hi + lo, both TF32: hi = TF32(FP32(x)), lo = TF32(FP32(x - hi)).  Conversions from and to FP64 are the
+// slowest operations here, so hi is widened by integer operations (138 x 69, 112 x 97 x 101: 721 -> 703 us).  Rounding
+// x and x - hi by integer operations as well took 983.
+__device__ __forceinline__ void split_tf32(double x, uint32_t& hi, uint32_t& lo) {
+    hi = to_tf32((float)x);
+    const uint32_t m = hi & 0x7fffffffu;
+    double w = __hiloint2double((int)(((m >> 3) + 0x38000000u) | (hi & 0x80000000u)), 0);
+    // zero, denormal, infinite, NaN; predicated, so that the elements of a slice stay one straight piece of code
+    asm("{\n\t.reg .pred p;\n\tsetp.ge.u32 p, %2, 0x7f000000;\n\t@p cvt.f64.f32 %0, %1;\n\t}"
+        : "+d"(w)
+        : "f"(__uint_as_float(hi)), "r"(m - 0x00800000u));
+    lo = to_tf32((float)(x - w));
 }
+
+// Canonical K-major, no-swizzle placement of element (row, k) of an R-row slice (ring, TMA and rotation
+// kernels): core matrix (8 rows x 4 fp32) index = (k/4) * (R/8) + row/8, 128 bytes each.
 
 // UMMA shared-memory matrix descriptor (sm_100: version 1, no swizzle)
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
@@ -53,6 +65,12 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes,
     d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
     d |= (uint64_t)1 << 46;  // version
     return d;                // layout type 0 = SWIZZLE_NONE, base offset 0
+}
+
+// the same for rows of 128 bytes, 8 rows to a 1024-byte atom whose 16-byte chunks are swizzled by the row
+// (layout type 2 = SWIZZLE_128B; the leading offset is not used within one atom of K)
+__device__ __forceinline__ uint64_t smem_desc_128(uint32_t addr) {
+    return smem_desc(addr, 16, 1024) | (uint64_t)2 << 61;
 }
 
 // instruction descriptor: D = F32, A = B = TF32, both K-major, M = 128, N = n
@@ -95,139 +113,149 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                  : "memory");
 }
 
-// Gram tile.  grid = (ceil(ka/128), ceil(kb/nt), nchunks); dynamic smem = 2 stages x
-// (A hi, A lo: 128 x 32 fp32; B hi, B lo: NC x 32 fp32).  Row r of a slice is read by warp
-// r % 8 (one point per lane); each thread holds the next slice's raw FP64 values in
-// registers, loaded while the tensor cores work on the current slice.
-template <int NC>
-__global__ void __launch_bounds__(TC_THREADS, 1)
-    gram_tc_kernel(const double* __restrict__ A, long long lda, int ka, const double* __restrict__ B, long long ldb,
-                   int kb, int nt, long long n, long long chunk, double* __restrict__ partial,
-                   int* __restrict__ error) {
-    extern __shared__ __align__(1024) uint32_t sm[];
+// Gram tile of M rows (<= 128, the accumulator's lanes) and N rows (<= 256, its columns); either operand may
+// be the M side (swapped: B is).  grid = (M tiles, N tiles, chunks); dynamic smem = 2 stages x (M hi, M lo,
+// N hi, N lo).  A warp loads 32 points of one row, 256 contiguous bytes, and writes them as one
+// swizzled 128-byte row per plane, free of bank conflicts.  Only rows that exist are loaded and
+// split; the rest of the tile is zeroed once.  The products of a step go hi*hi, A hi * B lo, A lo * B hi on
+// either side, so an element's sum does not depend on the tiling.
+//
+// Bound by memory (each operand once where one tile holds the product) and the conversions.  138 x 69,
+// 112 x 97 x 101: 1500 -> 703 us.  A tile of 128 rows of A per block read B a second time for the ten
+// rows left over, split 512 rows of which 207 exist, and loaded and converted by turns.
+//
+// Two groups of eight warps take the slices in turn, each into its own stage, and a warp of its own issues the
+// products: one group's loads and barriers run under the other's conversions.  With all sixteen warps on every
+// slice, block barriers around it and core matrices without swizzle, 786 us.
+constexpr int TG_WARPS = 8;                          // per group
+constexpr int TG_THREADS = (2 * TG_WARPS + 1) * 32;  // and the issuing warp
+
+template <int PW>  // rows per warp, both sides
+__global__ void __launch_bounds__(TG_THREADS, 1)
+    gram_tc_kernel(const double* __restrict__ M, long long ldm, int km, const double* __restrict__ Nn, long long ldn,
+                   int kn, int nt, int ncols, int swapped, long long n, long long chunk, double* __restrict__ partial,
+                   int kb, int* __restrict__ error) {
+    extern __shared__ uint32_t sm_raw[];
+    uint32_t* const sm = (uint32_t*)(((uintptr_t)sm_raw + 1023) & ~(uintptr_t)1023);
     __shared__ uint32_t s_tmem;
-    __shared__ __align__(8) uint64_t bar[2];
-    constexpr int NW = TC_THREADS / 32;
-    constexpr int RA = TC_M / NW, RB = NC / NW;  // rows per warp
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __shared__ __align__(8) uint64_t full[2], bar[2];  // a stage is written; its products are done
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+    const int group = wid / TG_WARPS, warp = wid % TG_WARPS;  // group 2: the issuing warp
     const int m0 = blockIdx.x * TC_M, n0 = blockIdx.y * nt;
-    const int mrows = min(TC_M, ka - m0), nrows = min(nt, kb - n0);
+    const int mrows = min(TC_M, km - m0), nrows = min(nt, kn - n0);
+    const int rn = (nt + 15) / 16 * 16;  // columns of the MMA
     const long long p0 = (long long)blockIdx.z * chunk, p1 = min(n, p0 + chunk);
-    constexpr int a_words = TC_M * TC_KT, b_words = NC * TC_KT;
-    constexpr int stage_words = 2 * a_words + 2 * b_words;
-    // TMEM: NC fp32 columns x 128 lanes, allocated by warp 0
-    if (warp == 0) {
+    const int m_words = TC_M * TC_KT, n_words = rn * TC_KT, stage_words = 2 * m_words + 2 * n_words;
+    if (wid == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
-                     "r"(NC));
+                     "r"(ncols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int st = 0; st < 2; ++st) {
+            mbar_init(&full[st], TG_WARPS * 32);
+            mbar_init(&bar[st], 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    for (int w = tid; w < 2 * stage_words; w += TG_THREADS) sm[w] = 0;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
-    const uint32_t idesc = idesc_tf32(NC);
-    // Thread (warp, lane) owns element (row 8 rg + lane / 4, point 4 kg + lane % 4) of core
-    // matrix cm = warp + 8 i (rg = cm / 8, kg = cm % 8): a warp writes one whole 128-byte core
-    // matrix per store, so the shared-memory stores are free of bank conflicts.
-    double xa[RA], xb[RB];
-    const int lr = lane >> 2, lk = lane & 3;
-    auto load = [&](long long ps) {
+    const uint32_t idesc = idesc_tf32(rn);
+    // Slot i of a warp is M row warp + 8 i below `first`, then N row warp + 8 (i - first): every slot of a side is a
+    // fixed step from the last, in global and in shared memory (one atom).
+    const int first = (mrows + TG_WARPS - 1) / TG_WARPS;
+    const long long step_m = TG_WARPS * ldm, step_n = TG_WARPS * ldn;
+    const double* const at_m = M + (long long)(m0 + warp) * ldm + lane;
+    const double* const at_n = Nn + (long long)(n0 + warp) * ldn + lane;
+    const int end_m = mrows - warp, end_n = nrows - warp + TG_WARPS * first;  // slot i exists below these: 8 i
+    const int to_m = warp * TC_KT + (((lane >> 2) ^ warp) << 2) + (lane & 3);
+    const int to_n = 2 * m_words + to_m - TG_WARPS * TC_KT * first;
+    auto load = [&](double (&x)[PW], long long ps) {
+        const bool in = ps + lane < p1;
+        const double* q = at_m + ps;  // stepped: products with the slot's number would be kept, two registers each
+        long long step = step_m;
 #pragma unroll
-        for (int i = 0; i < RA; ++i) {
-            const int cm = warp + i * NW, r = (cm >> 3) * 8 + lr;
-            const long long pt = ps + (cm & 7) * 4 + lk;
-            xa[i] = (r < mrows && pt < p1) ? __ldg(A + (long long)(m0 + r) * lda + pt) : 0.0;
-        }
-#pragma unroll
-        for (int i = 0; i < RB; ++i) {
-            const int cm = warp + i * NW, r = (cm >> 3) * 8 + lr;
-            const long long pt = ps + (cm & 7) * 4 + lk;
-            xb[i] = (r < nrows && pt < p1) ? __ldg(B + (long long)(n0 + r) * ldb + pt) : 0.0;
+        for (int i = 0; i < PW; ++i) {
+            if (i == first) q = at_n + ps, step = step_n;
+            x[i] = in && TG_WARPS * i < (i < first ? end_m : end_n) ? __ldg(q) : 0.0;
+            q += step;
         }
     };
-    if (p0 < p1) load(p0);
     bool ok = true;
-    uint32_t phase[2] = {0, 0};
-    bool pending[2] = {false, false};
-    int step = 0;
-    for (long long ps = p0; ps < p1; ps += TC_KT, ++step) {
-        const int st = step & 1;
-        // the MMAs that last read this stage must be done before it is overwritten
-        if (pending[st]) {
-            if (!mbar_wait(&bar[st], phase[st])) ok = false;
-            phase[st] ^= 1;
-            pending[st] = false;
-        }
-        if (!__syncthreads_and(ok)) break;
-        uint32_t* ahi = sm + st * stage_words;
-        uint32_t* alo = ahi + a_words;
-        uint32_t* bhi = alo + a_words;
-        uint32_t* blo = bhi + b_words;
+    const int steps = p0 < p1 ? (int)((p1 - p0 + TC_KT - 1) / TC_KT) : 0;
+    if (group < 2) {
+        const int st = group;
+        double x[PW];
+        if (st < steps) load(x, p0 + st * TC_KT);
+        uint32_t* const stage = sm + st * stage_words;
+        uint32_t phase = 0;
+        for (int step = st; step < steps; step += 2) {
+            // the products that last read this stage must be done before it is overwritten
+            if (step >= 2) {
+                ok = mbar_wait(&bar[st], phase);
+                if (!ok) break;
+                phase ^= 1;
+            }
 #pragma unroll
-        for (int i = 0; i < RA; ++i) {
-            const int cm = warp + i * NW;
-            const uint32_t h = to_tf32((float)xa[i]);
-            const uint32_t l = to_tf32((float)(xa[i] - (double)__uint_as_float(h)));
-            const int o = (((cm & 7) * (TC_M / 8) + (cm >> 3)) << 5) + lane;  // = kmajor_offset_words(row, k, TC_M)
-            ahi[o] = h;
-            alo[o] = l;
+            for (int i = 0; i < PW; ++i) {
+                const bool side = i < first;
+                uint32_t h, l;
+                split_tf32(x[i], h, l);
+                uint32_t* o = stage + (side ? to_m : to_n) + TG_WARPS * TC_KT * i;
+                if (TG_WARPS * i < (side ? end_m : end_n)) {
+                    o[0] = h;
+                    o[side ? m_words : n_words] = l;
+                }
+            }
+            // generic-proxy smem writes -> visible to the tensor core (async proxy)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[st])) : "memory");
+            if (step + 2 < steps) load(x, p0 + (long long)(step + 2) * TC_KT);
         }
-#pragma unroll
-        for (int i = 0; i < RB; ++i) {
-            const int cm = warp + i * NW;
-            const uint32_t h = to_tf32((float)xb[i]);
-            const uint32_t l = to_tf32((float)(xb[i] - (double)__uint_as_float(h)));
-            const int o = (((cm & 7) * (NC / 8) + (cm >> 3)) << 5) + lane;
-            bhi[o] = h;
-            blo[o] = l;
-        }
-        // generic-proxy smem writes -> visible to the tensor core (async proxy)
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+    } else if (lane == 0) {
+        int issued[2] = {0, 0};
+        for (int step = 0; step < steps; ++step) {
+            const int st = step & 1;
+            ok = mbar_wait(&full[st], issued[st] & 1);
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            constexpr uint32_t lbo_a = (TC_M / 8) * 128, lbo_b = (uint32_t)(NC / 8) * 128, sbo = 128;
-            const uint32_t sa_hi = smem_u32(ahi), sa_lo = smem_u32(alo), sb_hi = smem_u32(bhi), sb_lo = smem_u32(blo);
+            const uint32_t sm_hi = smem_u32(sm + st * stage_words), sm_lo = sm_hi + 4 * m_words;
+            const uint32_t sn_hi = sm_lo + 4 * m_words, sn_lo = sn_hi + 4 * n_words;
 #pragma unroll
             for (int kk = 0; kk < TC_KT / 8; ++kk) {
-                // K = 8 tf32 = two 4-element core-matrix columns
-                const uint32_t oa = kk * 2 * lbo_a, ob = kk * 2 * lbo_b;
-                const uint64_t dah = smem_desc(sa_hi + oa, lbo_a, sbo), dal = smem_desc(sa_lo + oa, lbo_a, sbo);
-                const uint64_t dbh = smem_desc(sb_hi + ob, lbo_b, sbo), dbl = smem_desc(sb_lo + ob, lbo_b, sbo);
-                const uint32_t first = (step == 0 && kk == 0) ? 0u : 1u;
-                mma_tf32(tmem, dah, dbh, idesc, first);
-                mma_tf32(tmem, dah, dbl, idesc, 1u);
-                mma_tf32(tmem, dal, dbh, idesc, 1u);
+                const uint32_t o = kk * 32;  // K = 8 tf32
+                const uint64_t dmh = smem_desc_128(sm_hi + o), dml = smem_desc_128(sm_lo + o);
+                const uint64_t dnh = smem_desc_128(sn_hi + o), dnl = smem_desc_128(sn_lo + o);
+                mma_tf32(tmem, dmh, dnh, idesc, step == 0 && kk == 0 ? 0u : 1u);
+                mma_tf32(tmem, swapped ? dml : dmh, swapped ? dnh : dnl, idesc, 1u);
+                mma_tf32(tmem, swapped ? dmh : dml, swapped ? dnl : dnh, idesc, 1u);
             }
             mma_commit(&bar[st]);
+            ++issued[st];
         }
-        pending[st] = true;
-        // the next slice's loads overlap the MMAs just issued
-        if (ps + TC_KT < p1) load(ps + TC_KT);
+        // drain: the last products of each stage (those before are done: the stage was written again)
+        for (int st = 0; st < 2; ++st)
+            if (issued[st] > 0 && !mbar_wait(&bar[st], (issued[st] - 1) & 1)) ok = false;
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
-    // drain: wait (bounded) for every stage that still has MMAs in flight
-    for (int st = 0; st < 2; ++st)
-        if (pending[st]) {
-            if (!mbar_wait(&bar[st], phase[st])) ok = false;
-            phase[st] ^= 1;
-        }
+    __syncwarp();
     ok = __syncthreads_and(ok);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // M row m0 + r lives in TMEM lane r: warp w reads lanes 32 (w % 4) .. +31; w / 4 picks the
+    // columns
+    double* out = partial + (long long)blockIdx.z * km * kn;
+    auto put = [&](int r, int c, double v) {
+        out[swapped ? (long long)(n0 + c) * kb + m0 + r : (long long)(m0 + r) * kb + n0 + c] = v;
+    };
     if (!ok) {
         if (tid == 0) atomicExch(error, 1);
-    } else if (step > 0) {
-        // accumulator row r = A vector m0 + r lives in TMEM lane r: warp w reads lanes
-        // 32 (w % 4) .. +31; warps w and w + 4 split the columns
-        double* out = partial + (long long)blockIdx.z * ka * kb;
-        const int q4 = warp & 3, half = warp >> 2;
-        const int row = q4 * 32 + lane;
-        constexpr int CH = NC / (NW / 4);
-        for (int c0 = half * CH; c0 < half * CH + CH; c0 += 8) {
+    } else if (p0 < p1 && group < 2) {
+        const int q4 = wid & 3, row = q4 * 32 + lane;
+        for (int c0 = (wid >> 2) * 8; c0 < nrows; c0 += 2 * TG_WARPS / 4 * 8) {
             uint32_t v[8];
             const uint32_t addr = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)c0;
             asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -238,17 +266,39 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             if (row < mrows)
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
-                    if (c0 + q < nrows) out[(long long)(m0 + row) * kb + (n0 + c0 + q)] = (double)__uint_as_float(v[q]);
+                    if (c0 + q < nrows) put(row, c0 + q, (double)__uint_as_float(v[q]));
         }
-    } else {
+    } else if (p0 >= p1) {
         // empty K range: this block contributes zeros
-        double* out = partial + (long long)blockIdx.z * ka * kb;
-        for (int e = tid; e < mrows * nrows; e += TC_THREADS)
-            out[(long long)(m0 + e / nrows) * kb + (n0 + e % nrows)] = 0.0;
+        for (int e = tid; e < mrows * nrows; e += TG_THREADS) put(e / nrows, e % nrows, 0.0);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NC));
+    if (wid == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
+}
+
+// Launches the Gram tiles with the operand on the M side that takes fewer of them.
+void gram_tiles(dft_context* ctx, const double* A, long long lda, int ka, const double* B, long long ldb, int kb,
+                long long n, long long chunk, long long nch, double* partial, int* err) {
+    const auto up = [](int a, int b) { return (a + b - 1) / b; };
+    const bool swapped = up(kb, TC_M) * up(ka, TC_NMAX) < up(ka, TC_M) * up(kb, TC_NMAX);
+    const int km = swapped ? kb : ka, kn = swapped ? ka : kb;
+    const int mt = up(km, TC_M), nts = up(kn, TC_NMAX), nt = up(kn, nts);
+    int ncols = 32;
+    while (ncols < nt) ncols <<= 1;
+    const size_t smem = sizeof(uint32_t) * 2 * 2 * TC_KT * ((size_t)TC_M + up(nt, 16) * 16) + 1024;
+    const int per = up(std::min(km, TC_M), TG_WARPS) + up(nt, TG_WARPS);  // at most 16 + 32
+    const auto launch = [&](auto kernel) {
+        DFT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        kernel<<<dim3(mt, nts, (unsigned)nch), TG_THREADS, smem, ctx->stream>>>(
+            swapped ? B : A, swapped ? ldb : lda, km, swapped ? A : B, swapped ? lda : ldb, kn, nt, ncols, swapped, n,
+            chunk, partial, kb, err);
+    };
+    if (per <= 10) launch(gram_tc_kernel<10>);
+    else if (per <= 18) launch(gram_tc_kernel<18>);
+    else if (per <= 27) launch(gram_tc_kernel<27>);
+    else if (per <= 36) launch(gram_tc_kernel<36>);
+    else launch(gram_tc_kernel<48>);
 }
 
 // Ring variant of the Gram tile (tuning key "tensor_core_ring"): the FP64 slices are staged
@@ -781,7 +831,6 @@ void gram_tc(dft_context* ctx, const Grid& g, const double* A, long long lda, in
     int ncols = 32;
     while (ncols < nt) ncols <<= 1;
     const int mtiles = (ka + TC_M - 1) / TC_M;
-    const size_t smem = sizeof(uint32_t) * 2 * (size_t)(2 * TC_M * TC_KT + 2 * ncols * TC_KT);
     // split K so that each block accumulates <= 8192 points in FP32 and the machine is covered
     long long nch = std::max<long long>(1, (2LL * ctx->num_sms) / (mtiles * ntiles));
     nch = std::max<long long>(nch, (g.N + 8191) / 8192);
@@ -792,14 +841,6 @@ void gram_tc(dft_context* ctx, const Grid& g, const double* A, long long lda, in
     double* partial = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * (nel * nch + nel) + 64);
     double* res = partial + nel * nch;
     int* err = (int*)(res + nel);
-    static bool attr = false;
-    if (!attr) {
-        DFT_CUDA(cudaFuncSetAttribute(gram_tc_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        DFT_CUDA(cudaFuncSetAttribute(gram_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        DFT_CUDA(cudaFuncSetAttribute(gram_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        DFT_CUDA(cudaFuncSetAttribute(gram_tc_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr = true;
-    }
     DFT_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
     const bool tma = ctx->tc_tma && lda % 2 == 0 && ldb % 2 == 0 && ((uintptr_t)A & 15) == 0 &&
                      ((uintptr_t)B & 15) == 0 && tensor_map_encoder() != nullptr;
@@ -865,23 +906,8 @@ void gram_tc(dft_context* ctx, const Grid& g, const double* A, long long lda, in
         else
             gram_tc_ring_kernel<128><<<grid, TC_THREADS, ring_smem<128>(), ctx->stream>>>(A, lda, ka, B, ldb, kb, nt,
                                                                                          g.N, chunk, partial, err);
-    } else switch (ncols) {
-        case 32:
-            gram_tc_kernel<32><<<grid, TC_THREADS, smem, ctx->stream>>>(A, lda, ka, B, ldb, kb, nt, g.N, chunk,
-                                                                        partial, err);
-            break;
-        case 64:
-            gram_tc_kernel<64><<<grid, TC_THREADS, smem, ctx->stream>>>(A, lda, ka, B, ldb, kb, nt, g.N, chunk,
-                                                                        partial, err);
-            break;
-        case 128:
-            gram_tc_kernel<128><<<grid, TC_THREADS, smem, ctx->stream>>>(A, lda, ka, B, ldb, kb, nt, g.N, chunk,
-                                                                         partial, err);
-            break;
-        default:
-            gram_tc_kernel<256><<<grid, TC_THREADS, smem, ctx->stream>>>(A, lda, ka, B, ldb, kb, nt, g.N, chunk,
-                                                                         partial, err);
-            break;
+    } else {
+        gram_tiles(ctx, A, lda, ka, B, ldb, kb, g.N, chunk, nch, partial, err);
     }
     DFT_LAUNCH_CHECK();
     const int rb = (int)std::min<size_t>((nel + 7) / 8, 4096);
