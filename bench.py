@@ -265,11 +265,10 @@ def measure_jacobi(eng, torch, stream, w):
     interior = (nx - 2) * (ny - 2) * (nz - 2)
     bytes_per_sweep = 24.0 * interior
     # the launch shape the library picks by default (grid_ops.cu: hartree)
-    pmax = (nz + 15) // 16
-    if nz >= 32 and 3 * pmax * nx * ny * 8 <= 200 * 1024:
-        kernel, spl, note = ("jacobi_cluster_kernel", sweeps,
-                             "whole solve in one launch; V, V', rho live in the shared memory of a 16-block "
-                             "cluster, so HBM is not the binding resource (latency/FP64 bound)")
+    if nx * ny * nz <= 64 ** 3:
+        kernel, spl, note = ("jacobi_resident_kernel", sweeps,
+                             "whole solve in one launch; V, V', rho live in the shared memory of all SMs, so HBM is "
+                             "not the binding resource (exchange latency bound)")
     else:
         kernel, spl, note = "jacobi_sweep_kernel", 1, "one sweep per launch"
     return {"sweeps": sweeps, "ms_per_sweep": ms / sweeps, "bytes_per_sweep": bytes_per_sweep,
@@ -279,8 +278,8 @@ def measure_jacobi(eng, torch, stream, w):
 
 def measure_gram(eng, torch, stream, w, ka, kb, reps=20):
     """The eigensolver's FP64 Gram product at the workload's grid with the basis/new-block
-    widths of its Davidson iterations (narrow blocks: gram_small_kernel, one launch with the
-    reduction done by the last block).  Algorithmic bytes per call = N (ka + kb) 8."""
+    widths of its Davidson iterations (narrow blocks: gram_lanes_kernel or gram_chunk_kernel and
+    their sums).  Algorithmic bytes per call = N (ka + kb) 8."""
     import dft_b200
     g = dft_b200.CartesianGrid(*w["n"], *w["bounds"])
     N = g.getSize()

@@ -62,9 +62,10 @@ dft_status_t dft_context_destroy(dft_context* ctx);
  * stays usable. */
 dft_status_t dft_context_synchronize(dft_context* ctx);
 /* Kernel-shape knobs.  Keys:
- *   "jacobi_sweeps_per_launch": 0 = auto (default), -2 = the whole solve in the shared memory
- *                               of one 16-block cluster (small grids), -1 = the whole solve in
- *                               one persistent (cooperative) launch, 1 = one sweep per launch,
+ *   "jacobi_sweeps_per_launch": 0 = auto (default: as -1 for small grids), -2 = the whole solve in
+ *                               the shared memory of one 16-block cluster (small grids), -1 =
+ *                               the whole solve in one cooperative launch (in the shared memory
+ *                               of all SMs where the grid fits), 1 = one sweep per launch,
  *                               2, 4 or 8 = temporally blocked sweeps per launch (results are
  *                               identical for every value).
  *   "network_tensor_cores":     1 (default) = the Poisson-start network's 16- and 32-channel
@@ -75,10 +76,10 @@ dft_status_t dft_context_synchronize(dft_context* ctx);
  *                               "hpsi_variant" = 2 the bands (1, 2, 4, 8) each block walks
  *                               (results identical for every value).
  *   "multigrid_graphs":         1 (default) = each Poisson multigrid cycle is captured once per
- *                               grid and buffers as a CUDA graph and replayed; 0 = launched kernel
- *                               by kernel (same results).
- *   "tensor_core_ring":         0 (default) = the tensor-core Gram product stages its FP64 slices
- *                               through registers; 1 = through a 2-deep cp.async shared-memory
+ *                               grid and direction as a CUDA graph and replayed; 0 = launched
+ *                               kernel by kernel (same results).
+ *   "tensor_core_ring":         0 (default) = the tensor-core Gram product takes its FP64 slices
+ *                               through registers, two warp groups in turn; 1 = through a 2-deep cp.async shared-memory
  *                               ring (even leading dimensions, 16-byte-aligned blocks, <= 128
  *                               columns per tile; otherwise the register path).  Same results.
  *   "tensor_core_tma":          0 (default) = as "tensor_core_ring" says; 1 = the tensor-core Gram
@@ -87,7 +88,8 @@ dft_status_t dft_context_synchronize(dft_context* ctx);
  *                               256-column tiles) and splits them from shared memory (even
  *                               leading dimensions, 16-byte-aligned blocks; otherwise the other
  *                               paths).  Same accuracy class (TF32 hi+lo, FP32 accumulation).
- *   "hpsi_variant":             0 (default) = the H psi kernel reads x/y neighbours through L1;
+ *   "hpsi_variant":             0 (default) = the H psi kernel reads x/y neighbours through L1
+ *                               (two columns per thread where rows and arrays allow 16-byte loads);
  *                               1 = through a shared-memory plane tile (at most 2 bands per
  *                               thread); 2 = plane tiles with their halo loaded by TMA
  *                               (cp.async.bulk.tensor) into a 6-stage shared-memory ring, each
@@ -100,8 +102,9 @@ dft_status_t dft_context_synchronize(dft_context* ctx);
  *                               fails with DFT_CUDA_ERROR and the context stays usable.
  *   "hpsi_zchunk":              0 = auto (default), else the number of z-planes each block of the
  *                               register-march H psi kernels walks (same results for every value).
- *   "multigrid_fused_restriction": 1 (default) = the Poisson multigrid restricts in one 3-D pass
- *                               on fine grids up to 64^3 (0: three separable passes).
+ *   "multigrid_fused_restriction": 1 (default) = the Poisson multigrid's passes are fused and its
+ *                               restriction is one 3-D pass (0: separate passes, three of them
+ *                               for the restriction).
  *   "multigrid_coarsest_sor":   1 (default) = the coarsest multigrid level is solved by red-black
  *                               SOR at the optimal relaxation (0: 8 Jacobi sweeps per point of the
  *                               longest axis).
