@@ -215,7 +215,8 @@ __global__ void __launch_bounds__(HB_X* HB_Y) hpsi1_kernel(Grid g, const double*
 // The same for even row lengths and 16-byte aligned arrays: a thread takes two columns with 16-byte loads, half
 // the load instructions per byte and half as much again in flight (more planes per thread instead cost
 // occupancy: 480 to 520 us).  Bound by memory: psi once, H psi once, V about once.  192^3, 16
-// bands: 484 -> 409 us.
+// bands: 484 -> 409 us, and 412 -> 390 (both timed in turn) with psi's plane after next on its way to the L2, which
+// costs no registers; V as well, or further ahead, is slower.
 constexpr int HP_BLOCKS = 6;  // per SM: 40 registers
 __global__ void __launch_bounds__(256, HP_BLOCKS)
     hpsi_pair_kernel(Grid g, const double* __restrict__ V, const double* __restrict__ psi, double* __restrict__ out,
@@ -237,6 +238,7 @@ __global__ void __launch_bounds__(256, HP_BLOCKS)
     double2 cur = two(p);
     for (int k = kb; k < ke; ++k) {
         const bool zl = k > 0, zr = k + 1 < g.nz;
+        if (k + 2 < min(ke + 1, g.nz)) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 2LL * sxy));
         const double2 ab = zr ? two(p + sxy) : make_double2(0.0, 0.0);
         const double2 w = two(v), ym = two(p + oyl), yp = two(p + oyr);
         const double xm = __ldg(p + oxl), xp = __ldg(p + oxr);
