@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(CBX* CBY) mg_interpolate_kernel(Grid f, Grid c
 // sweep is six reads, a handful of FP64 operations and a barrier (it was integer divisions, an FP64
 // division and a global read per point: 32 us for 9^3, 7 here).
 template <int K>
-__device__ void sor_block(const Grid& g, const double* src, double* e, int sweeps, double omega, double* x) {
+__device__ void sor_block(const Grid& g, const double* src, double s, double* e, int sweeps, double omega, double* x) {
     const int n = (int)g.N, nt = blockDim.x, sxy = g.nx * g.ny;
     for (int p = threadIdx.x; p < n; p += nt) x[p] = 0.0;
     const double den = 2.0 * (g.ix2 + g.iy2 + g.iz2), inv = 1.0 / den;
@@ -394,10 +394,10 @@ __device__ void sor_block(const Grid& g, const double* src, double* e, int sweep
             const int i = 1 + 2 * (r % half) + ((1 + j + k + c) & 1);
             if (i > g.nx - 2) continue;
             at[c][q] = (k * g.ny + j) * g.nx + i;
-            b[c][q] = __ldcg(src + at[c][q]);
+            b[c][q] = s * __ldcg(src + at[c][q]);
         }
     __syncthreads();
-    for (int s = 0; s < sweeps; ++s)
+    for (int it = 0; it < sweeps; ++it)
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
 #pragma unroll
@@ -415,10 +415,10 @@ __device__ void sor_block(const Grid& g, const double* src, double* e, int sweep
 }
 
 template <int K>
-__global__ void __launch_bounds__(1024) mg_coarsest_sor_kernel(Grid g, const double* __restrict__ src,
+__global__ void __launch_bounds__(1024) mg_coarsest_sor_kernel(Grid g, const double* __restrict__ src, double s,
                                                                double* __restrict__ e, int sweeps, double omega) {
     extern __shared__ double sm[];
-    sor_block<K>(g, src, e, sweeps, omega, sm);
+    sor_block<K>(g, src, s, e, sweeps, omega, sm);
 }
 
 // Doubles of shared memory that jacobi_block uses: two iterates with a border of zeros.
@@ -811,14 +811,15 @@ void sor_parameters(const Grid& g, double* omega, int* sweeps) {
 }
 
 template <int K>
-void coarsest_sor_launch(dft_context* ctx, const MGLevel& l, const double* src, int sweeps, double omega, int threads) {
+void coarsest_sor_launch(dft_context* ctx, const MGLevel& l, const double* src, double s, int sweeps, double omega,
+                         int threads) {
     const size_t smem = sizeof(double) * (size_t)l.g.N;
     DFT_CUDA(cudaFuncSetAttribute(mg_coarsest_sor_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(sizeof(double) * MG_COARSEST_MAX)));
-    mg_coarsest_sor_kernel<K><<<1, threads, smem, ctx->stream>>>(l.g, src, l.v, sweeps, omega);
+    mg_coarsest_sor_kernel<K><<<1, threads, smem, ctx->stream>>>(l.g, src, s, l.v, sweeps, omega);
 }
 
-// l.v = the coarsest level's solution for src (scale 1)
+// l.v = the coarsest level's solution for s src
 void coarsest(dft_context* ctx, const MGLevel& l, const double* src, const int* map, int open, double s,
               const double* shift, int nb, bool sor) {
     const Grid& g = l.g;
@@ -829,9 +830,9 @@ void coarsest(dft_context* ctx, const MGLevel& l, const double* src, const int* 
         const int total = (g.nx - 1) / 2 * (g.ny - 2) * (g.nz - 2);
         const int threads = std::max(32, std::min(1024, (total + 31) / 32 * 32));
         const int k = (total + threads - 1) / threads;
-        if (k <= 1) coarsest_sor_launch<1>(ctx, l, src, sweeps, omega, threads);
-        else if (k <= 2) coarsest_sor_launch<2>(ctx, l, src, sweeps, omega, threads);
-        else coarsest_sor_launch<6>(ctx, l, src, sweeps, omega, threads);
+        if (k <= 1) coarsest_sor_launch<1>(ctx, l, src, s, sweeps, omega, threads);
+        else if (k <= 2) coarsest_sor_launch<2>(ctx, l, src, s, sweeps, omega, threads);
+        else coarsest_sor_launch<6>(ctx, l, src, s, sweeps, omega, threads);
     } else {
         const int sweeps = 8 * std::max({g.nx, g.ny, g.nz});
         // three points a thread: independent chains, and a barrier of few warps (9^3: 8)

@@ -508,7 +508,7 @@ int multigrid(dft_context* ctx, const Grid& g, const double* rho, double* v, dou
         }
         c += m;
         // a single level is solved from zero: every further cycle would repeat this one
-        if (L.size() == 1 && !met) c = max_cycles;
+        if (L.size() == 1) break;
     }
     if (c > 0) DFT_CUDA(cudaMemcpyAsync(v, buf[cur], bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     if (resid_out) *resid_out = r;
