@@ -970,13 +970,18 @@ void configuration(int Z, std::vector<std::array<int, 4>>& rows) {
 
 namespace {
 
+constexpr long RADIAL_MAX_POINTS = 12000;
+constexpr size_t radial_smem(long points) {  // at most 175 KB
+    return sizeof(double) * ((size_t)(points + 1) / 2 * 2 + (size_t)RW * WARP_STAGE);
+}
+
 // Builds the run specs, launches the batch and leaves every run's arrays in the WS_RADIAL
 // workspace (returned; per_run doubles per run: A_* per block, then at `orbitals` MAXORB x O_*).
 double* run_batch(dft_context* ctx, int nruns, const int* Z, const int* kinds, long points, double rmax,
                   dft_atom_result* results, std::vector<RunSpec>& specs, long long& per_run,
                   long long& orbitals) {
     if (points < 2) fail(DFT_INVALID_ARGUMENT, "La malla radial debe contener al menos dos puntos.");
-    if (points > 12000) fail(DFT_INVALID_ARGUMENT, "at most 12000 radial points per run");
+    if (points > RADIAL_MAX_POINTS) fail(DFT_INVALID_ARGUMENT, "at most %ld radial points per run", RADIAL_MAX_POINTS);
     if (!(rmax > 0.0)) fail(DFT_INVALID_ARGUMENT, "RMAX debe ser mayor que cero.");
     specs.assign(nruns, RunSpec{});
     for (int rr = 0; rr < nruns; ++rr) {
@@ -1016,8 +1021,11 @@ double* run_batch(dft_context* ctx, int nruns, const int* Z, const int* kinds, l
     dft_atom_result* dres = (dft_atom_result*)(dbuf + spec_bytes);
     DFT_CUDA(cudaMemcpyAsync(dspec, specs.data(), sizeof(RunSpec) * nruns, cudaMemcpyHostToDevice, ctx->stream));
     DFT_CUDA(cudaMemsetAsync(dres, 0, sizeof(dft_atom_result) * nruns, ctx->stream));
-    const size_t smem = sizeof(double) * ((size_t)(points + 1) / 2 * 2 + (size_t)RW * WARP_STAGE);  // at most 175 KB
-    DFT_CUDA(cudaFuncSetAttribute(radial_scf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // The limit is the process's, not the context's: the same value from every thread, so that none lowers it
+    // between another's two calls.
+    const size_t smem = radial_smem(points);
+    DFT_CUDA(cudaFuncSetAttribute(radial_scf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)radial_smem(RADIAL_MAX_POINTS)));
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = cl;
