@@ -5,9 +5,13 @@
 // Here every power of 1 +- z comes from one cube root each, those of the density from one, and quotients by
 // the same value share a reciprocal: 5 cube roots, 4 logarithms, 10 divisions.  z is still the
 // correctly rounded quotient and 1 +- z are rounded as before, because (1 - z)^(1/3) turns on their last bit where
-// the density is nearly polarised.  Potentials against an independent evaluation: 2e-15 of
-// their norm (plain: 1.3e-15 to 2.4e-15).  Points whose intermediates could leave the range of the rearranged
-// products (extreme gradients, vanishing spin densities) return false and take the plain functional.
+// the density is nearly polarised.  A product with a rounded reciprocal is a rounding more than the quotient it
+// stands for; where that reaches the results its remainder goes back in (quotient, dg), and small terms are
+// summed before they meet the large ones.  On the device, against an 80-bit evaluation, rms over densities of 1e-3 to
+// 10 and all polarisations, relative to the plain functional's: PBE eps 0.91 to 0.98, potentials 0.89
+// to 1.00, gradient coefficients 0.88 to 1.00; PZ81 eps 0.93 to 1.02, potentials 0.94 to 1.02.  Points whose
+// intermediates could leave the range of the rearranged products (extreme gradients, vanishing spin
+// densities) return false and take the plain functional.
 #pragma once
 
 #include "xc_device.cuh"
@@ -17,11 +21,15 @@ namespace xcf {
 
 constexpr double RS_C = 0.62035049089940001667;     // (3 / (4 pi))^(1/3)
 constexpr double RS_C_INV = 1.6119919540164696407;  // its reciprocal
-constexpr double IKS = 0.63971943089250433554;      // 1 / sqrt(4 kf / pi) = IKS sqrt(rs)
+constexpr double IKS2 = 0.40924095026142963;       // pi / (4 kf) = IKS2 rs
 
+// a / n from inv = 1 / n, the product's rounding taken out by the remainder
+__device__ __forceinline__ double quotient(double a, double n, double inv) {
+    const double q = a * inv;
+    return fma(fma(-n, q, a), inv, q);
+}
 __device__ __forceinline__ double polarisation(double a, double b, double n, double inv) {
-    const double d = a - b, q = d * inv;
-    return clamp1(fma(fma(-n, q, d), inv, q));
+    return clamp1(quotient(a - b, n, inv));
 }
 
 __device__ __forceinline__ bool pz81_fast(double na_in, double nb_in, Result& r) {
@@ -79,15 +87,18 @@ __device__ __forceinline__ double gcor2_fast(double a, double a1, double b1, dou
 __device__ __forceinline__ bool pbe_exchange_fast(double rho, double r13, double g, double& ed, double& dn, double& dg) {
     ed = dn = dg = 0.0;
     if (rho <= 0.0) return true;
-    constexpr double MK = MU / KAPPA;
-    const double exu = EXCHANGE_A * r13, den = 2.0 * KF_COEFFICIENT * r13 * rho;
-    const double d2 = den * den, g2 = g * g, t = fma(MK, g2, d2);
+    constexpr double MK = MU / KAPPA, TWO_KAPPA = 2.0 * KAPPA;
+    const double den = 2.0 * KF_COEFFICIENT * r13 * rho;
+    const double d2 = den * den, mg = MK * g, mg2 = mg * g, t = fma(mg, g, d2);
     if (!(rho >= 1e-30 && t <= 1e150)) return false;
-    const double ip = 1.0 / t, i0 = d2 * ip;        // 1 / (1 + mk s^2)
-    const double fx = 1.0 + KAPPA - KAPPA * i0;
-    dn = exu * FOUR_THIRDS * (fx - g2 * ip * (2.0 * KAPPA * MK) * i0);
-    dg = EXCHANGE_A * 0.161620459673995 * g * den * ip * (2.0 * KAPPA * MK) * i0;
-    ed = rho * exu * fx;
+    const double ip = 1.0 / t, i0 = d2 * ip, w = mg2 * ip;  // 1 / (1 + mk s^2), mk s^2 / (1 + mk s^2)
+    const double fx = fma(KAPPA, w, 1.0);
+    dn = EXCHANGE_A * FOUR_THIRDS * r13 * fma(-TWO_KAPPA * w, i0, fx);
+    // 1 / t enters twice: what its rounding and t's left out
+    const double e = fma(-fma(mg, g, d2 - t), ip, fma(-t, ip, 1.0));
+    const double d = EXCHANGE_A * 0.161620459673995 * TWO_KAPPA * MK * g * (den * ip) * i0;
+    dg = fma(d, e + e, d);
+    ed = rho * (EXCHANGE_A * r13 * fx);
     return true;
 }
 
@@ -116,9 +127,10 @@ __device__ __forceinline__ bool pbe96_fast(double na_in, double nb_in, double ga
     const double gm = fabs(ga + gb);
     const double rs = RS_C / n13, srs = sqrt(rs), isr = srs * n13 * RS_C_INV;
     const double pa2 = pa * pa, pb2 = pb * pb;
-    const double phi = 0.5 * (pa2 + pb2), iphi = 1.0 / phi;
-    const double itkp = 0.5 * IKS * srs * iphi;
-    const double t = gm * itkp * inv;
+    const double phi = 0.5 * (pa2 + pb2), phi2 = phi * phi, phi3 = phi2 * phi;
+    const double iphi3 = 1.0 / phi3, iphi = phi2 * iphi3;
+    const double gn = quotient(gm, n, inv);
+    const double itkp2 = 0.25 * IKS2 * rs * (phi * iphi3);  // 1 / (2 ks phi)^2
     double eud, epd, ad;
     const double eu = gcor2_fast(0.0310907, 0.21370, 7.5957, 3.5876, 1.6382, 0.49294, srs, isr, eud);
     const double ep = gcor2_fast(0.01554535, 0.20548, 14.1189, 6.1977, 3.3662, 0.62517, srs, isr, epd);
@@ -132,12 +144,11 @@ __device__ __forceinline__ bool pbe96_fast(double na_in, double nb_in, double ga
     const double fz = FOUR_THIRDS / SPIN_GAMMA * (pa - pb);
     const double alz = al * IFZZ;
     const double ecz = 4.0 * z * z2 * f * (ep - eu + alz) + fz * (z4 * (ep - eu) - (1.0 - z4) * alz);
-    const double phi3 = phi * phi * phi, iphi3 = iphi * iphi * iphi;
     const double ex = -ec * (1.0 / GAMMA) * iphi3;
     const double em1 = expm1(ex);
     ok &= ex < 600.0 && em1 > 1e-200;
     const double bb = DELTA / em1, fac = em1 + 1.0;
-    const double b2 = bb * bb, t2 = t * t, t4 = t2 * t2, t6 = t4 * t2;
+    const double b2 = bb * bb, t2 = gn * gn * itkp2, t4 = t2 * t2, t6 = t4 * t2;
     const double bt2 = bb * t2, q4 = 1.0 + bt2, q5 = 1.0 + bt2 + b2 * t4;
     const double dq = DELTA * q4 * t2, q58 = q5 + dq, q8 = q5 * q58;
     ok &= q8 < 1e250 && b2 < 1e250;
@@ -146,18 +157,18 @@ __device__ __forceinline__ bool pbe96_fast(double na_in, double nb_in, double ga
     const double b2f = b2 * fac * (1.0 / BETA) * iphi3, bec = b2f;
     const double hb = -BETA * phi3 * bb * t6 * (2.0 + bt2) * i8;
     const double hrs = -(rs * THIRD) * hb * bec * ecrs;
-    const double ht = 2.0 * BETA * phi3 * (1.0 + 2.0 * bt2) * i8;
+    const double ht = quotient(2.0 * BETA * phi3 * (1.0 + 2.0 * bt2), q8, i8);
     const double comm = h + hrs - (7.0 / 6.0) * t2 * ht;
     const double gz = (ma - mb) * THIRD;
     const double bg = -3.0 * b2f * ec * iphi;
     const double hz = 3.0 * gz * h * iphi + hb * (bg * gz + bec * ecz);
     const double pref = hz - gz * t2 * ht * iphi;
     const double common = ec - rs * ecrs * THIRD - z * ecz;
-    const double dgc = gm > 0.0 ? t * ht * itkp : 0.0;
+    const double dgc = gm > 0.0 ? gn * itkp2 * ht : 0.0;
 
-    r.eps = 0.5 * (eda + edb) * inv + ec + h;
-    r.va = dna + common + ecz + comm + pref * omz;
-    r.vb = dnb + common - ecz + comm - pref * opz;
+    r.eps = 0.5 * quotient(eda + edb, n, inv) + (ec + h);
+    r.va = dna + (common + ecz + comm + pref * omz);
+    r.vb = dnb + (common - ecz + comm - pref * opz);
     const double cs = sign_of(ga + gb);
     r.ca = dga * sign_of(ga) + dgc * cs;
     r.cb = dgb * sign_of(gb) + dgc * cs;
