@@ -171,11 +171,21 @@ void screened_poisson_vcycle(dft_context* ctx, const Grid& g, const double* src,
     double* shift = (double*)ws_get(ctx, WS_PG3, sizeof(double) * (size_t)nb + 64);
     pc_fill_kernel<<<(nb + 127) / 128, 128, 0, ctx->stream>>>(nb, q2, shift);
     count_launch(ctx);
+    // a cycle reads its right-hand side while it writes x, and the refinement reads it again: a caller's
+    // source that x overlaps is copied first
+    const size_t block = (size_t)nb * ld;
+    const bool overlap = src < x + block && x < src + block;
+    const size_t fields = (cycles > 1 ? 2 : 0) + (overlap ? 1 : 0);
+    double* scratch = fields ? (double*)ws_get(ctx, WS_PG4, sizeof(double) * fields * block) : nullptr;
+    if (overlap) {
+        double* copy = scratch + (fields - 1) * block;
+        DFT_CUDA(cudaMemcpyAsync(copy, src, sizeof(double) * (block - ld + g.N), cudaMemcpyDeviceToDevice, ctx->stream));
+        src = copy;
+    }
     vcycle_batch(ctx, g, src, nullptr, nb, shift, 1.0, x, ld);
     if (cycles == 1) return;
     // iterative refinement: res = src - (-lap + q2) x, e = V-cycle(res), x += e
-    double* scratch = (double*)ws_get(ctx, WS_PG4, sizeof(double) * 2 * (size_t)nb * ld);
-    double *res = scratch, *e = scratch + (size_t)nb * ld;
+    double *res = scratch, *e = scratch + block;
     for (int c = 1; c < cycles; ++c) {
         const ColShape cs = col_shape(ctx, g, nb);
         pc_residual_kernel<<<cs.grid, cs.block, 0, ctx->stream>>>(g, ld, src, 1.0, shift, x, res, cs.zc, cs.nzc);
