@@ -169,6 +169,9 @@ _SIGS = {
     "dft_scf_default_options": ([C.POINTER(dft_scf_opts)], None),
     "dft_scf_molecule": ([_P, C.POINTER(dft_grid), C.c_int, C.POINTER(C.c_int), _D, C.c_int, C.c_int, C.c_int,
                           C.POINTER(dft_scf_opts), C.POINTER(dft_scf_result)], C.c_int),
+    "dft_radial_quotients_dev": ([_P, C.c_long, _P, _P, _P], C.c_int),
+    "dft_radial_tridiagonal_dev": ([_P, C.c_long, _P, C.c_double, C.c_double, _P, _P, _P, _P, C.c_int, _P, _P],
+                                   C.c_int),
     "dft_solve_atoms": ([_P, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int), C.c_long, C.c_double,
                          C.POINTER(dft_atom_result)], C.c_int),
     "dft_hartree_from_guess_dev": ([_P, C.POINTER(dft_grid), _P, _P, C.c_double, C.c_long, C.POINTER(C.c_long),
@@ -548,6 +551,16 @@ class Engine:
         _check(load().dft_solve_atoms(self.ctx, n, Za.ctypes.data_as(C.POINTER(C.c_int)),
                                       Ka.ctypes.data_as(C.POINTER(C.c_int)), points, rmax, out))
         return [AtomResult.from_c(o) for o in out]
+
+    def radial_quotients(self, m, a, g, out):
+        """out = a / g as the radial solver's chains take it (exposed for testing)."""
+        _check(load().dft_radial_quotients_dev(self.ctx, int(m), _ptr(a), _ptr(g), _ptr(out)))
+
+    def radial_tridiagonal(self, n, diag, off, shift, u, f, w, x, m, E, counts):
+        """The radial solver's factors, solution and eigenvalue counts of one tridiagonal matrix (exposed for
+        testing); counts is a device array of m 32-bit integers."""
+        _check(load().dft_radial_tridiagonal_dev(self.ctx, int(n), _ptr(diag), float(off), float(shift), _ptr(u), _ptr(f),
+                                                 _ptr(w), _ptr(x), int(m), _ptr(E), _ptr(counts)))
 
 
 class PoissonNet:

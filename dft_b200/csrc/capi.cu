@@ -522,6 +522,22 @@ dft_status_t dft_solve_atoms(dft_context* ctx, int nruns, const int* Z, const in
     });
 }
 
+dft_status_t dft_radial_quotients_dev(dft_context* ctx, long m, const double* a, const double* g, double* out) {
+    return guard(ctx, [&] {
+        NEED(ctx && a && g && out && m > 0, "NULL argument or no quotients");
+        dftb::radial_quotients(ctx, m, a, g, out);
+    });
+}
+
+dft_status_t dft_radial_tridiagonal_dev(dft_context* ctx, long n, const double* diag, double off, double shift,
+                                        const double* u, double* f, double* w, double* x, int m, const double* E,
+                                        int* counts) {
+    return guard(ctx, [&] {
+        NEED(ctx && diag && u && f && w && x && E && counts && m > 0, "NULL argument or no counts");
+        dftb::radial_tridiagonal(ctx, n, diag, off, shift, u, f, w, x, m, E, counts);
+    });
+}
+
 }  // extern "C"
 
 // ---------------------------------------------------------------- learned Poisson start --

@@ -192,6 +192,10 @@ void scf_molecule(dft_context* ctx, const dft_grid* grid, int nnuc, const int* Z
 // Radial atoms, one persistent launch (radial.cu).
 void solve_atoms(dft_context* ctx, int nruns, const int* Z, const int* kinds, long points, double rmax,
                  dft_atom_result* results);
+// the radial solver's serial chains by themselves (radial.cu), for tests
+void radial_quotients(dft_context* ctx, long long m, const double* a, const double* g, double* out);
+void radial_tridiagonal(dft_context* ctx, long n, const double* diag, double off, double shift, const double* u,
+                        double* f, double* w, double* x, int m, const double* E, int* counts);
 // The same batch for nz atoms with one functional, keeping the converged atoms on the device:
 // dens (nz x points) the total density n(r), orbs (nz x RADIAL_MAX_SHELLS x points) the radial
 // functions u_nl(r) = r R_nl(r) of the alpha shells, listed per atom as (n, l) in shells.

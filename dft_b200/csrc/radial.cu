@@ -19,7 +19,8 @@
 // The file is compiled without FMA contraction.  Remaining differences from the reference
 // come from the device's transcendental functions (a few ulp) in XC and the start vectors.
 //
-// Bound by the latency of the serial chains.  60 atoms, 2000 points: 412 -> 59 ms, the same bits (steps
+// Bound by the latency of the serial chains.  60 atoms, 2000 points: 412 -> 59 ms, with the bits that general
+// divisions gave (the chains' own quotients differ from those only next to the middle of two numbers; steps
 // from global memory 300 cycles -> shared 73 or less; 13 to 19 rounds of counts -> 3; clusters).
 #include <algorithm>
 #include <array>
@@ -159,11 +160,13 @@ __device__ void seq_prefix(int n, double* st, double* out, Load load, Term term)
     }
 }
 
-// a / g in seven dependent operations (a general division: 126 cycles, here 65).  A third-order
-// Newton step on the approximate reciprocal y0 (error below 2^-18) gives y1, and a quotient q1 within two
-// units in the last place; the remainder's correction is Markstein's (exact_div.cuh).  With the errors of
-// y1 and r the result is the correctly rounded quotient unless that lies within 2^-50 units of a
-// rounding boundary.  a and g in [2^-100, 2^100].
+// a / g in seven dependent operations (a general division: 126 cycles, here 65).  One step y0 (1 + e + e^2),
+// e = 1 - g y0, of Chebyshev's third-order iteration for 1 / g (Traub, Iterative Methods for the Solution of
+// Equations, 1964) on the approximate reciprocal y0 (error below 2^-18) gives y1, and a quotient q1 within two
+// units in the last place; the remainder's correction is Markstein's (exact_div.cuh).  y1 is not the
+// correctly rounded reciprocal, so neither is every quotient: it is wherever a / g is 2^-50 units or more from the
+// middle of two neighbouring numbers, and else one of the two (of 12000 operands made to lie closest, all
+// were right).  a and g in [2^-100, 2^100].
 __device__ __forceinline__ double quotient(double a, double g) {
     double y0;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(g));
@@ -410,10 +413,10 @@ __device__ bool factor(int n, const double* __restrict__ diag, double off, doubl
 // x = the solution of the factored system for u: forwards y_i = u_i - f_i y_{i-1}, backwards
 // x_i = (y_i - off x_{i+1}) / w_i.  The backward chain is four operations: q0 = y_i/w_i - (off/w_i) x_{i+1} from
 // products taken before, the numerator, its remainder and the correction q0 + r / w_i.  q0 is off by
-// 2^k units when the difference loses k bits, and the result is the correctly rounded quotient
-// unless that lies within 2^(k-51) units of a rounding boundary.  As k bits are lost at one point in 2^k, the
-// odds are those of k = 0 times the 24 that are let through.  A stage where more are lost, or where
-// something leaves the range of the theorem, is divided point by point.
+// 2^k units when the difference loses k bits; the result is then the correctly rounded quotient
+// wherever that is 2^(k-51) units or more from the middle of two neighbouring numbers, and else one of the two.
+// k is at most 24 (more are lost at one point in 2^24): a stage where more are lost, or where something
+// leaves the range of the theorem, is divided point by point.
 __device__ void solve(int n, const double* u, const double* f, const double* dw, const double* zh, double off, double* x,
                       double* st) {
     const int lane = threadIdx.x & 31;
@@ -940,6 +943,34 @@ __global__ void __launch_bounds__(RT, 1)
     cluster.sync();  // no block leaves while another may still read its status
 }
 
+// The chains by themselves, for tests.
+__global__ void radial_quotient_kernel(long long m, const double* __restrict__ a, const double* __restrict__ g,
+                                       double* __restrict__ out) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (long long)gridDim.x * blockDim.x)
+        out[i] = quotient(a[i], g[i]);
+}
+// block 0: the factors at `shift` and the solution for u; block 1 + b: counts at 32 values of E
+__global__ void __launch_bounds__(32)
+    radial_tridiagonal_kernel(int n, const double* __restrict__ diag, double off, double shift, const double* u, double* f,
+                              double* w, double* x, double* zh, int m, const double* __restrict__ E,
+                              int* __restrict__ counts, int* __restrict__ ok) {
+    __shared__ __align__(16) double st[WARP_STAGE];
+    const int lane = threadIdx.x;
+    double top = 0.0;
+    for (int i = lane; i < n; i += 32) top = fmax(top, fabs(diag[i]));
+    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (blockIdx.x > 0) {
+        const int e = (blockIdx.x - 1) * 32 + lane;
+        const int c = sturm_count(n, diag, off * off, top, E[min(e, m - 1)], st);
+        if (e < m) counts[e] = c;
+        return;
+    }
+    const bool good = factor(n, diag, off, top, shift, EPS, f, w, zh, st);
+    __syncwarp();
+    if (good) solve(n, u, f, w, zh, off, x, st);
+    if (lane == 0) *ok = good;
+}
+
 // getAtomicConfiguration (ElectronicConfiguration.cpp:16-146) as (n,l,alpha,beta) rows
 void configuration(int Z, std::vector<std::array<int, 4>>& rows) {
     rows.clear();
@@ -1051,6 +1082,29 @@ void solve_atoms(dft_context* ctx, int nruns, const int* Z, const int* kinds, lo
     std::vector<RunSpec> specs;
     long long per_run = 0, orbitals = 0;
     run_batch(ctx, nruns, Z, kinds, points, rmax, results, specs, per_run, orbitals);
+}
+
+void radial_quotients(dft_context* ctx, long long m, const double* a, const double* g, double* out) {
+    radial_quotient_kernel<<<(unsigned)std::min<long long>((m + 255) / 256, 8LL * ctx->num_sms), 256, 0, ctx->stream>>>(
+        m, a, g, out);
+    DFT_LAUNCH_CHECK();
+    count_launch(ctx);
+    sync(ctx);
+}
+
+void radial_tridiagonal(dft_context* ctx, long n, const double* diag, double off, double shift, const double* u,
+                        double* f, double* w, double* x, int m, const double* E, int* counts) {
+    if (n < 2 || n > RADIAL_MAX_POINTS) fail(DFT_INVALID_ARGUMENT, "2 to %ld points", RADIAL_MAX_POINTS);
+    double* zh = (double*)ws_get(ctx, WS_RADIAL, sizeof(double) * (size_t)n);
+    int* ok = (int*)ws_get(ctx, WS_TMP2, sizeof(int));
+    radial_tridiagonal_kernel<<<1 + (m + 31) / 32, 32, 0, ctx->stream>>>((int)n, diag, off, shift, u, f, w, x, zh, m, E,
+                                                                         counts, ok);
+    DFT_LAUNCH_CHECK();
+    count_launch(ctx);
+    int* h = (int*)pinned(ctx, 1);
+    DFT_CUDA(cudaMemcpyAsync(h, ok, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    sync(ctx);
+    if (!*h) fail(DFT_SINGULAR, "a pivot of the shifted radial Hamiltonian is below %g", EPS);
 }
 
 int atomic_orbital_count(int nnuc, const int* Z) {

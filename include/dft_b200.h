@@ -472,9 +472,21 @@ typedef struct {
 /* solveAtom / solveSelfConsistentField (reference AtomicDFT.h:7-11, AtomicDFT.cpp:7-42,
  * SelfConsistentField.cpp:539-786) for nruns independent atoms (Z[r] in 1..30 with the
  * reference's configurations, kinds[r]) on RadialGrid(points, rmax), all advanced by one
- * persistent kernel launch, one thread block per run.  results: host array of nruns. */
+ * persistent kernel launch, one to four thread blocks per run.  results: host array of nruns. */
 dft_status_t dft_solve_atoms(dft_context* ctx, int nruns, const int* Z, const int* kinds, long points, double rmax,
                              dft_atom_result* results);
+
+/* The radial solver's serial chains, exposed for testing (all arrays on the device).
+ * quotients: out[i] = a[i] / g[i] as the chains take it (|a|, |g| in [2^-100, 2^100]): the correctly rounded
+ *   quotient wherever it is 2^-50 units in the last place or more from the middle of two neighbouring
+ *   numbers, else one of the two.
+ * tridiagonal: for the n x n matrix with diagonal diag and off-diagonals off: counts[i] = eigenvalues below
+ *   E[i] (i < m; EigenvalueSolver.cpp:13-92); f, w = the factors of (matrix - shift) and x = its solution
+ *   for u (NumericalMethods.cpp:85-139).  DFT_SINGULAR when a pivot is below 1e-14. */
+dft_status_t dft_radial_quotients_dev(dft_context* ctx, long m, const double* a, const double* g, double* out);
+dft_status_t dft_radial_tridiagonal_dev(dft_context* ctx, long n, const double* diag, double off, double shift,
+                                        const double* u, double* f, double* w, double* x, int m, const double* E,
+                                        int* counts);
 
 /* ---- learned Poisson start (no counterpart in the reference) ------------------------- */
 /* A coarse grid with the same bounds and about a quarter of the points per axis carries the
