@@ -256,16 +256,18 @@ def measure_jacobi(eng, torch, stream, w):
     eng.hartree(g, d_rho, d_vh)  # warm
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     with torch.cuda.stream(stream):
+        launched = eng.launches
         e0.record(stream)
         sweeps, _ = eng.hartree(g, d_rho, d_vh)
         e1.record(stream)
+        launched = eng.launches - launched
     e1.synchronize()
     ms = e0.elapsed_time(e1)
     nx, ny, nz = w["n"]
     interior = (nx - 2) * (ny - 2) * (nz - 2)
     bytes_per_sweep = 24.0 * interior
-    # the launch shape the library picks by default (grid_ops.cu: hartree)
-    if nx * ny * nz <= 64 ** 3:
+    # the launch shape the library picked (grid_ops.cu: hartree): an init launch, then one or one per sweep
+    if launched < sweeps:
         kernel, spl, note = ("jacobi_resident_kernel", sweeps,
                              "whole solve in one launch; V, V', rho live in the shared memory of all SMs, so HBM is "
                              "not the binding resource (exchange latency bound)")

@@ -1338,9 +1338,10 @@ static bool hartree_cluster(dft_context* ctx, const Grid& g, const double* rho, 
     return true;
 }
 
-// The whole solve in one cooperative launch (small grids).
-static JacobiResult hartree_persistent(dft_context* ctx, const Grid& g, const double* rho, double* vh, double* buf1,
-                                       double tol, long max_sweeps) {
+// Jacobi sweeps from `start` in one cooperative launch, the grid in global memory; both buffers hold the
+// faces.  *result: the buffer that holds the final iterate.
+static JacobiResult hartree_persistent(dft_context* ctx, const Grid& g, const double* rho, double* start, double* other,
+                                       double tol, long max_sweeps, double** result) {
     JacobiPCtrl* ctrl = (JacobiPCtrl*)ws_get(ctx, WS_CTRL, sizeof(JacobiPCtrl) + 64);
     DFT_CUDA(cudaMemsetAsync(ctrl, 0, sizeof(JacobiPCtrl), ctx->stream));
     int per_sm = 0;
@@ -1351,8 +1352,8 @@ static JacobiResult hartree_persistent(dft_context* ctx, const Grid& g, const do
     long long cap = max_sweeps;
     Grid gg = g;
     const double* r = rho;
-    double* b0 = vh;
-    double* b1 = buf1;
+    double* b0 = start;
+    double* b1 = other;
     long long polls = ctx->grid_barrier_poll_limit > 0 ? ctx->grid_barrier_poll_limit : (1LL << 24);
     void* args[] = {&gg, &r, &b0, &b1, &ctrl, &den, &tol, &cap, &polls};
     DFT_CUDA(cudaLaunchCooperativeKernel((const void*)jacobi_persistent_kernel, dim3(nblocks), dim3(256), args, 0,
@@ -1362,8 +1363,7 @@ static JacobiResult hartree_persistent(dft_context* ctx, const Grid& g, const do
     DFT_CUDA(cudaMemcpyAsync(hc, ctrl, sizeof(JacobiPCtrl), cudaMemcpyDeviceToHost, ctx->stream));
     sync(ctx);
     if (hc->error) fail(DFT_CUDA_ERROR, "Jacobi grid barrier timed out");
-    if (hc->sweeps & 1)
-        DFT_CUDA(cudaMemcpyAsync(vh, buf1, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));
+    *result = hc->sweeps & 1 ? other : start;
     return {(long)hc->sweeps, hc->last_diff};
 }
 
@@ -1481,8 +1481,11 @@ JacobiResult hartree(dft_context* ctx, const Grid& g, const double* rho, double*
         DFT_CUDA(cudaMemcpyAsync(hc, ctrl, sizeof(JacobiCtrl), cudaMemcpyDeviceToHost, ctx->stream));
         sync(ctx);
     };
-    // launch shape: one launch with the grid resident in shared memory where it fits, one sweep per
-    // launch otherwise; 2/4/8 select the temporally blocked kernel
+    // Launch shape: one launch with the grid resident in shared memory where it fits (cubes up to 86^3), one with
+    // it in global memory for the other grids of up to 64^3 points (three or four planes of 200 x 300 or
+    // more), else one sweep per launch; 2/4/8 select the temporally blocked kernel.  Microseconds per
+    // sweep: resident against one launch each, 64^3 2.75 / 8.3, 72^3 3.16 / 8.3, 80^3 3.96 / 10.4, 86^3
+    // 4.17 / 10.2; one launch in global memory against one each, 250 x 250 x 3 5.7 / 6.3, 256 x 256 x 4 6.2 / 6.8.
     int tmax = ctx->jacobi_sweeps_per_launch;
     if (tmax == 0) {
         auto t = ctx->tuned.find({(long long)g.nx, (long long)g.ny, (long long)g.nz});
@@ -1499,21 +1502,23 @@ JacobiResult hartree(dft_context* ctx, const Grid& g, const double* rho, double*
                 return {1L, hc->last_diff};
             }
         }
-        double *from = launched ? buf1 : vh, *result = nullptr;
-        if (hartree_resident(ctx, g, rho, from, launched ? vh : buf1, tol, max_sweeps - launched, &r, &result)) {
+        double *from = launched ? buf1 : vh, *other = launched ? vh : buf1, *result = nullptr;
+        bool solved = hartree_resident(ctx, g, rho, from, other, tol, max_sweeps - launched, &r, &result);
+        if (!solved && (tmax == -1 || g.N <= 64LL * 64 * 64)) {
+            r = hartree_persistent(ctx, g, rho, from, other, tol, max_sweeps - launched, &result);
+            solved = true;
+        }
+        if (solved) {
             if (result != vh)
                 DFT_CUDA(cudaMemcpyAsync(vh, buf1, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));
             r.sweeps += launched;
             return r;
         }
-        if (launched && tmax == -1) tmax = 1;  // the sweep above stays
     }
     if (tmax == -2) {
         if (hartree_cluster(ctx, g, rho, vh, tol, max_sweeps, &r)) return r;
         fail(DFT_INVALID_ARGUMENT, "grid does not fit the cluster-resident Jacobi");
     }
-    if (tmax == 0) tmax = 1;
-    if (tmax == -1) return hartree_persistent(ctx, g, rho, vh, buf1, tol, max_sweeps);
     if (tmax == 2 || tmax == 4 || tmax == 8) return hartree_tb(ctx, g, rho, vh, buf1, tol, max_sweeps, tmax);
     // Sweeps are launched in batches; a launch after the stop rule fired returns at once, so
     // a batch may overrun the stopping sweep without changing the result.

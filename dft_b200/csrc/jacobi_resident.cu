@@ -1,5 +1,5 @@
-// Jacobi Poisson solve in one cooperative launch with the grid resident in shared memory (grids up to
-// about 64^3), T sweeps per exchange between blocks.
+// Jacobi Poisson solve in one cooperative launch with the grid resident in shared memory (cubes up to
+// 86^3), T sweeps per exchange between blocks.
 //
 // The sweep of a small grid is a fraction of a microsecond of work, so what bounds a solve of
 // thousands of sweeps is the exchange between SMs.  Every block owns a box of interior points and keeps it, a
@@ -21,7 +21,7 @@
 // A half warp sweeps one row (two rows of at most 16 points are two shared-memory wavefronts whatever
 // their pitch); shared-memory reads, 7 per point, are what bounds a sweep.
 //
-// 48^3 to the stop rule: 1.44 us per sweep; 6.46 for the 16-block cluster that exchanged whole planes
+// 48^3 to the stop rule (T = 3): 1.44 us per sweep; 6.46 for the 16-block cluster that exchanged whole planes
 // every sweep, 3.57 for this layout behind a grid barrier, 7.6 to 8.3 for one launch per sweep.
 //
 // Every wait is bounded: a thread that polls poll_limit times, or sees the error word set,

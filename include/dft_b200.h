@@ -65,7 +65,8 @@ dft_status_t dft_context_synchronize(dft_context* ctx);
  *   "jacobi_sweeps_per_launch": 0 = auto (default: as -1 for small grids), -2 = the whole solve in
  *                               the shared memory of one 16-block cluster (small grids), -1 =
  *                               the whole solve in one cooperative launch (in the shared memory
- *                               of all SMs where the grid fits), 1 = one sweep per launch,
+ *                               of all SMs where the grid fits; a warm start takes its first
+ *                               sweep by itself), 1 = one sweep per launch,
  *                               2, 4 or 8 = temporally blocked sweeps per launch (results are
  *                               identical for every value).
  *   "network_tensor_cores":     1 (default) = the Poisson-start network's 16- and 32-channel

@@ -1,0 +1,69 @@
+"""GPU: the Jacobi solve's launch shapes at the edges of the rule that picks them: the largest boxes that fit the
+shared memory of all SMs, and the boxes beyond it, where one cooperative launch keeps the grid in global memory
+(flat grids of up to 64^3 points, or key -1).  Same bits, sweep count and last difference as one sweep per
+launch, from cold and warm starts."""
+import numpy as np
+import pytest
+
+import dft_b200
+
+pytestmark = pytest.mark.gpu
+
+
+def _grid(dims):
+    b = []
+    for n in dims:
+        half = 0.5 * 0.25 * (n - 1)
+        b += [-half, half]
+    return dft_b200.CartesianGrid(*dims, *b)
+
+
+def _solve(engine, mode, g, rho, tol, cap, guess=None):
+    vh = engine.upload(guess) if guess is not None else engine.array(g.getSize())
+    engine.set_tuning("jacobi_sweeps_per_launch", mode)
+    before = engine.launches
+    try:
+        f = engine.hartree_from_guess if guess is not None else engine.hartree
+        s, d = f(g, engine.upload(rho), vh, tol, cap)
+    finally:
+        engine.set_tuning("jacobi_sweeps_per_launch", 0)
+    return s, d, vh.to_host().tobytes(), engine.launches - before
+
+
+# (box, key, whether the solve is one launch)
+SHAPES = [((80, 80, 80), 0, True), ((86, 86, 86), 0, True), ((88, 88, 88), 0, False), ((250, 250, 3), 0, True),
+          ((256, 256, 4), 0, True), ((20, 4000, 3), 0, True), ((257, 256, 4), 0, False), ((88, 88, 88), -1, True),
+          ((96, 90, 80), -1, True), ((257, 256, 4), -1, True)]
+
+
+@pytest.mark.parametrize("dims,mode,one", SHAPES)
+# the caps stop before, at and after a round of two to four sweeps; the last stops by the rule
+@pytest.mark.parametrize("cap", [1, 2, 7, 40, 10000])
+def test_same_bits(engine, dims, mode, one, cap):
+    g = _grid(dims)
+    rng = np.random.default_rng(cap)
+    rho = rng.uniform(0.0, 1.0, g.getSize()) ** 8
+    tol = 3e-3 if cap == 10000 else 0.0
+    warm = rng.standard_normal(g.getSize())
+    for guess in (None, warm):
+        ref = _solve(engine, 1, g, rho, tol, cap, guess)
+        got = _solve(engine, mode, g, rho, tol, cap, guess)
+        assert got[:3] == ref[:3]
+        if cap == 40:  # init and the solve; a warm start takes its first sweep by itself
+            assert got[3] == (2 if guess is None else 3) if one else got[3] >= 40
+
+
+def test_global_memory_launch_gives_up(engine):
+    """A grid beyond the shared memory with a barrier poll limit of 1: an error with a message, and the context solves
+    normally afterwards."""
+    g = _grid((256, 256, 4))
+    rho = np.random.default_rng(1).uniform(0.0, 1.0, g.getSize())
+    d_rho, d_vh = engine.upload(rho), engine.array(g.getSize())
+    engine.set_tuning("grid_barrier_poll_limit", 1)
+    try:
+        with pytest.raises(dft_b200.DFTError) as ei:
+            engine.hartree(g, d_rho, d_vh, 1e-8, 10000)
+        assert ei.value.status == dft_b200.DFT_CUDA_ERROR and "grid barrier timed out" in str(ei.value)
+    finally:
+        engine.set_tuning("grid_barrier_poll_limit", 0)
+    assert _solve(engine, 0, g, rho, 0.0, 30)[:3] == _solve(engine, 1, g, rho, 0.0, 30)[:3]
