@@ -1445,7 +1445,7 @@ void pnet_train_poisson(dft_context* ctx, dft_pnet* n, const dft_pnet_train_opts
         synthetic_density(ctx, g, o->seed * 0x9E3779B97F4A7C15ULL + (unsigned long long)s, o->kmin, o->kmax, o->wmin,
                           o->wmax, o->ne_min, o->ne_max, r);
         double* sdev = nullptr;
-        coarse_start(ctx, slab.get(coarse_slab_doubles(g)), g, r, u, &sdev);
+        coarse_start(ctx, slab.get(coarse_slab_doubles(ctx, g)), g, r, u, &sdev);
         // target: the Jacobi fixed point to target_tol, reached by multigrid cycles from the
         // coarse start and finished by Jacobi sweeps under the stop rule
         DFT_CUDA(cudaMemcpyAsync(v, u, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));

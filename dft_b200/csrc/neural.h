@@ -30,8 +30,8 @@ int coarse_points(int n);
 
 // Nested coarse-grid start (poisson_start.cu): vup = the interpolated solution of the coarse
 // levels; *scale_dev = max |first coarse level's solution| on the device.  slab holds
-// coarse_slab_doubles(g) doubles.  Returns the multigrid cycles spent on the coarse levels.
-size_t coarse_slab_doubles(const Grid& g);
+// coarse_slab_doubles(ctx, g) doubles.  Returns the multigrid cycles spent on the coarse levels.
+size_t coarse_slab_doubles(dft_context* ctx, const Grid& g);
 long coarse_start(dft_context* ctx, double* slab, const Grid& g, const double* rho, double* vup, double** scale_dev);
 
 // Multigrid V(2,2) cycles on v in place (faces held at their values, coarse corrections zero

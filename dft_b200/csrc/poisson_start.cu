@@ -134,11 +134,13 @@ std::vector<Level> plan_levels(const Grid& fine) {
     return L;
 }
 
-size_t slab_doubles(const Grid& fine, const std::vector<Level>& L) {
+// separate: with the temporaries of the separate restriction passes
+size_t slab_doubles(const Grid& fine, const std::vector<Level>& L, bool separate) {
     size_t n = 8;  // the scale s
     Grid prev = fine;
     for (const Level& l : L) {
-        n += (size_t)prev.nz * prev.ny * l.g.nx + (size_t)prev.nz * l.g.ny * l.g.nx + 2 * (size_t)l.g.N + 8;
+        if (separate) n += (size_t)prev.nz * prev.ny * l.g.nx + (size_t)prev.nz * l.g.ny * l.g.nx + 4;
+        n += 2 * (size_t)l.g.N + 4;
         // the transfer table between prev and l
         n += 6 * (size_t)(l.g.nx + l.g.ny + l.g.nz) + 2 * (size_t)(prev.nx + prev.ny + prev.nz) + 4;
         prev = l.g;
@@ -147,7 +149,7 @@ size_t slab_doubles(const Grid& fine, const std::vector<Level>& L) {
 }
 
 // Carves the level arrays and the place of the transfer tables; returns the scale slot.
-double* carve(double* slab, const Grid& fine, std::vector<Level>& L, double** tables) {
+double* carve(double* slab, const Grid& fine, std::vector<Level>& L, bool separate, double** tables) {
     double* s = slab;
     double* p = slab + 8;
     Grid prev = fine;
@@ -157,8 +159,10 @@ double* carve(double* slab, const Grid& fine, std::vector<Level>& L, double** ta
         return q;
     };
     for (Level& l : L) {
-        l.t1 = take((size_t)prev.nz * prev.ny * l.g.nx);
-        l.t2 = take((size_t)prev.nz * l.g.ny * l.g.nx);
+        if (separate) {
+            l.t1 = take((size_t)prev.nz * prev.ny * l.g.nx);
+            l.t2 = take((size_t)prev.nz * l.g.ny * l.g.nx);
+        }
         l.rc = take((size_t)l.g.N);
         l.vc = take((size_t)l.g.N);
         prev = l.g;
@@ -180,12 +184,12 @@ void restrict3(dft_context* ctx, const Grid& f, const Grid& c, const double* in,
 }
 
 // vup = the nested coarse solution interpolated to g; *s (device) = max |level-0 solution|.
-// Returns the Jacobi sweeps of all coarse levels.
+// Returns the multigrid cycles of all coarse levels.
 long coarse_solve(dft_context* ctx, double* slab, const Grid& g, const double* rho, double* vup, double** s_out,
                   Grid* gc_out) {
     std::vector<Level> L = plan_levels(g);
     double* tables;
-    double* s = carve(slab, g, L, &tables);
+    double* s = carve(slab, g, L, !ctx->mg_fused_restrict, &tables);
     const bool zero = faces_exact(g);  // the coarse boundary follows the fine grid's
     const double* src = rho;
     Grid sg = g;
@@ -226,11 +230,6 @@ long coarse_solve(dft_context* ctx, double* slab, const Grid& g, const double* r
     if (s_out) *s_out = s;
     if (gc_out) *gc_out = L[0].g;
     return cycles;
-}
-
-double* coarse_slab(dft_context* ctx, const Grid& g) {
-    const std::vector<Level> L = plan_levels(g);
-    return (double*)ws_get(ctx, WS_PG0, sizeof(double) * slab_doubles(g, L));
 }
 
 // ---------------------------------------------------------------- multigrid ------------
@@ -306,22 +305,23 @@ struct Restriction {
     double *t1, *t2;  // temporaries of the separate restriction passes
 };
 
-size_t mg_doubles(const std::vector<MGLevel>& L) {
-    size_t n = 16 + sizeof(MGHistory) / sizeof(double) + mg_table_doubles(L) + 2 + 6 * ((size_t)L[0].g.N + 2);
+// Four fields of the finest grid, three of each coarser one; separate: with the passes' temporaries.
+size_t mg_doubles(const std::vector<MGLevel>& L, bool separate) {
+    size_t n = sizeof(MGHistory) / sizeof(double) + mg_table_doubles(L) + 64 + 4 * ((size_t)L[0].g.N + 32);
     for (size_t i = 0; i < L.size(); ++i) {
         const Grid& g = L[i].g;
-        if (i > 0) n += 4 * ((size_t)g.N + 2);
-        if (i + 1 < L.size()) {
+        if (i > 0) n += 3 * ((size_t)g.N + 32);
+        if (separate && i + 1 < L.size()) {
             const Grid& c = L[i + 1].g;
-            n += (size_t)g.nz * g.ny * c.nx + (size_t)g.nz * c.ny * c.nx + 4;
+            n += (size_t)g.nz * g.ny * c.nx + (size_t)g.nz * c.ny * c.nx + 64;
         }
     }
     return n;
 }
 
-// One cycle by separate passes below and at level i: v -> v (tmp, res scratch)
-void separate_cycle(dft_context* ctx, std::vector<MGLevel>& L, std::vector<Restriction>& T, std::vector<double*>& res,
-                    size_t i, double sscale, double* v, double* tmp) {
+// One cycle by separate passes below and at level i: v -> v (tmp scratch)
+void separate_cycle(dft_context* ctx, std::vector<MGLevel>& L, std::vector<Restriction>& T, size_t i, double sscale,
+                    double* v, double* tmp) {
     MGLevel& l = L[i];
     auto smooth = [&](const double* from, double* to) {
         mg_smooth_kernel<<<mg_blocks(ctx, l.g.N), 256, 0, ctx->stream>>>(l.g, l.src, sscale, from, to, 0.8);
@@ -329,15 +329,15 @@ void separate_cycle(dft_context* ctx, std::vector<MGLevel>& L, std::vector<Restr
     };
     smooth(v, tmp);
     smooth(tmp, v);
-    mg_residual_kernel<<<mg_blocks(ctx, l.g.N), 256, 0, ctx->stream>>>(l.g, l.src, sscale, v, res[i]);
+    mg_residual_kernel<<<mg_blocks(ctx, l.g.N), 256, 0, ctx->stream>>>(l.g, l.src, sscale, v, tmp);
     count_launch(ctx);
     MGLevel& c = L[i + 1];
-    restrict3(ctx, l.g, c.g, res[i], T[i].t1, T[i].t2, c.src);
+    restrict3(ctx, l.g, c.g, tmp, T[i].t1, T[i].t2, c.src);
     if (i + 2 == L.size()) {
         mg_coarsest_solve(ctx, c, c.src, ctx->mg_coarsest_sor != 0);
     } else {
         DFT_CUDA(cudaMemsetAsync(c.v, 0, sizeof(double) * (size_t)c.g.N, ctx->stream));
-        separate_cycle(ctx, L, T, res, i + 1, 1.0, c.v, c.tmp);
+        separate_cycle(ctx, L, T, i + 1, 1.0, c.v, c.tmp);
     }
     prolong_add_kernel<<<mg_blocks(ctx, l.g.N), 256, 0, ctx->stream>>>(l.g, c.g, c.v, v);
     count_launch(ctx);
@@ -348,7 +348,9 @@ void separate_cycle(dft_context* ctx, std::vector<MGLevel>& L, std::vector<Restr
 
 }  // namespace
 
-size_t coarse_slab_doubles(const Grid& g) { return slab_doubles(g, plan_levels(g)); }
+size_t coarse_slab_doubles(dft_context* ctx, const Grid& g) {
+    return slab_doubles(g, plan_levels(g), !ctx->mg_fused_restrict);
+}
 
 long coarse_start(dft_context* ctx, double* slab, const Grid& g, const double* rho, double* vup, double** scale_dev) {
     return coarse_solve(ctx, slab, g, rho, vup, scale_dev, nullptr);
@@ -358,23 +360,24 @@ int multigrid(dft_context* ctx, const Grid& g, const double* rho, double* v, dou
               double* resid_out) {
     std::vector<MGLevel> L = mg_levels(g);
     if (L.back().g.N > MG_COARSEST_MAX) fail(DFT_INVALID_ARGUMENT, "grid too small or too anisotropic for multigrid");
-    double* slab = (double*)ws_get(ctx, WS_PG1, sizeof(double) * mg_doubles(L));
-    double* next = slab + 16;
+    const bool separate = !ctx->mg_fused_restrict && L.size() > 1;
+    double* slab = (double*)ws_get(ctx, WS_PG1, sizeof(double) * mg_doubles(L, separate));
+    double* next = slab;
     auto take = [&](size_t n) {
         double* q = next;
-        next += (n + 1) / 2 * 2;  // keep 16-byte alignment
+        next += (n + 31) / 32 * 32;  // 256-byte alignment
         return q;
     };
     MGHistory* hist = (MGHistory*)take(sizeof(MGHistory) / sizeof(double));
     mg_tables(ctx, L, take(mg_table_doubles(L)));
     // The solve runs on its own copies: the captured cycles below then depend on the grid alone.
-    // Cycles alternate between buf[0] and buf[1], so the last two iterates are at hand.
+    // Cycles alternate between buf[0] and buf[1], so the last two iterates are at hand; v itself, once copied,
+    // holds the iterate that a batch of cycles starts from.
     const size_t N = (size_t)g.N, bytes = sizeof(double) * N;
     double* rhs = take(N);
     double* buf[2] = {take(N), take(N)};
-    double *tmp = take(N), *tmp2 = take(N), *saved = take(N);
+    double *tmp = take(N), *saved = v;
     std::vector<Restriction> T(L.size());
-    std::vector<double*> res(L.size(), tmp2);
     L[0].src = rhs;
     L[0].tmp = tmp;
     for (size_t i = 0; i < L.size(); ++i) {
@@ -382,9 +385,8 @@ int multigrid(dft_context* ctx, const Grid& g, const double* rho, double* v, dou
             L[i].src = take((size_t)L[i].g.N);
             L[i].v = take((size_t)L[i].g.N);
             L[i].tmp = take((size_t)L[i].g.N);
-            res[i] = take((size_t)L[i].g.N);
         }
-        if (i + 1 < L.size()) {
+        if (separate && i + 1 < L.size()) {
             T[i].t1 = take((size_t)L[i].g.nz * L[i].g.ny * L[i + 1].g.nx);
             T[i].t2 = take((size_t)L[i].g.nz * L[i + 1].g.ny * L[i + 1].g.nx);
         }
@@ -397,13 +399,13 @@ int multigrid(dft_context* ctx, const Grid& g, const double* rho, double* v, dou
     const bool sor = ctx->mg_coarsest_sor != 0;
     // one cycle in -> out (in is kept), then the residual's max norm into the history
     auto cycle = [&](const double* in, double* out) {
-        if (ctx->mg_fused_restrict || L.size() == 1) {
+        if (!separate) {
             L[0].v = out;
             mg_cycle(ctx, L, 0, rhs, nullptr, in, 0, fourpi, nullptr, 1, sor, hist);
         } else {
             mg_start_cycle(ctx, hist);
             DFT_CUDA(cudaMemcpyAsync(out, in, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-            separate_cycle(ctx, L, T, res, 0, fourpi, out, tmp);
+            separate_cycle(ctx, L, T, 0, fourpi, out, tmp);
             mg_residual_max(ctx, g, rhs, fourpi, out, hist);
         }
     };
@@ -517,7 +519,7 @@ int multigrid(dft_context* ctx, const Grid& g, const double* rho, double* v, dou
 
 void poisson_start(dft_context* ctx, dft_pnet* net, const Grid& g, const double* rho, double* out, int cycles,
                    PoissonGuessInfo* info) {
-    double* slab = (double*)ws_get(ctx, WS_PG0, sizeof(double) * coarse_slab_doubles(g));
+    double* slab = (double*)ws_get(ctx, WS_PG0, sizeof(double) * coarse_slab_doubles(ctx, g));
     double* sdev = nullptr;
     const long sw = coarse_start(ctx, slab, g, rho, out, &sdev);
     if (net) pnet_correct(ctx, net, g, rho, out, sdev);
