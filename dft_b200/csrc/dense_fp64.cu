@@ -214,9 +214,10 @@ __global__ void __launch_bounds__(256) gram_sum_kernel(int nch, int nel, const d
 // ---------------------------------------------------------------- ordered Gram ---------
 // Blocks of up to 64 x 16 (the eigensolver of a small molecule) keep a fixed order of summation, so that
 // nothing downstream that turns on the last bit (the sign of an eigenvector of the projected
-// matrix) depends on how the work is split.  An MMA adds its four products one after the
-// other like four FMAs, so a chain of MMAs along the points is the scalar chain, bit for bit; each
-// element is a set of such chains, added in a fixed tree.
+// matrix) depends on how the work is split.  On this chip an MMA adds its four products one after the
+// other like four FMAs (nothing promises it; the tests hold these products to the chains bit for
+// bit), so a chain of MMAs along the points is the scalar chain; each element is a set of such chains,
+// added in a fixed tree.
 //
 // gram_lanes_kernel (kb <= 4, 8 or 16 with ka <= 64, 64, 32): the points are dealt to nblk blocks of 32
 // chains; chain (b, l) takes the points 32 b + l + 32 m nblk.  The 32 chains of block b are added as a
