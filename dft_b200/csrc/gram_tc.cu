@@ -40,8 +40,8 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
     return x == x ? r : 0x7fffffffu;
 }
 
-// x ~ hi + lo, both TF32: hi = TF32(FP32(x)), lo = TF32(FP32(x - hi)).  Conversions from and to FP64 are the
-// slowest operations here, so hi is widened by integer operations (138 x 69, 112 x 97 x 101: 721 -> 703 us).  Rounding
+// x ~ hi + lo, both TF32: hi = TF32(FP32(x)), lo = TF32(FP32(x - hi)).  Conversions from and to FP64 are
+// slow, so hi is widened by integer operations (138 x 69, 112 x 97 x 101: 721 -> 703 us).  Rounding
 // x and x - hi by integer operations as well took 983.
 __device__ __forceinline__ void split_tf32(double x, uint32_t& hi, uint32_t& lo) {
     hi = to_tf32((float)x);
@@ -54,10 +54,8 @@ __device__ __forceinline__ void split_tf32(double x, uint32_t& hi, uint32_t& lo)
     lo = to_tf32((float)(x - w));
 }
 
-// Canonical K-major, no-swizzle placement of element (row, k) of an R-row slice (ring, TMA and rotation
-// kernels): core matrix (8 rows x 4 fp32) index = (k/4) * (R/8) + row/8, 128 bytes each.
-
-// UMMA shared-memory matrix descriptor (sm_100: version 1, no swizzle)
+// UMMA shared-memory matrix descriptor (sm_100: version 1) of the ring, TMA and rotation kernels' slices: K-major
+// without swizzle, element (row, k) of R rows in core matrix (k/4) * (R/8) + row/8 of 8 rows x 4 fp32, 128 bytes each
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
     uint64_t d = 0;
     d |= (uint64_t)((addr >> 4) & 0x3FFF);
@@ -120,17 +118,21 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 // split; the rest of the tile is zeroed once.  The products of a step go hi*hi, A hi * B lo, A lo * B hi on
 // either side, so an element's sum does not depend on the tiling.
 //
-// Bound by memory (each operand once where one tile holds the product) and the conversions.  138 x 69,
-// 112 x 97 x 101: 1500 -> 703 us.  A tile of 128 rows of A per block read B a second time for the ten
-// rows left over, split 512 rows of which 207 exist, and loaded and converted by turns.
+// Bound by the instructions of the split (ALU pipe 65 % busy, issue slots 54 %, conversions 26 %, DRAM at 2.7 TB/s:
+// 138 x 69, 112 x 97 x 101, where this took 1500 -> 703 us).  A tile of 128 rows of A per block read B a second
+// time for the ten rows left over, split 512 rows of which 207 exist, and loaded and converted by turns.
 //
-// Two groups of eight warps take the slices in turn, each into its own stage, and a warp of its own issues the
-// products: one group's loads and barriers run under the other's conversions.  With all sixteen warps on every
-// slice, block barriers around it and core matrices without swizzle, 786 us.
-constexpr int TG_WARPS = 8;                          // per group
-constexpr int TG_THREADS = (2 * TG_WARPS + 1) * 32;  // and the issuing warp
+// W = 8: two groups of eight warps take the slices in turn, each into its own stage, and a warp of its own issues the
+// products: one group's loads and barriers run under the other's conversions.  W = 16: all sixteen warps take
+// every slice, so a warp has half the rows.  Up to 144 rows the groups are faster (96^3, groups / all: 40 x 40 259
+// / 321 us, 69 x 69 418 / 447), from there on their rows no longer fit the 96 registers with all loads in
+// flight (138 x 69 565 / 563, 128 x 128 753 / 655, 207 x 69 757 / 691, 256 x 256 2471 / 1715; 48^3, 256 x 256 499 / 404).
+constexpr int TG_ALL = 16;                     // loading warps
+constexpr int TG_THREADS = (TG_ALL + 1) * 32;  // and the issuing warp
 
-template <int PW>  // rows per warp, both sides
+// PW: most slots (rows of either side) of a warp; of these, slots from LOW on are checked four at a time, so that a
+// tile of fewer rows does not split what is not there (checks in the groups' kernels cost more than they save).
+template <int PW, int LOW, int W>
 __global__ void __launch_bounds__(TG_THREADS, 1)
     gram_tc_kernel(const double* __restrict__ M, long long ldm, int km, const double* __restrict__ Nn, long long ldn,
                    int kn, int nt, int ncols, int swapped, long long n, long long chunk, double* __restrict__ partial,
@@ -140,7 +142,8 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
     __shared__ uint32_t s_tmem;
     __shared__ __align__(8) uint64_t full[2], bar[2];  // a stage is written; its products are done
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    const int group = wid / TG_WARPS, warp = wid % TG_WARPS;  // group 2: the issuing warp
+    constexpr int GROUPS = TG_ALL / W;
+    const int group = wid / W, warp = wid % W;  // group GROUPS: the issuing warp
     const int m0 = blockIdx.x * TC_M, n0 = blockIdx.y * nt;
     const int mrows = min(TC_M, km - m0), nrows = min(nt, kn - n0);
     const int rn = (nt + 15) / 16 * 16;  // columns of the MMA
@@ -153,7 +156,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
     }
     if (tid == 0) {
         for (int st = 0; st < 2; ++st) {
-            mbar_init(&full[st], TG_WARPS * 32);
+            mbar_init(&full[st], W * 32);
             mbar_init(&bar[st], 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -165,48 +168,49 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
     const uint32_t idesc = idesc_tf32(rn);
-    // Slot i of a warp is M row warp + 8 i below `first`, then N row warp + 8 (i - first): every slot of a side is a
-    // fixed step from the last, in global and in shared memory (one atom).
-    const int first = (mrows + TG_WARPS - 1) / TG_WARPS;
-    const long long step_m = TG_WARPS * ldm, step_n = TG_WARPS * ldn;
+    // Slot i of a warp is M row warp + W i below `first`, then N row warp + W (i - first): every slot of a side is a
+    // fixed step from the last, in global and in shared memory (one or two atoms).
+    const int first = (mrows + W - 1) / W, slots = first + (nrows + W - 1) / W;
+    const long long step_m = W * ldm, step_n = W * ldn;
     const double* const at_m = M + (long long)(m0 + warp) * ldm + lane;
     const double* const at_n = Nn + (long long)(n0 + warp) * ldn + lane;
-    const int end_m = mrows - warp, end_n = nrows - warp + TG_WARPS * first;  // slot i exists below these: 8 i
-    const int to_m = warp * TC_KT + (((lane >> 2) ^ warp) << 2) + (lane & 3);
-    const int to_n = 2 * m_words + to_m - TG_WARPS * TC_KT * first;
+    const int end_m = mrows - warp, end_n = nrows - warp + W * first;  // slot i exists below these: W i
+    const int to_m = warp * TC_KT + (((lane >> 2) ^ (warp & 7)) << 2) + (lane & 3);
+    const int to_n = 2 * m_words + to_m - W * TC_KT * first;
+    auto past = [&](int i) { return i >= LOW && i % 4 == 0 && i >= slots; };
     auto load = [&](double (&x)[PW], long long ps) {
         const bool in = ps + lane < p1;
         const double* q = at_m + ps;  // stepped: products with the slot's number would be kept, two registers each
         long long step = step_m;
 #pragma unroll
         for (int i = 0; i < PW; ++i) {
+            if (past(i)) break;
             if (i == first) q = at_n + ps, step = step_n;
-            x[i] = in && TG_WARPS * i < (i < first ? end_m : end_n) ? __ldg(q) : 0.0;
+            x[i] = in && W * i < (i < first ? end_m : end_n) ? __ldg(q) : 0.0;
             q += step;
         }
     };
     bool ok = true;
     const int steps = p0 < p1 ? (int)((p1 - p0 + TC_KT - 1) / TC_KT) : 0;
-    if (group < 2) {
-        const int st = group;
+    if (group < GROUPS) {
         double x[PW];
-        if (st < steps) load(x, p0 + st * TC_KT);
-        uint32_t* const stage = sm + st * stage_words;
-        uint32_t phase = 0;
-        for (int step = st; step < steps; step += 2) {
+        if (group < steps) load(x, p0 + group * TC_KT);
+        for (int step = group; step < steps; step += GROUPS) {
+            const int st = GROUPS == 2 ? group : step & 1;
+            uint32_t* const stage = sm + st * stage_words;
             // the products that last read this stage must be done before it is overwritten
             if (step >= 2) {
-                ok = mbar_wait(&bar[st], phase);
+                ok = mbar_wait(&bar[st], (step / 2 - 1) & 1);
                 if (!ok) break;
-                phase ^= 1;
             }
 #pragma unroll
             for (int i = 0; i < PW; ++i) {
+                if (past(i)) break;
                 const bool side = i < first;
                 uint32_t h, l;
                 split_tf32(x[i], h, l);
-                uint32_t* o = stage + (side ? to_m : to_n) + TG_WARPS * TC_KT * i;
-                if (TG_WARPS * i < (side ? end_m : end_n)) {
+                uint32_t* o = stage + (side ? to_m : to_n) + W * TC_KT * i;
+                if (W * i < (side ? end_m : end_n)) {
                     o[0] = h;
                     o[side ? m_words : n_words] = l;
                 }
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
             // generic-proxy smem writes -> visible to the tensor core (async proxy)
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[st])) : "memory");
-            if (step + 2 < steps) load(x, p0 + (long long)(step + 2) * TC_KT);
+            if (step + GROUPS < steps) load(x, p0 + (long long)(step + GROUPS) * TC_KT);
         }
     } else if (lane == 0) {
         int issued[2] = {0, 0};
@@ -253,9 +257,9 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
     };
     if (!ok) {
         if (tid == 0) atomicExch(error, 1);
-    } else if (p0 < p1 && group < 2) {
+    } else if (p0 < p1 && wid < TG_ALL) {
         const int q4 = wid & 3, row = q4 * 32 + lane;
-        for (int c0 = (wid >> 2) * 8; c0 < nrows; c0 += 2 * TG_WARPS / 4 * 8) {
+        for (int c0 = (wid >> 2) * 8; c0 < nrows; c0 += TG_ALL / 4 * 8) {
             uint32_t v[8];
             const uint32_t addr = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)c0;
             asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -287,18 +291,20 @@ void gram_tiles(dft_context* ctx, const double* A, long long lda, int ka, const 
     int ncols = 32;
     while (ncols < nt) ncols <<= 1;
     const size_t smem = sizeof(uint32_t) * 2 * 2 * TC_KT * ((size_t)TC_M + up(nt, 16) * 16) + 1024;
-    const int per = up(std::min(km, TC_M), TG_WARPS) + up(nt, TG_WARPS);  // at most 16 + 32
+    // slots of a warp, of eight and of sixteen; the instances' steps cost up to a third of the time just above a
+    // step (96^3: 40 x 40 259 us, 44 x 44 346, 69 x 69 418)
+    const int s8 = up(std::min(km, TC_M), 8) + up(nt, 8), s16 = up(std::min(km, TC_M), 16) + up(nt, 16);
     const auto launch = [&](auto kernel) {
         DFT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         kernel<<<dim3(mt, nts, (unsigned)nch), TG_THREADS, smem, ctx->stream>>>(
             swapped ? B : A, swapped ? ldb : lda, km, swapped ? A : B, swapped ? lda : ldb, kn, nt, ncols, swapped, n,
             chunk, partial, kb, err);
     };
-    if (per <= 10) launch(gram_tc_kernel<10>);
-    else if (per <= 18) launch(gram_tc_kernel<18>);
-    else if (per <= 27) launch(gram_tc_kernel<27>);
-    else if (per <= 36) launch(gram_tc_kernel<36>);
-    else launch(gram_tc_kernel<48>);
+    if (s8 <= 10) launch(gram_tc_kernel<10, 10, 8>);
+    else if (s8 <= 18) launch(gram_tc_kernel<18, 18, 8>);
+    else if (s16 <= 14) launch(gram_tc_kernel<14, 12, 16>);
+    else if (s16 <= 19) launch(gram_tc_kernel<19, 16, 16>);
+    else launch(gram_tc_kernel<24, 12, 16>);
 }
 
 // Ring variant of the Gram tile (tuning key "tensor_core_ring"): the FP64 slices are staged
