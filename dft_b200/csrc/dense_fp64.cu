@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(256) gram_sum_kernel(int nch, int nel, const d
 // gram_lanes_kernel (kb <= 4, 8 or 16 with ka <= 64, 64, 32): the points are dealt to nblk blocks of 32
 // chains; chain (b, l) takes the points 32 b + l + 32 m nblk.  The 32 chains of block b are added as a
 // butterfly (xor 16, 8, 4, 2, 1), then the blocks in order, GM_GROUP at a time.  A thread block works
-// through its blocks b in turn; four m of 32 points and all rows are staged ahead in shared memory by
+// through its blocks b in turn; 4 U m of 32 points and all rows are staged ahead in shared memory by
 // cp.async (reading fragments straight from global memory costs 32 L1 lookups per load, one per
 // row and m: 50 us for 24 x 12 at 64^3).  A warp runs two chains for all RB x CB tiles.  The 272-byte pitch of
 // a staged 256-byte segment makes the 16-byte fragment reads free of bank conflicts.
@@ -237,7 +237,12 @@ __device__ __forceinline__ void stage(void* dst, const void* src, bool wide, int
 
 template <int RB, int CB>
 struct LanesShape {
-    static constexpr int ROWS = 8 * (RB + CB), STAGE = ROWS * 4 * GL_PITCH, SUM = 16 * RB * CB * 64 * 8;
+    static constexpr int ROWS = 8 * (RB + CB), SUM = 16 * RB * CB * 64 * 8;
+    // groups of four m per stage: few rows make short stages, whose barriers then take the time (128^3, one group / as
+    // here: 2 x 2 82 / 52 us, 8 x 8 95 / 72)
+    static constexpr int U = ROWS <= 16 ? 4 : ROWS <= 24 ? 2 : 1;
+    static constexpr int PITCH = 4 * U * GL_PITCH + (U > 1 ? 64 : 0);  // of a row: 16 banks apart
+    static constexpr int STAGE = ROWS * PITCH;
     static constexpr int S = (220 * 1024 - SUM) / STAGE >= 4 ? 4 : (220 * 1024 - SUM) / STAGE;  // stages in flight
     static constexpr size_t SMEM = (size_t)S * STAGE + SUM;
 };
@@ -247,12 +252,12 @@ __global__ void __launch_bounds__(512, 1)
     gram_lanes_kernel(const double* __restrict__ A, long long lda, int ka, const double* __restrict__ B, long long ldb,
                       int kb, long long n, int nblk, double* __restrict__ partial) {
     using Shape = LanesShape<RB, CB>;
-    extern __shared__ __align__(16) char stages[];  // S x (8 (RB + CB) rows) x 4 m; then the butterfly's sums
-    constexpr int TILES = RB * CB, ROWS = Shape::ROWS, STAGE = Shape::STAGE, S = Shape::S;
+    extern __shared__ __align__(16) char stages[];  // S x (8 (RB + CB) rows) x 4 U m; then the butterfly's sums
+    constexpr int TILES = RB * CB, STAGE = Shape::STAGE, S = Shape::S, U = Shape::U, M = 4 * U;
     double* sum = reinterpret_cast<double*>(stages + S * STAGE);  // 8 warps x 2 chains x TILES x 64
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const long long stride = (long long)nblk * 32;
-    const int steps = (int)((n + 4 * stride - 1) / (4 * stride));  // per block b (the last ones may be empty)
+    const int steps = (int)((n + M * stride - 1) / (M * stride));  // per block b (the last ones may be empty)
     const int nb = ((int)blockIdx.x < nblk) ? (nblk - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     const int total = nb * steps;
     // stage q of this thread block: step q % steps of its block number q / steps
@@ -261,15 +266,16 @@ __global__ void __launch_bounds__(512, 1)
             const int b = (int)blockIdx.x + q / steps * (int)gridDim.x, s = q % steps;
             char* to = stages + q % S * STAGE;
             constexpr int PER = AL ? 16 : 32;  // copies per segment
-            for (int e = threadIdx.x; e < ROWS * 4 * PER; e += 512) {
-                const int c = e % PER, m = e / PER & 3, row = e / (4 * PER);
-                const bool of_a = row < 8 * RB;
-                const int r = of_a ? row : row - 8 * RB;
-                const bool real = r < (of_a ? ka : kb);
-                const double* base = of_a ? A + (long long)(real ? r : 0) * lda : B + (long long)(real ? r : 0) * ldb;
-                const long long p = (long long)b * 32 + (4 * s + m) * stride + c * (AL ? 2 : 1);
-                const int in = !real || p >= n ? 0 : AL ? (p + 1 < n ? 16 : 8) : 8;
-                stage(to + (row * 4 + m) * GL_PITCH + c * (AL ? 16 : 8), in ? base + p : base, AL, in);
+            // (rows that do not exist are not staged: what their shared memory holds reaches only elements that
+            // are not stored; 20 x 4 at 128^3 with zeros in their place 183 us, 131 here)
+            for (int e = threadIdx.x; e < (ka + kb) * M * PER; e += 512) {
+                const int c = e % PER, m = e / PER % M, r = e / (M * PER);
+                const bool of_a = r < ka;
+                const double* base = of_a ? A + (long long)r * lda : B + (long long)(r - ka) * ldb;
+                const int row = of_a ? r : 8 * RB + r - ka;
+                const long long p = (long long)b * 32 + (long long)(M * s + m) * stride + c * (AL ? 2 : 1);
+                const int in = p >= n ? 0 : AL ? (p + 1 < n ? 16 : 8) : 8;
+                stage(to + row * Shape::PITCH + m * GL_PITCH + c * (AL ? 16 : 8), in ? base + p : base, AL, in);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -285,21 +291,22 @@ __global__ void __launch_bounds__(512, 1)
             for (int c = 0; c < 2; ++c)
 #pragma unroll
                 for (int x = 0; x < TILES; ++x) acc[c][x][0] = acc[c][x][1] = 0.0;
-        const char* from = stages + q % S * STAGE + warp * 16;
-        double2 a[RB], b[CB];
+        const char* from = stages + q % S * STAGE + t * GL_PITCH + warp * 16;
 #pragma unroll
-        for (int r = 0; r < RB; ++r)
-            a[r] = *reinterpret_cast<const double2*>(from + ((8 * r + g) * 4 + t) * GL_PITCH);
+        for (int u = 0; u < U; ++u, from += 4 * GL_PITCH) {
+            double2 a[RB], b[CB];
 #pragma unroll
-        for (int j = 0; j < CB; ++j)
-            b[j] = *reinterpret_cast<const double2*>(from + ((8 * (RB + j) + g) * 4 + t) * GL_PITCH);
+            for (int r = 0; r < RB; ++r) a[r] = *reinterpret_cast<const double2*>(from + (8 * r + g) * Shape::PITCH);
 #pragma unroll
-        for (int r = 0; r < RB; ++r)
+            for (int j = 0; j < CB; ++j) b[j] = *reinterpret_cast<const double2*>(from + (8 * (RB + j) + g) * Shape::PITCH);
 #pragma unroll
-            for (int j = 0; j < CB; ++j) {
-                mma_f64(acc[0][r * CB + j], a[r].x, b[j].x);
-                mma_f64(acc[1][r * CB + j], a[r].y, b[j].y);
-            }
+            for (int r = 0; r < RB; ++r)
+#pragma unroll
+                for (int j = 0; j < CB; ++j) {
+                    mma_f64(acc[0][r * CB + j], a[r].x, b[j].x);
+                    mma_f64(acc[1][r * CB + j], a[r].y, b[j].y);
+                }
+        }
         if (q % steps != steps - 1) continue;
         // butterfly over the block's 32 chains: chain 2 w + c is in warp w
 #pragma unroll
@@ -875,7 +882,11 @@ unsigned rotate_pick(dft_context* ctx, const double* in, const double* in2, long
     const int rj = ((m + tiles - 1) / tiles + 7) / 8;
 #define DFT_ROT(R, P) return rotate_launch<R, P, AL>(ctx, in, in2, ldi, k1, k, Y, m, out, ldo, n, alpha, beta, ss)
     switch (rj) {
-        case 1: DFT_ROT(1, 2);
+        case 1:
+            // one step of few rows: more points per warp keep more loads in flight (128^3, 1 -> 1 41 -> 37 us, 3 -> 3
+            // 50 -> 42; no gain from 4 rows on)
+            if (k <= 3) DFT_ROT(1, 4);
+            DFT_ROT(1, 2);
         case 2: DFT_ROT(2, 2);
         case 3: DFT_ROT(3, 1);
         case 4: DFT_ROT(4, 1);

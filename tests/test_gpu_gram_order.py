@@ -1,4 +1,5 @@
-"""GPU: the order of summation of the narrow FP64 Gram products (dense_fp64.cu), bit for bit.
+"""GPU: the order of summation of the narrow FP64 Gram products (dense_fp64.cu), bit for bit, and rotations of few
+rows.
 
 The signs of the eigensolver's vectors turn on the last bits of these products, which rest on an FP64 matrix
 instruction adding its four products one after the other like four FMAs.  The chains, their tree and the
@@ -68,7 +69,7 @@ def host(tmp_path_factory):
 
 # both sides of every width at which the order changes, both kernels; even and odd leading dimensions
 @pytest.mark.parametrize("dims", [(4, 5, 6), (13, 11, 17), (33, 31, 17), (40, 40, 40)])
-@pytest.mark.parametrize("ka,kb", [(1, 1), (9, 5), (20, 4), (24, 12), (33, 8), (64, 4), (33, 9), (64, 16)])
+@pytest.mark.parametrize("ka,kb", [(1, 1), (8, 8), (5, 12), (9, 5), (20, 4), (24, 12), (33, 8), (64, 4), (33, 9), (64, 16)])
 def test_narrow_gram_bits(engine, host, dims, ka, kb):
     torch = pytest.importorskip("torch")
     sms = torch.cuda.get_device_properties(0).multi_processor_count
@@ -103,3 +104,18 @@ def test_narrow_gram_bits(engine, host, dims, ka, kb):
     for i in sorted({0, ka // 2, ka - 1, min(7, ka - 1), min(8, ka - 1)}):
         for j in sorted({0, kb // 2, kb - 1, min(7, kb - 1)}):
             assert got[i, j] == one(A[i], B[j]), (i, j)
+
+
+# few rows of the block that is rotated: a warp then takes more points (ragged ends of 64)
+@pytest.mark.parametrize("dims", [(2, 2, 2), (5, 7, 3), (8, 8, 8), (33, 31, 17)])
+@pytest.mark.parametrize("k,m", [(1, 8), (2, 5), (3, 3), (3, 9), (4, 4)])
+def test_rotation_of_few_rows(engine, dims, k, m):
+    g = dft_b200.CartesianGrid(*dims, -1.0, 1.0, -1.5, 1.5, -2.0, 2.0)
+    N = g.getSize()
+    rng = np.random.default_rng(k * 100 + m)
+    V, Y = rng.standard_normal((k, N)), rng.standard_normal((k, m))
+    X = engine.upload(np.full((m, N), 7.0))
+    engine.rotate(g, engine.upload(V), N, k, Y, X, N)
+    # k products and sums in any order: |error| <= (k + 2) eps sum |y||v|
+    bound = (k + 2) * 2.0 ** -53 * (np.abs(Y).T @ np.abs(V))
+    assert np.all(np.abs(X.to_host((m, N)) - Y.T @ V) <= 2 * bound)
