@@ -754,9 +754,14 @@ void apply_hamiltonian(dft_context* ctx, const Grid& g, const double* V, const d
     if (zset == 0 && tuned != ctx->tuned.end()) zset = tuned->second[3];
     const bool single = nbt == 1 && ctx->hpsi_variant != 1 && variant != 3;
     if (single && g.nx % 2 == 0 && ld % 2 == 0 && ((uintptr_t)V | (uintptr_t)psi | (uintptr_t)hpsi) % 16 == 0) {
-        // two columns per thread; 16 threads across where that leaves fewer of them idle
-        const int pairs = g.nx / 2, tx = (pairs + 15) / 16 * 16 < (pairs + 31) / 32 * 32 ? 16 : 32, ty = 256 / tx;
+        // two columns per thread; 16 threads across where that leaves fewer of them idle, and one per pair of
+        // shorter rows, the blocks then of equal height (16 bands, 16 across / one per pair: 20 x 20 x 500 27 / 15 us,
+        // 10 x 200 x 300 95 / 35)
+        const int pairs = g.nx / 2;
+        const int tx = pairs < 16 ? pairs : (pairs + 15) / 16 * 16 < (pairs + 31) / 32 * 32 ? 16 : 32;
+        int ty = 256 / tx;
         const int px = (pairs + tx - 1) / tx, py = (g.ny + ty - 1) / ty;
+        if (pairs < 16) ty = (g.ny + py - 1) / py;
         const int pz = zset > 0 ? std::min(zset, g.nz)
                                 : march_chunk(g.nz, (long long)px * py * nbands, (long long)HP_BLOCKS * ctx->num_sms);
         const int chunks = (g.nz + pz - 1) / pz, most = std::max(1, 65535 / chunks);
