@@ -1477,9 +1477,15 @@ JacobiResult hartree(dft_context* ctx, const Grid& g, const double* rho, double*
     dim3 grid(bx, by, (g.nz + zc - 1) / zc);
     JacobiCtrl* hc = (JacobiCtrl*)pinned(ctx, (sizeof(JacobiCtrl) + 7) / 8);
     long launched = 0;
+    // both buffers hold the start; sweeps go b0 -> b1 -> b0, a warm start's first one into vh, where it mostly ends
+    double *b0 = guess ? buf1 : vh, *b1 = guess ? vh : buf1;
+    auto into_vh = [&](const double* result) {
+        if (result != vh)
+            DFT_CUDA(cudaMemcpyAsync(vh, result, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));
+    };
     auto sweeps_launch = [&](long nb) {
         for (long s = 0; s < nb; ++s)
-            jacobi_sweep_kernel<<<grid, block, 0, ctx->stream>>>(g, rho, vh, buf1, ctrl, den, tol, max_sweeps, zc);
+            jacobi_sweep_kernel<<<grid, block, 0, ctx->stream>>>(g, rho, b0, b1, ctrl, den, tol, max_sweeps, zc);
         DFT_LAUNCH_CHECK();
         count_launch(ctx, nb);
         launched += nb;
@@ -1491,6 +1497,8 @@ JacobiResult hartree(dft_context* ctx, const Grid& g, const double* rho, double*
     // more), else one sweep per launch; 2/4/8 select the temporally blocked kernel.  Microseconds per
     // sweep: resident against one launch each, 64^3 2.75 / 8.3, 72^3 3.16 / 8.3, 80^3 3.96 / 10.4, 86^3
     // 4.17 / 10.2; one launch in global memory against one each, 250 x 250 x 3 5.7 / 6.3, 256 x 256 x 4 6.2 / 6.8.
+    // A limit of fewer than six sweeps is not worth a resident launch (16^3 to 80^3: 2 sweeps 69 to 100 us, by
+    // single launches 41 to 51; 5 sweeps 60 to 102 and 69 to 87).
     int tmax = ctx->jacobi_sweeps_per_launch;
     if (tmax == 0) {
         auto t = ctx->tuned.find({(long long)g.nx, (long long)g.ny, (long long)g.nz});
@@ -1502,20 +1510,17 @@ JacobiResult hartree(dft_context* ctx, const Grid& g, const double* rho, double*
         // sweep by itself is 3 us, a resident launch with its exchange ring cleared 20
         if (guess) {
             sweeps_launch(1);
-            if (hc->done) {
-                DFT_CUDA(cudaMemcpyAsync(vh, buf1, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));
-                return {1L, hc->last_diff};
-            }
+            if (hc->done) return {1L, hc->last_diff};
         }
-        double *from = launched ? buf1 : vh, *other = launched ? vh : buf1, *result = nullptr;
-        bool solved = hartree_resident(ctx, g, rho, from, other, tol, max_sweeps - launched, &r, &result);
-        if (!solved && (tmax == -1 || g.N <= 64LL * 64 * 64)) {
+        double *from = launched ? b1 : b0, *other = launched ? b0 : b1, *result = nullptr;
+        const bool few = tmax == 0 && max_sweeps - launched < 6;
+        bool solved = !few && hartree_resident(ctx, g, rho, from, other, tol, max_sweeps - launched, &r, &result);
+        if (!solved && !few && (tmax == -1 || g.N <= 64LL * 64 * 64)) {
             r = hartree_persistent(ctx, g, rho, from, other, tol, max_sweeps - launched, &result);
             solved = true;
         }
         if (solved) {
-            if (result != vh)
-                DFT_CUDA(cudaMemcpyAsync(vh, buf1, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));
+            into_vh(result);
             r.sweeps += launched;
             return r;
         }
@@ -1531,9 +1536,7 @@ JacobiResult hartree(dft_context* ctx, const Grid& g, const double* rho, double*
          batch = std::min<long>(batch * 2, 512))
         sweeps_launch(std::min<long>(batch, max_sweeps - launched));
     const long sweeps = (long)hc->sweep;
-    if (sweeps & 1) {
-        DFT_CUDA(cudaMemcpyAsync(vh, buf1, sizeof(double) * (size_t)g.N, cudaMemcpyDeviceToDevice, ctx->stream));
-    }
+    into_vh(sweeps & 1 ? b1 : b0);
     return {sweeps, hc->last_diff};
 }
 

@@ -347,30 +347,25 @@ __global__ void __launch_bounds__(RJ_THREADS, 1)
 // and 2,000 per round.
 bool pick_shape(const Grid& g, int num_sms, int T, RJShape* best, double* cost) {
     bool found = false;
-    const int n[3] = {g.nx, g.ny, g.nz};
-    for (int bx = 1; bx <= std::min(num_sms, n[0] - 2); ++bx)
-        for (int by = 1; bx * by <= num_sms && by <= n[1] - 2; ++by) {
-            const int bz = std::min(num_sms / (bx * by), n[2] - 2);
-            const int m[3] = {bx, by, bz};
-            long long e[3];
-            for (int d = 0; d < 3; ++d) e[d] = (n[d] - 2 + m[d] - 1) / m[d];
-            double swept = 0.0;
-            long long region = 1, rows = 0;
-            for (int t = 0; t <= T; ++t) {
-                long long p[3];
-                for (int d = 0; d < 3; ++d) p[d] = std::min<long long>(n[d] - (t == T ? 0 : 2), e[d] + 2 * t);
-                if (t < T) {
-                    const long long r = (p[0] + 15) / 16 * p[1];
-                    rows = std::max(rows, r);
-                    swept += (double)(r * 16 * p[2]);
-                } else {
-                    region = p[0] * p[1] * p[2];
-                }
-            }
-            const long long halo = region - e[0] * e[1] * e[2];
-            if (3 * region * (long long)sizeof(double) > (long long)RJ_SMEM || rows > RJ_ROWS ||
-                halo > (long long)RJ_HALO * RJ_THREADS || region * 8 < halo * 4)
+    // per axis: interior points, and points of sweep T - t (t more per side than the e owned ones)
+    const int nx = g.nx - 2, ny = g.ny - 2, nz = g.nz - 2;
+    const auto swept_points = [](int n, int e, int t) { return std::min(n, e + 2 * t); };
+    for (int bx = 1; bx <= std::min(num_sms, nx); ++bx) {
+        const int ex = (nx + bx - 1) / bx, xs = (swept_points(nx, ex, T - 1) + 15) / 16;
+        if (xs > RJ_ROWS) continue;
+        for (int by = 1; bx * by <= num_sms && by <= ny; ++by) {
+            const int ey = (ny + by - 1) / by;
+            if (xs * swept_points(ny, ey, T - 1) > RJ_ROWS) continue;
+            const int bz = std::min(num_sms / (bx * by), nz), ez = (nz + bz - 1) / bz;
+            const long long region =
+                (long long)std::min(g.nx, ex + 2 * T) * std::min(g.ny, ey + 2 * T) * std::min(g.nz, ez + 2 * T);
+            const long long halo = region - (long long)ex * ey * ez;
+            if (3 * region * (long long)sizeof(double) > (long long)RJ_SMEM || halo > (long long)RJ_HALO * RJ_THREADS ||
+                region * 8 < halo * 4)
                 continue;
+            double swept = 0.0;
+            for (int t = 0; t < T; ++t)
+                swept += 16.0 * ((swept_points(nx, ex, t) + 15) / 16 * swept_points(ny, ey, t)) * swept_points(nz, ez, t);
             const double c = (800.0 * T + 0.5 * swept + 0.7 * (double)halo + 2000.0) / T;
             if (!found || c < *cost) {
                 found = true;
@@ -378,6 +373,7 @@ bool pick_shape(const Grid& g, int num_sms, int T, RJShape* best, double* cost) 
                 *best = {bx, by, bz, (int)region};
             }
         }
+    }
     return found;
 }
 

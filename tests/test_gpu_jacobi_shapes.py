@@ -53,6 +53,19 @@ def test_same_bits(engine, dims, mode, one, cap):
             assert got[3] == (2 if guess is None else 3) if one else got[3] >= 40
 
 
+# limits that fall in the first rounds of the resident solve, which the default leaves to single launches
+@pytest.mark.parametrize("dims", [(3, 3, 3), (4, 3, 9), (18, 33, 20), (48, 48, 48), (64, 40, 50), (80, 80, 80)])
+@pytest.mark.parametrize("cap", [1, 2, 3, 4, 5, 6, 7])
+def test_resident_solve_of_few_sweeps(engine, dims, cap):
+    g = _grid(dims)
+    rng = np.random.default_rng(cap)
+    rho = rng.uniform(0.0, 1.0, g.getSize()) ** 8
+    for guess in (None, rng.standard_normal(g.getSize())):
+        ref = _solve(engine, 1, g, rho, 0.0, cap, guess)
+        assert _solve(engine, -1, g, rho, 0.0, cap, guess)[:3] == ref[:3]
+        assert _solve(engine, 0, g, rho, 0.0, cap, guess)[:3] == ref[:3]
+
+
 def test_global_memory_launch_gives_up(engine):
     """A grid beyond the shared memory with a barrier poll limit of 1: an error with a message, and the context solves
     normally afterwards."""
