@@ -300,7 +300,12 @@ def measure_gram(eng, torch, stream, w, ka, kb, reps=20):
         times.append(e0.elapsed_time(e1))
     ms = statistics.median(times)
     byts = 8.0 * N * (ka + kb)
-    return {"ka": ka, "kb": kb, "ms": ms, "bytes": byts, "gbs": byts / (ms * 1e-3) / 1e9,
+    # dense_fp64.cu: narrow products keep their order of summation
+    rows, cols = (1 if ka <= 8 else 2 if ka <= 16 else 4 if ka <= 32 else 8), (4 if kb <= 4 else 8 if kb <= 8 else 16)
+    kernel = ("gram_mma_kernel" if ka > 64 or kb > 16 else
+              "gram_lanes_kernel + gram_lanes_sum_kernel" if rows * cols <= 64 else
+              "gram_chunk_kernel + gram_chunk_sum_kernel")
+    return {"ka": ka, "kb": kb, "ms": ms, "bytes": byts, "gbs": byts / (ms * 1e-3) / 1e9, "kernel": kernel,
             "tflops": 2.0 * N * ka * kb / (ms * 1e-3) / 1e12}
 
 
@@ -430,7 +435,7 @@ def kernel_table(eng, torch, stream, flush, peak, n=192, h=0.2, reps=3):
         gbs = 32.0 * N / (ms * 1e-3) / 1e9
         out[f"xc_{kind}"] = {"ms": ms, "gbs": gbs, "frac": gbs / peak,
                              "kernels": "xc_point_kernel + xc_div_kernel" if kind == "PBE96" else
-                             "xc_point_kernel + xc_lda_copy_kernel"}
+                             "xc_point_kernel"}
     return out
 
 
@@ -728,15 +733,15 @@ def main():
                    **cmp},
         "gpu_launches": launches,
         "e2e": {"value": e2e_val, "unit": "SCF/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-        "roofline": {"bound": "hbm", "kernel": "gram_small_kernel (FP64 Gram of the eigensolver, one launch)",
+        "roofline": {"bound": "hbm", "kernel": gr["kernel"] + " (FP64 Gram of the eigensolver)",
                      "achieved": gr["gbs"], "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": gr["gbs"] / peaks["hbm_gbs"], "peak_source": peaks["source"],
-                     # ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of this shape
-                     # (48^3, 20 x 4): 21,251,072 + 0 bytes
-                     "traffic": 21251072.0 if (w["n"] == (48, 48, 48) and gr["ka"] == 20 and gr["kb"] == 4) else None,
+                     # ncu dram__bytes_read.sum + dram__bytes_write.sum of the two launches at this shape
+                     # (48^3, 20 x 4): 21,255,424 + 284,672 bytes, nothing written
+                     "traffic": 21540096.0 if (w["n"] == (48, 48, 48) and gr["ka"] == 20 and gr["kb"] == 4) else None,
                      "bytes_per_call": gr["bytes"], "ms_per_call": gr["ms"], "ka": gr["ka"], "kb": gr["kb"],
                      "note": "the eigensolver's narrow Gram product, timed per call with its read-back; at 48^3 "
-                             "one call moves 21 MB, so the in-launch reduction and the read-back bind, not HBM"},
+                             "one call moves 21 MB, so its launches (14 and 5 us) and the read-back bind, not HBM"},
         "plain_roofline": {"bound": "hbm", "kernel": jac["kernel"], "achieved": jac["gbs"],
                            "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": jac["gbs"] / peaks["hbm_gbs"],
                            "bytes_per_sweep": jac["bytes_per_sweep"], "ms_per_sweep": jac["ms_per_sweep"],

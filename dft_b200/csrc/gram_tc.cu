@@ -118,8 +118,8 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 // split; the rest of the tile is zeroed once.  The products of a step go hi*hi, A hi * B lo, A lo * B hi on
 // either side, so an element's sum does not depend on the tiling.
 //
-// Bound by the instructions of the split (ALU pipe 65 % busy, issue slots 54 %, conversions 26 %, DRAM at 2.7 TB/s:
-// 138 x 69, 112 x 97 x 101, where this took 1500 -> 703 us).  A tile of 128 rows of A per block read B a second
+// Bound by the instructions of the split (ALU pipe 72 % busy, issue slots 57 %, conversions 25 %, DRAM at 2.7 TB/s:
+// 138 x 69, 112 x 97 x 101, where this took 1500 -> 692 us).  A tile of 128 rows of A per block read B a second
 // time for the ten rows left over, split 512 rows of which 207 exist, and loaded and converted by turns.
 //
 // W = 8: two groups of eight warps take the slices in turn, each into its own stage, and a warp of its own issues the

@@ -1084,8 +1084,9 @@ __global__ void __launch_bounds__(TB_R* TB_R, 1)
     }
 }
 
-// ---- persistent Jacobi: the whole solve in one cooperative launch --------------------------
-// For small grids the sweep is a few microseconds of work and launch latency dominates.  All
+// ---- persistent Jacobi: the whole solve in one cooperative launch, the grid in global memory
+// For grids whose sweep is a few microseconds of work (launch latency dominates) and that do not fit the shared
+// memory of all SMs (jacobi_resident.cu).  All
 // blocks stay resident (cooperative launch) and meet at a grid barrier after every sweep;
 // every block reads the same global max|dV| after the barrier, so all stop at the same sweep.
 // Loads of the iterates bypass L1 (__ldcg): other SMs rewrite them every sweep.
@@ -1742,9 +1743,9 @@ constexpr int XP = 128;
 // Pass 1: functional at every point above the floor (xc_fast.cuh).  GGA: writes d f/d n_sigma and the
 // gradient coefficients c_sigma (zero below the floor, reference :626-706); LDA: the potentials themselves, either
 // of which may be absent.  partial: when given, per-block sums of n eps dV (reference :749-842).  One
-// evaluation serves both spins and the energy.  Bound by its instructions (FP64 pipe 43 % busy, of which
-// logarithms, cube roots and divisions are most); 128 threads and 96 registers leave 20 warps on an SM, 158 -> 146 us
-// against 16.  Both passes, PBE at 128^3: 568 -> 223 us; PZ81 at 75 x 63 x 91: 62 -> 34 us.
+// evaluation serves both spins and the energy.  Bound by its instructions (issue slots 57 %, FP64 pipe 47 %
+// busy; logarithms, cube roots and divisions are most of them); 128 threads and 96 registers leave 20 warps on an SM, 158 -> 146 us
+// against 16.  Both passes, PBE at 128^3: 568 -> 225 us; PZ81 at 75 x 63 x 91: 62 -> 34 us.
 template <int KIND, bool POT>
 __global__ void __launch_bounds__(XP, 5)
     xc_point_kernel(Grid g, XCScale h, const double* __restrict__ na, const double* __restrict__ nb,

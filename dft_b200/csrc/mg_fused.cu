@@ -13,8 +13,9 @@
 // launch with a cluster barrier between them took 64 us where these launches take 30: each pass paid an L2
 // round trip and the barrier.
 //
-// The restriction weights and interpolation cells of every level come from a table computed once per solve
-// (mg_tables): a tile's own divisions took longer than its passes.
+// The restriction weights and interpolation cells of every level come from a table (mg_tables; one launch per
+// Poisson solve, and per cycle of the eigensolver's preconditioner and the mixer): a tile's own divisions took
+// longer than its passes.
 //
 // Every pass keeps the operations and the order of the separate passes it replaces (divisions by the
 // diagonal through exact_div.cuh), so the preconditioner's results are the same bits however a level is

@@ -59,7 +59,7 @@ void mg_interpolate(dft_context* ctx, const Grid& f, const Grid& c, const double
 void mg_start_cycle(dft_context* ctx, MGHistory* hist);
 // the current word of hist = max |s src - (d v - sum w v)| over the interior
 void mg_residual_max(dft_context* ctx, const Grid& g, const double* src, double s, const double* v, MGHistory* hist);
-// L.back().v = the coarsest level's solution for its src by red-black SOR, or by Jacobi sweeps
+// l.v = the coarsest level's solution for src by red-black SOR, or by Jacobi sweeps
 void mg_coarsest_solve(dft_context* ctx, const MGLevel& l, const double* src, bool sor);
 
 }  // namespace dftb

@@ -98,9 +98,10 @@ dft_status_t dft_context_synchronize(dft_context* ctx);
  *                               tile; needs nx and ld even and a 16-byte-aligned psi, else 0 is
  *                               used; 3 = the single-band march of 0 with the next plane's loads
  *                               issued one step ahead.  Results identical for every value.
- *   "grid_barrier_poll_limit":  0 = 2^24 (default): polls a block of the persistent Jacobi
- *                               launch makes at a grid barrier before it gives up; the solve then
- *                               fails with DFT_CUDA_ERROR and the context stays usable.
+ *   "grid_barrier_poll_limit":  0 (default): polls a block of a one-launch Jacobi solve makes at a
+ *                               grid barrier (2^24) or a thread at a halo value (2^22) before it
+ *                               gives up; the solve then fails with DFT_CUDA_ERROR and the context
+ *                               stays usable.
  *   "hpsi_zchunk":              0 = auto (default), else the number of z-planes each block of the
  *                               register-march H psi kernels walks (same results for every value).
  *   "multigrid_fused_restriction": 1 (default) = the Poisson multigrid's passes are fused and its
